@@ -121,7 +121,7 @@ int tomoSweepDevice(void* ev_start, void* ev_stop, float* kernel_ms);
 int tomoFinish(float* Mo, float* Mss, float* Vtc);
 
 /* Launch accounting.  Kernel kinds, in order: reset, rotate, bin_count,
- * bin_scan, bin_fill, strip, bed, fold, strip re-runs.  tomoProfile(enable, reset) turns
+ * bin_scan, bin_fill, strip, bed, fold, strip re-runs, raster.  tomoProfile(enable, reset) turns
  * per-launch CUDA-event timing on or off (events are recorded on the stream
  * each kernel is launched on) and optionally clears the log;
  * tomoGetKernelLog fills launches / total ms / timed launches per kind and
@@ -235,7 +235,7 @@ int tomoSurrogateSearch(const float* f32info, const int* i32info, const float* Y
  * host arrays of nYPR floats that receive what getMo/getMss/getVtc return
  * after TomoSh_CUDA, and the return value is optID (or a negative error).
  * The render pixels, vm_info and mat4x4 are not produced.
- *   - allocates nothing: device scratch is one file-scope 8 MiB __device__
+ *   - allocates nothing: device scratch is one file-scope 16 MiB __device__
  *     array per device, host staging is file-scope arrays; no cudaMalloc,
  *     cudaFree or allocating library routine is called;
  *   - limits: at most 16384 triangles and 16384 vertices, and a footprint

@@ -106,6 +106,12 @@ struct EngineParams {
   int* bins;            // [Bo][bin_cap]
   int bin_cap;
 
+  // accepted pixels of each strip (normal strips: k_raster -> k_strip)
+  uint2* ents;          // [Bo][S][ent_cap] (z, nz) key; slot within the strip
+  int* ent_cnt;         // [Bo][S] pixels appended (may exceed ent_cap: the strip overflowed)
+  int hshift;           // log2(H)
+  int rast_lanes;       // lanes per triangle in k_raster (a power of two)
+
   // per-batch results
   long long* acc;       // [Bo][kAccLanes]
   int* flags;           // [Bo]
@@ -139,7 +145,7 @@ struct EngineParams {
 };
 
 // Kernel kinds for launch accounting.
-enum : int { kKReset = 0, kKRotate, kKCount, kKScan, kKFill, kKStrip, kKBed, kKFold, kKStripRedo, kKinds };
+enum : int { kKReset = 0, kKRotate, kKCount, kKScan, kKFill, kKStrip, kKBed, kKFold, kKStripRedo, kKRaster, kKinds };
 
 // Host-side launch log: launch counts per kernel kind and, when timing is
 // on, one event pair per launch recorded on the launching stream.

@@ -31,6 +31,7 @@ namespace tomo {
 
 size_t strip_smem_bytes(int mode, int H, int G, int ent_cap);
 size_t strip_four_per_sm_budget();
+int raster_lanes(int nT, int Bo);
 cudaError_t configure_kernels(size_t normal_smem, size_t safe_smem, size_t prio_smem);
 cudaError_t launch_batch(const EngineParams& p, cudaStream_t main, size_t strip_smem, LaunchLog* L);
 cudaError_t launch_fold(const EngineParams& p, cudaStream_t side, LaunchLog* L);
@@ -187,6 +188,11 @@ struct DevBuf {
 // Largest slot grid edge (columns of the rotated footprint at the voxel pitch).
 constexpr int kMaxGrid = 4096;
 
+// Most bytes of one batch's strip pixel lists (256 orientations of the
+// 501-column grid take 1.2 GB, two such sets at once; wide grids sweep fewer
+// orientations per batch).
+constexpr size_t kListBytes = size_t(6) << 30;
+
 // Orientations the last tomoSweepStatic call re-ran, per strip configuration.
 int g_static_reruns[5];
 
@@ -207,17 +213,19 @@ struct BatchSet {   // per-batch buffers read by the fold, double-buffered
   cudaEvent_t folded = nullptr;
 };
 
-struct PrepSet {    // a batch's rotated vertices and strip bins (binning -> strips)
+struct PrepSet {    // a batch's rotated vertices and strip lists (rasterizer or binning -> strips)
   DevBuf<float4> xf;
   DevBuf<unsigned> minkey;
   DevBuf<unsigned> trange;
   DevBuf<int> bin_off, bin_cur, bins, bbox;
+  DevBuf<uint2> ents;
+  DevBuf<int> ent_cnt;
   DevBuf<uint8_t> bedf;
   cudaEvent_t ready = nullptr;
   void release()
   {
     xf.release(); minkey.release(); trange.release(); bin_off.release(); bin_cur.release(); bins.release();
-    bbox.release(); bedf.release();
+    bbox.release(); ents.release(); ent_cnt.release(); bedf.release();
   }
 };
 
@@ -522,6 +530,7 @@ struct Engine {
     p.bed_outer = P.bed_outer; p.bed_inner = P.bed_inner; p.bed_type = P.bed_type;
     p.bed_r = (int)P.bed_outer; p.bed_thickness = P.bed_thickness;
     p.G = G; p.H = H; p.S = S; p.mode = mode;
+    while ((1 << p.hshift) < H) p.hshift++;   // strip heights are powers of two
     p.half = P.dVoxel * 0.5f;
     p.shell_off = (float)(int)(P.shell_thickness + 0.999f);
     p.twin = (P.shell && P.shell_thickness > 0.001f) ? 1 : 0;
@@ -537,17 +546,32 @@ struct Engine {
     return p;
   }
 
-  int reserve_batch(int Bo, int bin_cap, int nprep = 1)
+  // Orientations per batch: `want`, or fewer where the strips' pixel lists
+  // (normal strips, the current configuration) would pass kListBytes.
+  int batch_size(int want, int mode) const
+  {
+    if (mode != 0) return want;
+    const size_t per = (size_t)S * ent_cap * sizeof(uint2);
+    return (int)std::min<size_t>(want, std::max<size_t>(1, kListBytes / std::max<size_t>(per, 1)));
+  }
+
+  // Buffers of a batch of Bo orientations in the current strip configuration.
+  int reserve_batch(int mode, int Bo, int bin_cap, int nprep = 1)
   {
     const size_t GG = (size_t)G * G;
     for (int q = 0; q < nprep; q++) {
       PrepSet& b = W.prep[q];
       TOMO_CUDA(b.xf.reserve((size_t)Bo * std::max(P.n_vtx, 1)));
       TOMO_CUDA(b.minkey.reserve((size_t)Bo * 4));
-      TOMO_CUDA(b.trange.reserve((size_t)Bo * std::max(P.n_tri, 1)));
-      TOMO_CUDA(b.bin_off.reserve((size_t)Bo * (S + 1)));
-      TOMO_CUDA(b.bin_cur.reserve((size_t)Bo * S));
-      TOMO_CUDA(b.bins.reserve((size_t)Bo * bin_cap));
+      if (mode == 0) {
+        TOMO_CUDA(b.ents.reserve((size_t)Bo * S * ent_cap));
+        TOMO_CUDA(b.ent_cnt.reserve((size_t)Bo * S));
+      } else {
+        TOMO_CUDA(b.trange.reserve((size_t)Bo * std::max(P.n_tri, 1)));
+        TOMO_CUDA(b.bin_off.reserve((size_t)Bo * (S + 1)));
+        TOMO_CUDA(b.bin_cur.reserve((size_t)Bo * S));
+        TOMO_CUDA(b.bins.reserve((size_t)Bo * bin_cap));
+      }
       TOMO_CUDA(b.bbox.reserve((size_t)Bo * 4));
       TOMO_CUDA(b.bedf.reserve((size_t)Bo * GG));
     }
@@ -581,6 +605,7 @@ struct Engine {
     p.ori = ori.ptr + first;
     p.xf = b.xf.ptr; p.minkey = b.minkey.ptr; p.trange = b.trange.ptr;
     p.bin_off = b.bin_off.ptr; p.bin_cur = b.bin_cur.ptr; p.bins = b.bins.ptr; p.bin_cap = bin_cap;
+    p.ents = b.ents.ptr; p.ent_cnt = b.ent_cnt.ptr; p.rast_lanes = raster_lanes(p.nT, Bo);
     p.bbox = b.bbox.ptr; p.bedf = b.bedf.ptr;
     p.acc = set[which].acc.ptr; p.flags = set[which].flags.ptr;
     p.foldcnt = set[which].foldcnt.ptr; p.foldp = set[which].foldp.ptr; p.foldmeta = set[which].foldmeta.ptr;
@@ -655,7 +680,7 @@ struct Engine {
     choose_strips(c);
     H_sweep = H;
     TOMO_TRY(configure());
-    const int Bo = std::min(batch, n);
+    int Bo = batch_size(std::min(batch, n), cfg[c].mode);
     const int bin_cap = 4 * P.n_tri + 4096;
     TOMO_TRY(reserve_outputs());
     // Two batches in flight: batch k+1's binning (reset, rotate, bin
@@ -664,7 +689,7 @@ struct Engine {
     // on the side stream.  A set is rebinned only after the fold of the
     // batch that last used it.
     const bool pipe = n > Bo;
-    TOMO_TRY(reserve_batch(Bo, bin_cap, pipe ? 2 : 1));
+    TOMO_TRY(reserve_batch(cfg[c].mode, Bo, bin_cap, pipe ? 2 : 1));
     if (ids) TOMO_CUDA(launch_zero_ids(o_nbed.ptr, ids, n, main));
     else TOMO_CUDA(cudaMemsetAsync(o_nbed.ptr, 0, sizeof(int) * nYPR, main));
     if (pipe) {
@@ -673,8 +698,9 @@ struct Engine {
     }
     EngineParams p = base_params(cfg[c].mode);
     int k = 0;
-    for (int first = 0; first < n; first += Bo, k++) {
-      const int nb = std::min(Bo, n - first);
+    int nb = 0;
+    for (int first = 0; first < n; first += nb, k++) {
+      nb = std::min(Bo, n - first);
       const int which = k & 1;
       const int q = pipe ? which : 0;
       cudaStream_t bs = pipe ? W.binning : main;
@@ -695,7 +721,13 @@ struct Engine {
       if (adapt && k < 3 && first + nb < n) {
         bool changed = false;
         TOMO_TRY(adapt_after(first, nb, &c, &changed));
-        if (changed) p = base_params(cfg[c].mode);
+        if (changed) {
+          // every launch so far has finished (adapt_after waited), so the
+          // lists may move; the rest of the sweep may need smaller batches
+          Bo = batch_size(Bo, cfg[c].mode);
+          TOMO_TRY(reserve_batch(cfg[c].mode, Bo, bin_cap, pipe ? 2 : 1));
+          p = base_params(cfg[c].mode);
+        }
       }
     }
     // join the side stream back into main
@@ -716,9 +748,9 @@ struct Engine {
     DevBuf<int> sub;
     TOMO_CUDA(sub.reserve(ids.size()));
     TOMO_CUDA(cudaMemcpyAsync(sub.ptr, ids.data(), sizeof(int) * ids.size(), cudaMemcpyHostToDevice, main));
-    const int Bo = std::min<int>(batch, (int)ids.size());
+    const int Bo = batch_size(std::min<int>(batch, (int)ids.size()), mode);
     const int normal_cap = 4 * P.n_tri + 4096;
-    TOMO_TRY(reserve_batch(Bo, mode != 1 ? normal_cap : 1));
+    TOMO_TRY(reserve_batch(mode, Bo, mode != 1 ? normal_cap : 1));
     EngineParams p = base_params(mode);
     p.variant = c;
     for (int first = 0; first < (int)ids.size(); first += Bo) {
@@ -977,7 +1009,7 @@ struct Engine {
     EngineParams p = base_params(mode);
     p.dump_slot = 0; p.dump_cols = dump_cols.ptr; p.dump_keys = dump_keys.ptr; p.dump_types = dump_types.ptr;
     int cap = 4 * P.n_tri + 4096;
-    TOMO_TRY(reserve_batch(1, mode != 1 ? cap : 1));
+    TOMO_TRY(reserve_batch(mode, 1, mode != 1 ? cap : 1));
     bind_batch(p, 1, mode != 1 ? cap : INT_MAX, 0, id);
     if (mode != 1) {
       TOMO_CUDA(launch_batch(p, main, smem, &log));
@@ -1584,7 +1616,8 @@ int tomoFinish(float* Mo, float* Mss, float* Vtc)
 
 namespace tomo {
 
-constexpr size_t kStaticArenaBytes = size_t(8) << 20;   // 8 MiB of device scratch per device
+constexpr size_t kStaticArenaBytes = size_t(16) << 20;  // 16 MiB of device scratch per device
+constexpr size_t kStaticListBytes = size_t(8) << 20;    // of which the strips' pixel lists
 constexpr int kStaticMaxTri = 16384;
 constexpr int kStaticMaxVtx = 16384;
 constexpr int kStaticBatch = 4;
@@ -1604,6 +1637,7 @@ constexpr size_t static_bytes(size_t nV, size_t nT)
   return static_round(16 * nV) * 2 + static_round(16 * nT) + static_round(4 * 9 * B) + static_round(4 * B) +
          static_round(16 * B * nV) + static_round(4 * 4 * B) + static_round(4 * B * nT) +
          static_round(4 * B * (S + 1)) + static_round(4 * B * S) + static_round(4 * B * (4 * nT + 4096)) +
+         static_round(4 * B * S) + static_round(kStaticListBytes) +
          static_round(4 * 4 * B) + static_round(B * GG) + static_round(8 * B * kAccLanes) + static_round(4 * B) +
          static_round(4 * B * S) + static_round(4 * B * GG) + static_round(2 * B * GG) + static_round(sizeof(FoldEscape) * kFoldEscapes) +
          static_round(4) + static_round(4 * B * S * 8) +
@@ -1616,8 +1650,9 @@ struct StaticLayout {
   float4 *vpos, *vnrm, *xf;
   int4* tri;
   float* rot;
-  int *ori, *bin_off, *bin_cur, *bins, *bbox, *flags, *foldcnt, *foldmeta, *o_nbed, *o_flags;
+  int *ori, *bin_off, *bin_cur, *bins, *ent_cnt, *bbox, *flags, *foldcnt, *foldmeta, *o_nbed, *o_flags;
   unsigned *minkey, *trange;
+  uint2* ents;
   uint8_t* bedf;
   long long *acc, *o_vo, *o_vss, *o_vtc, *o_ent, *o_col;
   unsigned* foldp;
@@ -1647,6 +1682,8 @@ StaticLayout static_layout(unsigned char* base, int nV, int nT)
   L.bin_cur = (int*)take(4 * B * S);
   L.bins_total = (long long)B * (4 * (long long)nT + 4096);
   L.bins = (int*)take(4 * (size_t)L.bins_total);
+  L.ent_cnt = (int*)take(4 * B * S);
+  L.ents = (uint2*)take(kStaticListBytes);
   L.bbox = (int*)take(4 * 4 * B);
   L.bedf = (uint8_t*)take(B * GG);
   L.acc = (long long*)take(8 * B * kAccLanes);
@@ -1697,6 +1734,9 @@ void static_bind(EngineParams& p, const StaticLayout& L, int nb, int slot, int b
   p.ori = L.ori + slot; p.Bo = nb;
   p.xf = L.xf; p.minkey = L.minkey; p.trange = L.trange;
   p.bin_off = L.bin_off; p.bin_cur = L.bin_cur; p.bins = L.bins; p.bin_cap = bin_cap;
+  p.ents = L.ents; p.ent_cnt = L.ent_cnt; p.rast_lanes = raster_lanes(p.nT, nb);
+  if (p.mode == 0)   // a list shorter than the strip's shared memory only flags overflow earlier
+    p.ent_cap = (int)std::min<size_t>(p.ent_cap, kStaticListBytes / ((size_t)nb * p.S * sizeof(uint2)));
   p.acc = L.acc; p.flags = L.flags; p.bbox = L.bbox; p.bedf = L.bedf;
   p.foldcnt = L.foldcnt; p.foldp = L.foldp; p.foldmeta = L.foldmeta;
   p.foldtc = p.explicit_ss ? nullptr : L.foldtc;
@@ -2009,7 +2049,7 @@ struct MultiEngine {
     std::vector<const void*> v;
     for (const auto& q : W.prep)
       v.insert(v.end(), {q.xf.ptr, q.minkey.ptr, q.trange.ptr, q.bin_off.ptr, q.bin_cur.ptr, q.bins.ptr, q.bbox.ptr,
-                         q.bedf.ptr});
+                         q.ents.ptr, q.ent_cnt.ptr, q.bedf.ptr});
     for (const auto& st : W.set) {
       v.insert(v.end(), {st.acc.ptr, st.flags.ptr, st.foldcnt.ptr, st.foldp.ptr, st.foldtc.ptr, st.foldx.ptr, st.foldxn.ptr,
                          st.foldmeta.ptr});
@@ -2027,10 +2067,12 @@ struct MultiEngine {
   {
     for (auto* e : meshes) {
       if (e->nYPR == 0 || e->P.n_tri == 0) continue;
-      e->choose_strips(0);
+      const int c = e->start_cfg == 4 ? 4 : 0, mode = e->cfg[c].mode;   // as sweep_batches starts
+      e->choose_strips(c);
       TOMO_TRY(e->configure());
       TOMO_TRY(e->reserve_outputs());
-      TOMO_TRY(e->reserve_batch(std::min(e->batch, e->nYPR), 4 * e->P.n_tri + 4096, e->nYPR > e->batch ? 2 : 1));
+      const int Bo = e->batch_size(std::min(e->batch, e->nYPR), mode);
+      TOMO_TRY(e->reserve_batch(mode, Bo, 4 * e->P.n_tri + 4096, e->nYPR > Bo ? 2 : 1));
     }
     return 0;
   }

@@ -1,24 +1,26 @@
 // B200 kernels of the orientation search (sm_100a).
 //
 // One batch of orientations runs as
-//   k_reset -> k_rotate -> k_bin_count -> k_bin_scan -> k_bin_fill -> k_strip
-//   -> k_bed, and k_fold on a second stream;
-// see the launch sequence in tomo_engine.cpp.  The work per orientation is the
+//   k_reset -> k_rotate -> k_raster -> k_strip -> k_bed, and k_fold on a
+//   second stream;
+// see the launch sequence in tomo_engine.cu.  The work per orientation is the
 // reference INT3 pipeline (Tomo_Shell2026.cpp thread_func:138-156):
 // Rotate -> Pixelize -> Pairing -> GenerateBed -> Calculate, re-organised so
 // that the per-column pixel lists never leave shared memory:
 //
-//  * the slot grid is cut into strips of H x-columns; triangles are binned
-//    per (orientation, strip) by their pixel bounding box (k_bin_*);
-//  * one CTA per (orientation, strip) rasterizes its triangles into
-//    per-column linked lists in shared memory, then runs the column stage
-//    (dedup, 63-pixel cap, sort, brief pairing, shadow casting) per column,
-//    reduces the column volumes to int64 and writes the non-zero column
-//    values in slot order for the float32 fold (k_strip);
-//  * the rare cases that a strip cannot resolve alone -- a hit whose slot
-//    lands in another strip, or a strip whose lists overflow shared memory --
-//    flag the orientation, which the host re-runs in "safe" mode (H = 1,
-//    every triangle pixel evaluated by every strip its extended box touches).
+//  * the slot grid is cut into strips of H x-columns; k_raster rasterizes
+//    every triangle once and appends its accepted pixels to their strips'
+//    lists in global memory;
+//  * one CTA per (orientation, strip) builds per-column linked lists of its
+//    pixels in shared memory, then runs the column stage (dedup, 63-pixel cap,
+//    sort, brief pairing, shadow casting) per column, reduces the column
+//    volumes to int64 and writes the column values in slot order for the
+//    float32 fold (k_strip);
+//  * an orientation whose strip lists overflow, or with a column past the
+//    63-pixel cap (where first-come order decides which pixels stay), is
+//    flagged and re-run by the host in a larger configuration, or in strips
+//    that rasterize their own triangles (binned per strip by their pixel
+//    boxes, k_bin_*) and carry each pixel's first-come priority.
 //
 // No kernel waits on another CTA; every shared and global index is checked.
 #include "tomo_common.cuh"
@@ -272,8 +274,9 @@ __global__ void k_reset(EngineParams p)
     if (o == 0) *p.foldxn = 0;
   }
   if (threadIdx.x < 4) p.minkey[o * 4 + threadIdx.x] = f2key(1e5f);  // STomoAABB3Df::Init
-  for (int s = threadIdx.x; s <= p.S; s += blockDim.x) p.bin_off[(size_t)o * (p.S + 1) + s] = 0;
-  for (int s = threadIdx.x; s < p.S; s += blockDim.x) { p.bin_cur[(size_t)o * p.S + s] = 0; p.foldcnt[(size_t)o * p.S + s] = 0; }
+  if (p.mode != 0)
+    for (int s = threadIdx.x; s <= p.S; s += blockDim.x) p.bin_off[(size_t)o * (p.S + 1) + s] = 0;
+  for (int s = threadIdx.x; s < p.S; s += blockDim.x) { if (p.mode == 0) p.ent_cnt[(size_t)o * p.S + s] = 0; else p.bin_cur[(size_t)o * p.S + s] = 0; p.foldcnt[(size_t)o * p.S + s] = 0; }
   for (int s = threadIdx.x; s < p.S * 8; s += blockDim.x) p.foldmeta[(size_t)o * p.S * 8 + s] = 0;
 }
 
@@ -490,6 +493,193 @@ __global__ void __launch_bounds__(256) k_bin_fill(EngineParams p)
       const int pos = off[s] + base[s] + atomicAdd(&lc[s], 1);
       if (pos < p.bin_cap) bins[pos] = t | ((r.code == 2) ? (int)0x80000000 : 0);
     }
+  }
+}
+
+// ---------------------------------------------------------------- K2 raster
+// Normal strips.  triVoxel (STomoSh_INT3.cpp:1138-1209) of every triangle,
+// each handled once: the accepted pixels are appended to the lists of their
+// strips in global memory (8 bytes each: (z, nz) key and slot in the strip),
+// from which k_strip builds its columns.
+//
+// One warp takes 32 / L triangles, L lanes each (L = 1 unless there are too
+// few triangles to fill the chip; then the lanes of a triangle share its
+// cells).  Per cell of 8 x 4 pixels a lane forms the mask of the pixels that
+// may pass the exact test (tomo_span.cuh); the set bits go to the warp's
+// queue, and 32 at a time every lane runs the reference's barycentric test on
+// one of them, so that the divisions, the double-precision u and the append
+// run on full warps.  A triangle whose box holds more than kLaneCells cells
+// per lane is finished by the whole warp, 32 cells at a time, so that a few
+// large triangles among small ones do not hold up a warp.  The warps of a
+// block share nothing: no barrier.
+//
+// Bound by instruction issue (8 bytes written per accepted pixel, 0.4 GB per
+// 256 orientations of the 82k solid: 0.3 TB/s).  Rasterizing in the strip
+// kernel instead loaded, set up and walked a triangle once per strip its box
+// touches (1.6 times on that mesh), needed a hit test while binning (so that a
+// triangle without a pixel falls back in one strip only) and ran between block
+// barriers: that whole sweep took 337 ms against 206 ms (B200, 82k solid,
+// 21,960 orientations; binning + strips 4.2 ms against raster + strips 2.4 ms
+// per 256 orientations), the 5k solid's 25.8 against 15.1 ms.
+constexpr int kRastWarps = 8;
+constexpr int kLaneCells = 8;
+
+struct RastWarp {
+  float4 q0[32], q1[32], q2[32];   // margined vertices, vertex-normal z
+  float4 q3[32];                   // d00, d01, d11, denom
+  unsigned org[32];                // first pixel of each lane's cell, x | y << 16
+  unsigned short q[32 * 32];       // candidates: lane of the cell << 5 | pixel in the cell
+};
+
+// Append the pixels of the calling lanes (`active`: all of them) to the lists
+// of their strips: one global atomic per strip and call, by the first lane of
+// each group of lanes with the same strip.
+__device__ __forceinline__ void append(const EngineParams& p, int o, unsigned active, int sx, int sy, unsigned key,
+                                       unsigned key2)
+{
+  const bool ok = (unsigned)sx < (unsigned)p.G && (unsigned)sy < (unsigned)p.G;
+  const int s = ok ? sx >> p.hshift : -1;
+  const unsigned peers = __match_any_sync(active, s);
+  const int lane = threadIdx.x & 31, leader = __ffs(peers) - 1;
+  const int per = p.twin ? 2 : 1;
+  int base = 0;
+  if (lane == leader && ok) base = atomicAdd(&p.ent_cnt[(size_t)o * p.S + s], per * __popc(peers));
+  base = __shfl_sync(active, base, leader);
+  if (!ok) { atomicOr(&p.flags[o], kFlagGrid); return; }
+  const int e = base + per * __popc(peers & ((1u << lane) - 1u));
+  if (e + per > p.ent_cap) { atomicOr(&p.flags[o], kFlagOverflow); return; }
+  const unsigned ls = (unsigned)((sx - (s << p.hshift)) * p.G + sy);
+  uint2* d = p.ents + ((size_t)o * p.S + s) * p.ent_cap + e;
+  d[0] = make_uint2(key, ls);
+  if (per == 2) d[1] = make_uint2(key2, ls);
+}
+
+__global__ void __launch_bounds__(32 * kRastWarps, 4) k_raster(EngineParams p)
+{
+  __shared__ RastWarp warps[kRastWarps];
+  const int o = blockIdx.y, lane = threadIdx.x & 31;
+  RastWarp& R = warps[threadIdx.x >> 5];
+  const int L = p.rast_lanes, sub = lane & (L - 1);
+  const int group = blockIdx.x * kRastWarps + (threadIdx.x >> 5);
+  const int t = group * (32 / L) + lane / L;
+  if (group * (32 / L) >= p.nT) return;   // warp-uniform
+  const Shift sh = load_shift(p, o);
+  const unsigned full = 0xFFFFFFFFu;
+
+  MaskTri T;
+  int own = lane & ~(L - 1);              // lane that holds this lane's triangle
+  int fb_x = 0, fb_y = 0;                 // centroid fallback pixel (STomoSh_INT3.cpp:1190-1206)
+  float fb_z = 0.f, n0 = 0.f;
+  unsigned hits = 0u;                     // lanes whose triangle has an accepted pixel (warp-uniform)
+  unsigned big = 0u;                      // triangles left to the whole warp
+  int tt = t, c = sub, step = L;          // cells c, c + step, ... of triangle tt
+  for (bool first = true;; first = false) {
+    int ncx = 0, ncell = 0;
+    if (tt < p.nT) {
+      TriGeo g;
+      float4 raw[3];
+      load_tri(p, o, tt, sh, g, raw);
+      if (g.x1 >= p.G) atomicOr(&p.flags[o], kFlagGrid);
+      Bary b;
+      bary_setup(g, b);
+      R.q0[own] = make_float4(g.ax, g.ay, g.az, g.n0);   // the same values from every lane of the triangle
+      R.q1[own] = make_float4(g.bx, g.by, g.bz, g.n1);
+      R.q2[own] = make_float4(g.cx, g.cy, g.cz, g.n2);
+      R.q3[own] = make_float4(b.d00, b.d01, b.d11, b.denom);
+      if (first) {
+        fb_x = __float2int_rz(centroid(__fsub_rn(raw[0].x, sh.dx), __fsub_rn(raw[1].x, sh.dx), __fsub_rn(raw[2].x, sh.dx)));
+        fb_y = __float2int_rz(centroid(__fsub_rn(raw[0].y, sh.dy), __fsub_rn(raw[1].y, sh.dy), __fsub_rn(raw[2].y, sh.dy)));
+        fb_z = centroid(__fsub_rn(raw[0].z, sh.dz), __fsub_rn(raw[1].z, sh.dz), __fsub_rn(raw[2].z, sh.dz));
+        n0 = g.n0;
+      }
+      if (b.ok) {
+        T = mask_setup(g.ax, g.ay, b.e0x, b.e0y, b.e1x, b.e1y, b.d00, b.d01, b.d11, b.denom,
+                       fminf(fminf(g.ax, g.bx), g.cx), fmaxf(fmaxf(g.ax, g.bx), g.cx), fminf(fminf(g.ay, g.by), g.cy),
+                       fmaxf(fmaxf(g.ay, g.by), g.cy), max(g.x0, 0), min(g.x1, p.G - 1), g.y0, g.y1, p.half);
+        if (T.nx > 0 && T.ny > 0) {
+          ncx = (T.nx + kCellX - 1) / kCellX;
+          ncell = ncx * ((T.ny + kCellY - 1) / kCellY);
+        }
+      }
+    }
+    int lim = ncell;
+    if (first) {
+      big = __ballot_sync(full, ncell > kLaneCells * L && sub == 0);
+      lim = min(ncell, kLaneCells * L);
+    }
+    const float rc = __frcp_rn((float)max(ncx, 1));
+    while (__any_sync(full, c < lim)) {
+      unsigned m = 0u;
+      if (c < lim) {
+        // c / ncx: at most 1,024 with ncx <= 512, so the float quotient of c + 1/2 truncates exactly
+        const int cj = __float2int_rz(((float)c + 0.5f) * rc), ci = c - cj * ncx;
+        m = mask_cell(T, ci, cj);
+        R.org[lane] = (unsigned)(T.x0 + kCellX * ci) | ((unsigned)(T.y0 + kCellY * cj) << 16);
+      }
+      c += step;
+      // queue the candidates in lane order
+      const int mine = __popc(m);
+      int at = mine;
+      for (int d = 1; d < 32; d <<= 1) {
+        const int y = __shfl_up_sync(full, at, d);
+        if (lane >= d) at += y;
+      }
+      const int n = __shfl_sync(full, at, 31);
+      at -= mine;
+      while (m) {
+        const int b = __clz(m);
+        m ^= 0x80000000u >> b;
+        R.q[at++] = (unsigned short)(lane << 5 | b);
+      }
+      __syncwarp();
+      for (int i = 0; i < n; i += 32) {
+        const bool valid = i + lane < n;
+        const unsigned item = valid ? R.q[i + lane] : 0u;
+        const int l = (int)(item >> 5), b = (int)(item & 31u);
+        const int w = first ? l & ~(L - 1) : own;
+        const unsigned org = R.org[l];
+        const int x = (int)(org & 0xFFFFu) + (b >> 2), y = (int)(org >> 16) + (b & 3);
+        const float4 A = R.q0[w], B = R.q1[w], C = R.q2[w], D = R.q3[w];
+        // _getBaryCoord (Tomo_types.cpp:86-115), the "+ 0*0" terms of _dot
+        // left out (they only turn -0 into +0, which changes no comparison
+        // and no stored value)
+        const float e0x = __fsub_rn(B.x, A.x), e0y = __fsub_rn(B.y, A.y);
+        const float e1x = __fsub_rn(C.x, A.x), e1y = __fsub_rn(C.y, A.y);
+        const float e2x = __fsub_rn(pix_center(x, p.half), A.x), e2y = __fsub_rn(pix_center(y, p.half), A.y);
+        const float d20 = __fadd_rn(__fmul_rn(e2x, e0x), __fmul_rn(e2y, e0y));
+        const float d21 = __fadd_rn(__fmul_rn(e2x, e1x), __fmul_rn(e2y, e1y));
+        const float v = __fdiv_rn(__fsub_rn(__fmul_rn(D.z, d20), __fmul_rn(D.y, d21)), D.w);
+        const float ww = __fdiv_rn(__fsub_rn(__fmul_rn(D.x, d21), __fmul_rn(D.y, d20)), D.w);
+        const float u = __double2float_rn(__dsub_rn(__dsub_rn(1.0, (double)v), (double)ww));
+        const bool hit = valid && (u >= -0.001f) && (v >= -0.001f) && (v <= p.vmax) && (__fadd_rn(u, v) <= p.vmax);
+        hits |= __reduce_or_sync(full, hit ? 1u << w : 0u);
+        const unsigned who = __ballot_sync(full, hit);
+        if (hit) {
+          const int sx = __float2int_rz(bary3(A.x, B.x, C.x, u, v, ww));
+          const int sy = __float2int_rz(bary3(A.y, B.y, C.y, u, v, ww));
+          const float fz = bary3(A.z, B.z, C.z, u, v, ww), fn = bary3(A.w, B.w, C.w, u, v, ww);
+          const float fz2 = __fadd_rn(fz, (fn >= 0.0f) ? -p.shell_off : p.shell_off);
+          append(p, o, who, sx, sy, make_key(to_i16(fz), to_i16(__fmul_rn(fn, 1000.0f))),
+                 make_key(to_i16(fz2), to_i16(__fmul_rn(-fn, 1000.0f))));
+        }
+      }
+      __syncwarp();
+    }
+    if (!big) break;
+    own = __ffs(big) - 1;
+    big &= big - 1;
+    tt = __shfl_sync(full, t, own);
+    c = kLaneCells * L + lane;
+    step = 32;
+    __syncwarp();
+  }
+  // centroid fallback of triangles without an accepted pixel, with the vertex-0 normal
+  const bool miss = t < p.nT && sub == 0 && !((hits >> lane) & 1u);
+  const unsigned who = __ballot_sync(full, miss);
+  if (miss) {
+    const float fz2 = __fadd_rn(fb_z, (n0 >= 0.0f) ? -p.shell_off : p.shell_off);
+    append(p, o, who, fb_x, fb_y, make_key(to_i16(fb_z), to_i16(__fmul_rn(n0, 1000.0f))),
+           make_key(to_i16(fz2), to_i16(__fmul_rn(-n0, 1000.0f))));
   }
 }
 
@@ -936,7 +1126,8 @@ __device__ __forceinline__ void emit(const EngineParams& p, const StripSmem& sm,
   if (e >= p.ent_cap) { atomicOr(sflag, MODE != 1 ? kFlagOverflow : kFlagSafeOverflow); return; }
   const int ls = (sx - xs0) * p.G + sy;
   sm.ekey[e] = make_key(z, nz);
-  if (MODE != 0) { sm.et[e] = t; sm.elo[e] = lo; }
+  sm.et[e] = t;
+  sm.elo[e] = lo;
   sm.enext[e] = (short)atomicExch(&sm.heads[ls], e);
 }
 
@@ -1080,11 +1271,17 @@ __global__ void __launch_bounds__(256, MODE == 0 ? 4 : 1) k_strip(EngineParams p
   sm.tkind = (uint8_t*)q; q += kChunk;
   sm.olist = (short*)chunk;
 
-  const int* off = p.bin_off + (size_t)o * (p.S + 1);
-  const int lbeg = off[s];
-  const int lend = min(off[s + 1], p.bin_cap);
-  const int nlist = max(lend - lbeg, 0);
-  const int* list = p.bins + (size_t)o * p.bin_cap + lbeg;
+  int nlist;
+  const int* list = nullptr;             // triangles of the strip (priority and safe strips)
+  if (MODE == 0) {
+    nlist = p.ent_cnt[(size_t)o * p.S + s];
+    if (nlist > C) return;               // k_raster flagged the orientation
+  } else {
+    const int* off = p.bin_off + (size_t)o * (p.S + 1);
+    const int lbeg = off[s];
+    nlist = max(min(off[s + 1], p.bin_cap) - lbeg, 0);
+    list = p.bins + (size_t)o * p.bin_cap + lbeg;
+  }
   uint8_t* bedf = p.bedf + (size_t)o * p.G * p.G + (size_t)xs0 * p.G;
 
   // bed flags of empty slots; occupied ones are overwritten in phase B
@@ -1100,6 +1297,15 @@ __global__ void __launch_bounds__(256, MODE == 0 ? 4 : 1) k_strip(EngineParams p
   if (threadIdx.x == 0) { nent = 0; sflag = 0; }
   __syncthreads();
 
+  if constexpr (MODE == 0) {
+  // ---- phase A: the strip's accepted pixels (k_raster) into per-column lists
+    const uint2* ents = p.ents + ((size_t)o * p.S + s) * C;
+    for (int i = threadIdx.x; i < nlist; i += blockDim.x) {
+      const uint2 e = __ldcs(ents + i);
+      sm.ekey[i] = e.x;
+      sm.enext[i] = (short)atomicExch(&sm.heads[e.y], i);
+    }
+  } else {
   const Shift sh = load_shift(p, o);
   const float half = p.half, vmax = p.vmax;
 
@@ -1118,9 +1324,8 @@ __global__ void __launch_bounds__(256, MODE == 0 ? 4 : 1) k_strip(EngineParams p
     if (!fb) return;
     const float n0 = sm.q0[i].w;
     const int tx = sm.tm[i].x;
-    const unsigned t = MODE == 0 ? 0u : (unsigned)tx;   // the priority is only read by priority strips
-    const int xy = MODE == 0 ? tx : fb_xy;
-    const int sx = (int)(short)(xy & 0xFFFF), sy = xy >> 16;
+    const unsigned t = (unsigned)tx;
+    const int sx = (int)(short)(fb_xy & 0xFFFF), sy = fb_xy >> 16;
     const float fb_z = sm.fbz[i];
     emit<MODE>(p, sm, &nent, &sflag, xs0, xs1, sx, sy, to_i16(fb_z), to_i16(__fmul_rn(n0, 1000.0f)), t, 0u);
     if (p.twin) {
@@ -1168,7 +1373,7 @@ __global__ void __launch_bounds__(256, MODE == 0 ? 4 : 1) k_strip(EngineParams p
       sm.q0[i] = make_float4(g.ax, g.ay, g.az, g.n0);
       sm.q1[i] = make_float4(g.bx, g.by, g.bz, g.n1);
       sm.q2[i] = make_float4(g.cx, g.cy, g.cz, g.n2);
-      sm.tm[i] = make_int4(MODE == 0 ? fb_xy : t, g.x0, g.y0, ylen);
+      sm.tm[i] = make_int4(t, g.x0, g.y0, ylen);
       sm.tkind[i] = (uint8_t)(fb_only | (single << 1));
     }
     if (i < kChunk / 32) sm.thit[i] = 0u;
@@ -1267,6 +1472,7 @@ __global__ void __launch_bounds__(256, MODE == 0 ? 4 : 1) k_strip(EngineParams p
     prev_n = nchunk;
   }
   if (prev_n) fallback(prev_n, thit_base + ((chunk_no + 1) & 1) * (kChunk / 32));
+  }
   __syncthreads();
 
   // ---- occupied slots in slot order (bitmap from the list heads -> list)
@@ -1768,22 +1974,40 @@ static dim3 tri_grid(const EngineParams& p)
   return dim3(b > 0 ? b : 1, p.Bo);
 }
 
-// Count pass of one batch (reset, rotate, bin count, bin scan).
+// Lanes per triangle in k_raster: one, unless that gives fewer warps than
+// kRastFill; then the lanes of a triangle share its cells.
+constexpr int kRastFill = 148 * 16;
+
+int raster_lanes(int nT, int Bo)
+{
+  int L = 1;
+  while (L < 32 && (long long)Bo * ((nT + 32 / L - 1) / (32 / L)) < kRastFill) L *= 2;
+  return L;
+}
+
+// Rotation and, for priority and safe strips, the triangle bins' count pass.
 cudaError_t launch_bin_count(const EngineParams& p, cudaStream_t main, LaunchLog* L)
 {
   TOMO_LAUNCH(kKReset, main, (k_reset<<<p.Bo, 256, 0, main>>>(p)));
   TOMO_LAUNCH(kKRotate, main,
               (k_rotate<<<dim3((p.nV + 255) / 256 > 0 ? (p.nV + 255) / 256 : 1, (p.Bo + kRotGroup - 1) / kRotGroup), 256,
                            0, main>>>(p)));
+  if (p.mode == 0) return cudaGetLastError();
   TOMO_LAUNCH(kKCount, main, (k_bin_count<<<tri_grid(p), 256, sizeof(int) * p.S, main>>>(p)));
   TOMO_LAUNCH(kKScan, main, (k_bin_scan<<<p.Bo, 1024, 0, main>>>(p)));
   return cudaGetLastError();
 }
 
-// The binning half of a batch after its count pass (bin fill).
+// The binning half of a batch after that: normal strips' pixel lists, or the
+// fill pass of the triangle bins.
 cudaError_t launch_fill(const EngineParams& p, cudaStream_t s, LaunchLog* L)
 {
-  TOMO_LAUNCH(kKFill, s, (k_bin_fill<<<tri_grid(p), 256, 2 * sizeof(int) * p.S, s>>>(p)));
+  if (p.mode == 0) {
+    const int per_block = kRastWarps * (32 / p.rast_lanes);
+    TOMO_LAUNCH(kKRaster, s, (k_raster<<<dim3((p.nT + per_block - 1) / per_block, p.Bo), 32 * kRastWarps, 0, s>>>(p)));
+  } else {
+    TOMO_LAUNCH(kKFill, s, (k_bin_fill<<<tri_grid(p), 256, 2 * sizeof(int) * p.S, s>>>(p)));
+  }
   return cudaGetLastError();
 }
 
@@ -1798,23 +2022,17 @@ cudaError_t launch_strip_bed(const EngineParams& p, cudaStream_t main, size_t st
   return cudaGetLastError();
 }
 
-// Remainder of a batch after launch_bin_count (bin fill, strips, bed).
+// Remainder of a batch after launch_bin_count.
 cudaError_t launch_after_count(const EngineParams& p, cudaStream_t main, size_t strip_smem, LaunchLog* L)
 {
-  TOMO_LAUNCH(kKFill, main, (k_bin_fill<<<tri_grid(p), 256, 2 * sizeof(int) * p.S, main>>>(p)));
-  const int kind = p.variant == 0 ? kKStrip : kKStripRedo;
-  if (p.mode == 0) TOMO_LAUNCH(kind, main, (k_strip<0><<<dim3(p.S, p.Bo), 256, strip_smem, main>>>(p)));
-  else if (p.mode == 2) TOMO_LAUNCH(kind, main, (k_strip<2><<<dim3(p.S, p.Bo), 256, strip_smem, main>>>(p)));
-  else TOMO_LAUNCH(kind, main, (k_strip<1><<<dim3(p.S, p.Bo), 256, strip_smem, main>>>(p)));
-  TOMO_LAUNCH(kKBed, main, (k_bed<<<dim3(8, p.Bo), 256, 0, main>>>(p)));
-  return cudaGetLastError();
+  const cudaError_t e = launch_fill(p, main, L);
+  return e != cudaSuccess ? e : launch_strip_bed(p, main, strip_smem, L);
 }
 
 cudaError_t launch_batch(const EngineParams& p, cudaStream_t main, size_t strip_smem, LaunchLog* L)
 {
-  cudaError_t e = launch_bin_count(p, main, L);
-  if (e != cudaSuccess) return e;
-  return launch_after_count(p, main, strip_smem, L);
+  const cudaError_t e = launch_bin_count(p, main, L);
+  return e != cudaSuccess ? e : launch_after_count(p, main, strip_smem, L);
 }
 
 cudaError_t launch_dump_scan(const int* cols8, int GG, int* off, int* totals, cudaStream_t s)

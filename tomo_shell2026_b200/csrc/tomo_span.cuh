@@ -153,4 +153,140 @@ TOMO_HD void span_rows(const SpanTri& T, float px, int y0, int ylen, int& lo, in
   hi = (int)h;
 }
 
+// ------------------------------------------------------------ candidate masks
+//
+// The rasterizer (k_raster) tests a triangle's pixels in cells of 8 columns
+// x 4 rows, one bit per pixel, with three affine functions per pixel (no
+// divisions, no reference arithmetic): a set bit means "may pass the exact
+// test", and every pixel the exact test accepts has its bit set.
+//
+//   V = s * vn + bound, W = s * wn + bound, U = bound - s * (vn + wn)
+//
+// are affine in the pixel's column and row; a pixel is a candidate when all
+// three are >= 0.  vn, wn are the barycentric numerators above and the bounds
+// are the pre-reject's (0.002, 1.003 of |denom|, twice the exact test's
+// margins) widened by every rounding, in units of the numerators:
+//   * the exact test's float numerators against the linear form, the float
+//     coefficients, and the evaluation below (at most nine roundings of values
+//     below S per function): less than 2^-19 S together; 2^-17 S is added
+//     (S as in span_setup);
+//   * a pixel centre ((x + 0.001f) + half) - ax is formed in float by the
+//     reference with three roundings, each within 2^-24 of a value below
+//     M = |x| + |half| + |ax| + 2, here for the cell grid's first pixel only
+//     and then stepped by whole numbers: they differ by less than 2^-21 M, and
+//     the functions are widened by slope x 2^-20 M.
+// Only the pixels whose centres lie within the triangle's bounding box widened
+// by d are looked at: with the roundings above at most 0.004 |denom| (else the
+// whole pixel box is used), an accepted pixel has v, w >= -0.0051 and
+// u >= -0.0102, so its centre is within 0.0205 of the box's extent;
+// d = 0.025 extent + 2^-19 M + 0.001.
+struct MaskTri {
+  float pv, pw, pu;        // change per column of V, W, U
+  float bv, bw, bu;        // change per row
+  float v0, w0, u0;        // values at pixel (x0, y0)
+  int x0, y0, nx, ny;      // pixels to look at: nx columns from x0, ny rows from y0
+};
+
+constexpr int kCellX = 8, kCellY = 4;
+
+TOMO_HD int ceil_int(float f)
+{
+#ifdef __CUDA_ARCH__
+  return __float2int_ru(f);
+#else
+  return (int)ceilf(f);
+#endif
+}
+TOMO_HD int floor_int(float f)
+{
+#ifdef __CUDA_ARCH__
+  return __float2int_rd(f);
+#else
+  return (int)floorf(f);
+#endif
+}
+
+// e0*, e1*, d00, d01, d11, denom: the float barycentric setup; x0..x1, y0..y1
+// the pixel box; minx..maxy the float bounding box it was truncated from.
+TOMO_HD MaskTri mask_setup(float ax, float ay, float e0x, float e0y, float e1x, float e1y, float d00, float d01,
+                           float d11, float denom, float minx, float maxx, float miny, float maxy, int x0, int x1,
+                           int y0, int y1, float half)
+{
+  MaskTri T;
+  const float ad = fabsf(denom), ah = fabsf(half);
+  const float sgn = denom > 0.0f ? 1.0f : -1.0f;
+  T.pv = sgn * fmaf(d11, e0x, -(d01 * e1x));
+  T.bv = sgn * fmaf(d11, e0y, -(d01 * e1y));
+  T.pw = sgn * fmaf(d00, e1x, -(d01 * e0x));
+  T.bw = sgn * fmaf(d00, e1y, -(d01 * e0y));
+  T.pu = -(T.pv + T.pw);
+  T.bu = -(T.bv + T.bw);
+  const float extx = maxx - minx, exty = maxy - miny;
+  const float mx = extx + (2.0f + ah), my = exty + (2.0f + ah);
+  const float s0 = fmaf(mx, fabsf(e0x), my * fabsf(e0y)), s1 = fmaf(mx, fabsf(e1x), my * fabsf(e1y));
+  const float k = 1.0f / 131072.0f;   // 2^-17
+  const float a01 = fabsf(d01);
+  const float ev = k * fmaf(d11, s0, a01 * s1), ew = k * fmaf(d00, s1, a01 * s0);
+  const float posx = fabsf(maxx) + fabsf(minx) + (2.0f + ah), posy = fabsf(maxy) + fabsf(miny) + (2.0f + ah);
+  const float ex = posx * (1.0f / 1048576.0f), ey = posy * (1.0f / 1048576.0f);   // 2^-20 M
+  T.x0 = x0; T.y0 = y0; T.nx = x1 - x0 + 1; T.ny = y1 - y0 + 1;
+  if (ev + ew <= 0.004f * ad) {
+    const float dx = fmaf(0.025f, extx, fmaf(2.0f, ex, 0.001f)), dy = fmaf(0.025f, exty, fmaf(2.0f, ey, 0.001f));
+    const float c = 0.001f + half;
+    const int cx0 = ceil_int((minx - dx) - c), cx1 = floor_int((maxx + dx) - c);
+    const int cy0 = ceil_int((miny - dy) - c), cy1 = floor_int((maxy + dy) - c);
+    T.x0 = cx0 > x0 ? cx0 : x0; T.y0 = cy0 > y0 ? cy0 : y0;
+    T.nx = (cx1 < x1 ? cx1 : x1) - T.x0 + 1; T.ny = (cy1 < y1 ? cy1 : y1) - T.y0 + 1;
+  }
+  const float cx = (((float)T.x0 + 0.001f) + half) - ax, cy = (((float)T.y0 + 0.001f) + half) - ay;
+  const float lv = fmaf(0.002f, ad, ev) + fmaf(fabsf(T.pv), ex, fabsf(T.bv) * ey);
+  const float lw = fmaf(0.002f, ad, ew) + fmaf(fabsf(T.pw), ex, fabsf(T.bw) * ey);
+  const float lu = fmaf(1.003f, ad, ev + ew) + fmaf(fabsf(T.pu), ex, fabsf(T.bu) * ey) + k * ad;
+  T.v0 = fmaf(T.pv, cx, fmaf(T.bv, cy, lv));
+  T.w0 = fmaf(T.pw, cx, fmaf(T.bw, cy, lw));
+  T.u0 = fmaf(T.pu, cx, fmaf(T.bu, cy, lu));
+  return T;
+}
+
+TOMO_HD unsigned sign_word(float a, float b, float c)
+{
+#ifdef __CUDA_ARCH__
+  return __float_as_uint(a) | __float_as_uint(b) | __float_as_uint(c);
+#else
+  return (signbit(a) || signbit(b) || signbit(c)) ? 0x80000000u : 0u;
+#endif
+}
+TOMO_HD unsigned shift_in_sign(unsigned m, unsigned word)
+{
+#ifdef __CUDA_ARCH__
+  return __funnelshift_l(word, m, 1);
+#else
+  return (m << 1) | (word >> 31);
+#endif
+}
+
+// Candidate mask of cell (ci, cj): columns 8 ci .. 8 ci + 7 and rows
+// 4 cj .. 4 cj + 3 of the triangle's pixel grid; bit 31 - (4 * column + row)
+// of the cell.
+TOMO_HD unsigned mask_cell(const MaskTri& T, int ci, int cj)
+{
+  const int nc = T.nx - kCellX * ci, nr = T.ny - kCellY * cj;
+  const int ncol = nc < kCellX ? nc : kCellX;
+  const float fx = (float)(kCellX * ci), fy = (float)(kCellY * cj);
+  float v = fmaf(T.bv, fy, fmaf(T.pv, fx, T.v0));
+  float w = fmaf(T.bw, fy, fmaf(T.pw, fx, T.w0));
+  float u = fmaf(T.bu, fy, fmaf(T.pu, fx, T.u0));
+  unsigned m = 0u;
+  for (int j = 0; j < ncol; j++) {
+    m = shift_in_sign(m, sign_word(v, w, u));
+    m = shift_in_sign(m, sign_word(v + T.bv, w + T.bw, u + T.bu));
+    m = shift_in_sign(m, sign_word(fmaf(T.bv, 2.0f, v), fmaf(T.bw, 2.0f, w), fmaf(T.bu, 2.0f, u)));
+    m = shift_in_sign(m, sign_word(fmaf(T.bv, 3.0f, v), fmaf(T.bw, 3.0f, w), fmaf(T.bu, 3.0f, u)));
+    v += T.pv; w += T.pw; u += T.pu;
+  }
+  // m holds a sign bit (1 = rejected) per pixel, the first column uppermost
+  const unsigned keep = nr >= kCellY ? 0xFFFFFFFFu : 0x11111111u * ((0xFu << (kCellY - nr)) & 0xFu);
+  return ncol <= 0 ? 0u : (~m << (32 - 4 * ncol)) & keep;
+}
+
 }  // namespace tomo

@@ -135,7 +135,7 @@ def vol_to_mass(f32info, i32info, vm22) -> np.ndarray:
 
 
 KERNEL_KINDS = ("k_reset", "k_rotate", "k_bin_count", "k_bin_scan", "k_bin_fill", "k_strip", "k_bed", "k_fold",
-                "k_strip_redo")
+                "k_strip_redo", "k_raster")
 
 
 def profile(enable: bool, reset: bool = True) -> None:
