@@ -110,7 +110,7 @@ struct EngineParams {
   uint2* ents;          // [Bo][S][ent_cap] (z, nz) key; slot within the strip
   int* ent_cnt;         // [Bo][S] pixels appended (may exceed ent_cap: the strip overflowed)
   int hshift;           // log2(H)
-  int rast_lanes;       // lanes per triangle in k_raster (a power of two)
+  int rast_shift;       // log2(lanes per triangle) in k_raster
 
   // per-batch results
   long long* acc;       // [Bo][kAccLanes]

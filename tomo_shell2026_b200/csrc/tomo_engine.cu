@@ -31,7 +31,7 @@ namespace tomo {
 
 size_t strip_smem_bytes(int mode, int H, int G, int ent_cap);
 size_t strip_four_per_sm_budget();
-int raster_lanes(int nT, int Bo);
+int raster_lanes_log2(int nT, int Bo);
 cudaError_t configure_kernels(size_t normal_smem, size_t safe_smem, size_t prio_smem);
 cudaError_t launch_batch(const EngineParams& p, cudaStream_t main, size_t strip_smem, LaunchLog* L);
 cudaError_t launch_fold(const EngineParams& p, cudaStream_t side, LaunchLog* L);
@@ -605,7 +605,7 @@ struct Engine {
     p.ori = ori.ptr + first;
     p.xf = b.xf.ptr; p.minkey = b.minkey.ptr; p.trange = b.trange.ptr;
     p.bin_off = b.bin_off.ptr; p.bin_cur = b.bin_cur.ptr; p.bins = b.bins.ptr; p.bin_cap = bin_cap;
-    p.ents = b.ents.ptr; p.ent_cnt = b.ent_cnt.ptr; p.rast_lanes = raster_lanes(p.nT, Bo);
+    p.ents = b.ents.ptr; p.ent_cnt = b.ent_cnt.ptr; p.rast_shift = raster_lanes_log2(p.nT, Bo);
     p.bbox = b.bbox.ptr; p.bedf = b.bedf.ptr;
     p.acc = set[which].acc.ptr; p.flags = set[which].flags.ptr;
     p.foldcnt = set[which].foldcnt.ptr; p.foldp = set[which].foldp.ptr; p.foldmeta = set[which].foldmeta.ptr;
@@ -1734,7 +1734,7 @@ void static_bind(EngineParams& p, const StaticLayout& L, int nb, int slot, int b
   p.ori = L.ori + slot; p.Bo = nb;
   p.xf = L.xf; p.minkey = L.minkey; p.trange = L.trange;
   p.bin_off = L.bin_off; p.bin_cur = L.bin_cur; p.bins = L.bins; p.bin_cap = bin_cap;
-  p.ents = L.ents; p.ent_cnt = L.ent_cnt; p.rast_lanes = raster_lanes(p.nT, nb);
+  p.ents = L.ents; p.ent_cnt = L.ent_cnt; p.rast_shift = raster_lanes_log2(p.nT, nb);
   if (p.mode == 0)   // a list shorter than the strip's shared memory only flags overflow earlier
     p.ent_cap = (int)std::min<size_t>(p.ent_cap, kStaticListBytes / ((size_t)nb * p.S * sizeof(uint2)));
   p.acc = L.acc; p.flags = L.flags; p.bbox = L.bbox; p.bedf = L.bedf;

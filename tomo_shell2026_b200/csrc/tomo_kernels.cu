@@ -26,7 +26,9 @@
 #include "tomo_common.cuh"
 #include "tomo_span.cuh"
 
+#include <algorithm>
 #include <climits>
+
 
 namespace tomo {
 
@@ -511,176 +513,293 @@ __global__ void __launch_bounds__(256) k_bin_fill(EngineParams p)
 // run on full warps.  A triangle whose box holds more than kLaneCells cells
 // per lane is finished by the whole warp, 32 cells at a time, so that a few
 // large triangles among small ones do not hold up a warp.  The warps of a
-// block share nothing: no barrier.
+// block share nothing: no barrier.  Accepted pixels collect in the warp's stash
+// and are appended in full rounds of 32, and consecutive blocks belong to
+// different orientations: with appends straight from the exact test and whole
+// orientations in turn the strip counters' atomics were waited for (1.33 ms
+// per 256 orientations of the 82k solid; orientations mixed 1.15, with the
+// cheaper masks, the stash and several groups per warp 0.95).  Blocks of four
+// warps, seven to an SM: the 72 registers the loop needs (64 spill: 0.96 ms at
+// 32 warps; 80 without spills at 24 warps: 1.01).
 //
-// Bound by instruction issue (8 bytes written per accepted pixel, 0.4 GB per
-// 256 orientations of the 82k solid: 0.3 TB/s).  Rasterizing in the strip
+// Bound by instruction issue (80 % of cycles; 8 bytes written per accepted
+// pixel, 0.4 GB per 256 orientations of the 82k solid: 0.4 TB/s).  Rasterizing in the strip
 // kernel instead loaded, set up and walked a triangle once per strip its box
 // touches (1.6 times on that mesh), needed a hit test while binning (so that a
 // triangle without a pixel falls back in one strip only) and ran between block
 // barriers: that whole sweep took 337 ms against 206 ms (B200, 82k solid,
 // 21,960 orientations; binning + strips 4.2 ms against raster + strips 2.4 ms
-// per 256 orientations), the 5k solid's 25.8 against 15.1 ms.
-constexpr int kRastWarps = 8;
+// per 256 orientations, with the first version of this kernel), the 5k solid's
+// 25.8 against 15.1 ms.
+constexpr int kRastWarps = 4;
+constexpr int kRastGroups = 4;  // groups of triangles a warp takes in turn
+constexpr int kRastMix = 16;   // orientations whose blocks run side by side
 constexpr int kLaneCells = 8;
+constexpr int kStash = 128;
 
 struct RastWarp {
   float4 q0[32], q1[32], q2[32];   // margined vertices, vertex-normal z
   float4 q3[32];                   // d00, d01, d11, denom
   unsigned org[32];                // first pixel of each lane's cell, x | y << 16
+  uint2 st[kStash];                // accepted pixels: key, slot x | y << 16 (0xFFFFFFFF: outside the grid)
+  unsigned st2[kStash];            // their shell twins' keys
   unsigned short q[32 * 32];       // candidates: lane of the cell << 5 | pixel in the cell
 };
 
-// Append the pixels of the calling lanes (`active`: all of them) to the lists
-// of their strips: one global atomic per strip and call, by the first lane of
-// each group of lanes with the same strip.
-__device__ __forceinline__ void append(const EngineParams& p, int o, unsigned active, int sx, int sy, unsigned key,
-                                       unsigned key2)
+// Two single-precision operations in one instruction, each rounded to nearest
+// as __fadd_rn / __fmul_rn round it.  The assembler fuses a packed product into
+// a packed sum that takes it (one rounding, other bits), so a mul2 result goes
+// to scalar sums only.
+struct F2 { float x, y; };
+__device__ __forceinline__ F2 add2(F2 a, F2 b)
 {
-  const bool ok = (unsigned)sx < (unsigned)p.G && (unsigned)sy < (unsigned)p.G;
-  const int s = ok ? sx >> p.hshift : -1;
-  const unsigned peers = __match_any_sync(active, s);
-  const int lane = threadIdx.x & 31, leader = __ffs(peers) - 1;
-  const int per = p.twin ? 2 : 1;
-  int base = 0;
-  if (lane == leader && ok) base = atomicAdd(&p.ent_cnt[(size_t)o * p.S + s], per * __popc(peers));
-  base = __shfl_sync(active, base, leader);
-  if (!ok) { atomicOr(&p.flags[o], kFlagGrid); return; }
-  const int e = base + per * __popc(peers & ((1u << lane) - 1u));
-  if (e + per > p.ent_cap) { atomicOr(&p.flags[o], kFlagOverflow); return; }
-  const unsigned ls = (unsigned)((sx - (s << p.hshift)) * p.G + sy);
-  uint2* d = p.ents + ((size_t)o * p.S + s) * p.ent_cap + e;
-  d[0] = make_uint2(key, ls);
-  if (per == 2) d[1] = make_uint2(key2, ls);
+  F2 r;
+  asm("{.reg .b64 a, b, r;\n\tmov.b64 a, {%2, %3};\n\tmov.b64 b, {%4, %5};\n\tadd.rn.f32x2 r, a, b;\n\tmov.b64 {%0, %1}, r;}"
+      : "=f"(r.x), "=f"(r.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return r;
+}
+__device__ __forceinline__ F2 mul2(F2 a, F2 b)
+{
+  F2 r;
+  asm("{.reg .b64 a, b, r;\n\tmov.b64 a, {%2, %3};\n\tmov.b64 b, {%4, %5};\n\tmul.rn.f32x2 r, a, b;\n\tmov.b64 {%0, %1}, r;}"
+      : "=f"(r.x), "=f"(r.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return r;
+}
+// b - a
+__device__ __forceinline__ F2 sub2(F2 b, F2 a)
+{
+  F2 r;
+  asm("{.reg .b64 a, b, m, r;\n\tmov.b64 a, {%2, %3};\n\tmov.b64 b, {%4, %5};\n\tmov.b64 m, {%6, %6};\n\tfma.rn.f32x2 r, a, m, b;\n\tmov.b64 {%0, %1}, r;}"
+      : "=f"(r.x), "=f"(r.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(-1.0f));
+  return r;
+}
+// bary3 of two components at once
+__device__ __forceinline__ F2 bary3x2(F2 a, F2 b, F2 c, float u, float v, float w)
+{
+  const F2 x = mul2(a, F2{u, u}), y = mul2(b, F2{v, v}), z = mul2(c, F2{w, w});
+  return F2{__fadd_rn(__fadd_rn(x.x, y.x), z.x), __fadd_rn(__fadd_rn(x.y, y.y), z.y)};
 }
 
-__global__ void __launch_bounds__(32 * kRastWarps, 4) k_raster(EngineParams p)
+// make_key of (int16)z and (int16)nz: both halves wrap, then shift by 32768.
+__device__ __forceinline__ unsigned pixel_key(float z, float n)
+{
+  return __byte_perm(__float2int_rz(__fmul_rn(n, 1000.0f)), __float2int_rz(z), 0x5410) ^ 0x80008000u;
+}
+
+// Slot of an accepted pixel, packed; outside the grid: 0xFFFFFFFF.
+__device__ __forceinline__ unsigned slot_xy(const EngineParams& p, float fx, float fy)
+{
+  const int sx = __float2int_rz(fx), sy = __float2int_rz(fy);
+  return max((unsigned)sx, (unsigned)sy) < (unsigned)p.G ? (unsigned)sx | (unsigned)sy << 16 : 0xFFFFFFFFu;
+}
+
+// Append the warp's first n stashed pixels (at most 32 kRounds) to the lists of
+// their strips: one global atomic per 32 pixels and strip, all issued before
+// the first is waited for.
+template <bool kTwin, int kRounds>
+__device__ __forceinline__ void flush(const EngineParams& p, int o, const RastWarp& R, int n)
+{
+  const unsigned full = 0xFFFFFFFFu;
+  const int lane = threadIdx.x & 31;
+  const unsigned below = (1u << lane) - 1u;
+  constexpr int per = kTwin ? 2 : 1;
+  int base[kRounds];
+  unsigned peers[kRounds], xy[kRounds];
+  const int strip0 = o * p.S;
+#pragma unroll
+  for (int r = 0; r < kRounds; r++) {
+    base[r] = 0; peers[r] = 0; xy[r] = 0xFFFFFFFFu;
+    if (32 * r >= n) continue;   // warp-uniform
+    if (32 * r + lane < n) xy[r] = R.st[32 * r + lane].y;
+    const int s = (int)(xy[r] & 0xFFFFu) >> p.hshift;   // no pixel: a strip past the last
+    peers[r] = __match_any_sync(full, s);
+    if ((peers[r] & below) == 0u && xy[r] != 0xFFFFFFFFu) base[r] = atomicAdd(p.ent_cnt + strip0 + s, per * __popc(peers[r]));
+  }
+#pragma unroll
+  for (int r = 0; r < kRounds; r++) {
+    if (32 * r >= n) continue;
+    const int at = __shfl_sync(full, base[r], __ffs(peers[r]) - 1) + per * __popc(peers[r] & below);
+    const bool fits = xy[r] != 0xFFFFFFFFu && at + per <= p.ent_cap;
+    if (fits) {
+      const int sx = (int)(xy[r] & 0xFFFFu);
+      const unsigned ls = (unsigned)((sx & ((1 << p.hshift) - 1)) * p.G) + (xy[r] >> 16);
+      uint2* d = p.ents + ((size_t)(unsigned)(strip0 + (sx >> p.hshift)) * (unsigned)p.ent_cap + (unsigned)at);
+      d[0] = make_uint2(R.st[32 * r + lane].x, ls);
+      if (kTwin) d[1] = make_uint2(R.st2[32 * r + lane], ls);
+    } else if (32 * r + lane < n) {
+      atomicOr(&p.flags[o], xy[r] == 0xFFFFFFFFu ? kFlagGrid : kFlagOverflow);
+    }
+  }
+}
+
+template <bool kTwin>
+__global__ void __launch_bounds__(32 * kRastWarps, 7) k_raster(EngineParams p)
 {
   __shared__ RastWarp warps[kRastWarps];
-  const int o = blockIdx.y, lane = threadIdx.x & 31;
+  // consecutive blocks take the same triangles of kRastMix orientations: the
+  // atomics in flight spread over their strip counters while their rotated
+  // vertices stay in L2
+  const int o = blockIdx.z * kRastMix + blockIdx.x, lane = threadIdx.x & 31;
+  if (o >= p.Bo) return;
   RastWarp& R = warps[threadIdx.x >> 5];
-  const int L = p.rast_lanes, sub = lane & (L - 1);
-  const int group = blockIdx.x * kRastWarps + (threadIdx.x >> 5);
-  const int t = group * (32 / L) + lane / L;
-  if (group * (32 / L) >= p.nT) return;   // warp-uniform
-  const Shift sh = load_shift(p, o);
+  const int lsh = p.rast_shift, L = 1 << lsh, sub = lane & (L - 1);
+  const int gshift = 5 - lsh;             // log2(triangles per warp)
+  const int ngroup = (p.nT + (1 << gshift) - 1) >> gshift;
   const unsigned full = 0xFFFFFFFFu;
+  const unsigned below = (1u << lane) - 1u;
+  const Shift sh = load_shift(p, o);
+  const float4* const X = p.xf + (size_t)o * p.nV;
+  int ns = 0;                             // stashed pixels (warp-uniform)
+  auto room = [&]() {                     // for 32 more
+    if (ns + 32 <= kStash) return;
+    __syncwarp();
+    flush<kTwin, kStash / 32 - 1>(p, o, R, ns);
+    const int rest = max(ns - (kStash - 32), 0);
+    uint2 e;
+    unsigned e2 = 0u;
+    if (lane < rest) { e = R.st[kStash - 32 + lane]; if (kTwin) e2 = R.st2[kStash - 32 + lane]; }
+    __syncwarp();
+    if (lane < rest) { R.st[lane] = e; if (kTwin) R.st2[lane] = e2; }
+    ns = rest;
+    __syncwarp();
+  };
 
-  MaskTri T;
-  int own = lane & ~(L - 1);              // lane that holds this lane's triangle
-  int fb_x = 0, fb_y = 0;                 // centroid fallback pixel (STomoSh_INT3.cpp:1190-1206)
-  float fb_z = 0.f, n0 = 0.f;
-  unsigned hits = 0u;                     // lanes whose triangle has an accepted pixel (warp-uniform)
-  unsigned big = 0u;                      // triangles left to the whole warp
-  int tt = t, c = sub, step = L;          // cells c, c + step, ... of triangle tt
-  for (bool first = true;; first = false) {
-    int ncx = 0, ncell = 0;
-    if (tt < p.nT) {
-      TriGeo g;
-      float4 raw[3];
-      load_tri(p, o, tt, sh, g, raw);
-      if (g.x1 >= p.G) atomicOr(&p.flags[o], kFlagGrid);
-      Bary b;
-      bary_setup(g, b);
-      R.q0[own] = make_float4(g.ax, g.ay, g.az, g.n0);   // the same values from every lane of the triangle
-      R.q1[own] = make_float4(g.bx, g.by, g.bz, g.n1);
-      R.q2[own] = make_float4(g.cx, g.cy, g.cz, g.n2);
-      R.q3[own] = make_float4(b.d00, b.d01, b.d11, b.denom);
+  for (int group = blockIdx.y * kRastWarps + (threadIdx.x >> 5); group < ngroup; group += gridDim.y * kRastWarps) {
+    const int t = (group << gshift) + (lane >> lsh);
+    MaskTri T;
+    int own = lane & ~(L - 1);            // lane that holds this lane's triangle
+    float fbx = 0.f, fby = 0.f, fbz = 0.f, n0 = 0.f;   // centroid fallback (STomoSh_INT3.cpp:1190-1206)
+    unsigned hits = 0u;                   // lanes whose triangle has an accepted pixel (warp-uniform)
+    unsigned big = 0u;                    // triangles left to the whole warp
+    int tt = t, c = sub, step = L;        // cells c, c + step, ... of triangle tt
+    for (bool first = true;; first = false) {
+      int ncx = 0, ncell = 0;
+      if (tt < p.nT) {
+        const int4 ix = p.tri[tt];
+        const float4 A = X[ix.x], B = X[ix.y], C = X[ix.z];
+        // load_tri's translation and margin, two coordinates at a time (the
+        // normal's z rides along unchanged)
+        const F2 sxy = {-sh.dx, -sh.dy}, sz = {-sh.dz, -0.0f}, mxy = {0.001f, 0.001f}, mz = {0.001f, -0.0f};
+        const F2 ua = add2(F2{A.x, A.y}, sxy), ub = add2(F2{B.x, B.y}, sxy), uc = add2(F2{C.x, C.y}, sxy);
+        const F2 va = add2(F2{A.z, A.w}, sz), vb = add2(F2{B.z, B.w}, sz), vc = add2(F2{C.z, C.w}, sz);
+        const F2 a = add2(ua, mxy), b = add2(ub, mxy), cc = add2(uc, mxy);
+        const F2 az = add2(va, mz), bz = add2(vb, mz), cz = add2(vc, mz);
+        const F2 e0 = sub2(b, a), e1 = sub2(cc, a);
+        // _getBaryCoord's constants (Tomo_types.cpp:86-101)
+        const float d00 = __fadd_rn(__fmul_rn(e0.x, e0.x), __fmul_rn(e0.y, e0.y));
+        const float d01 = __fadd_rn(__fmul_rn(e0.x, e1.x), __fmul_rn(e0.y, e1.y));
+        const float d11 = __fadd_rn(__fmul_rn(e1.x, e1.x), __fmul_rn(e1.y, e1.y));
+        const float denom = __fsub_rn(__fmul_rn(d00, d11), __fmul_rn(d01, d01));
+        R.q0[own] = make_float4(a.x, a.y, az.x, az.y);   // the same values from every lane of the triangle
+        R.q1[own] = make_float4(b.x, b.y, bz.x, bz.y);
+        R.q2[own] = make_float4(cc.x, cc.y, cz.x, cz.y);
+        R.q3[own] = make_float4(d00, d01, d11, denom);
+        if (first) {
+          fbx = centroid(ua.x, ub.x, uc.x); fby = centroid(ua.y, ub.y, uc.y); fbz = centroid(va.x, vb.x, vc.x);
+          n0 = az.y;
+        }
+        const float minx = fminf(fminf(a.x, b.x), cc.x), maxx = fmaxf(fmaxf(a.x, b.x), cc.x);
+        const float miny = fminf(fminf(a.y, b.y), cc.y), maxy = fmaxf(fmaxf(a.y, b.y), cc.y);
+        const int x1 = __float2int_rz(maxx);
+        if (x1 >= p.G) atomicOr(&p.flags[o], kFlagGrid);
+        if (fabsf(denom) > 0.001f) {
+          T = mask_setup(a.x, a.y, e0.x, e0.y, e1.x, e1.y, d00, d01, d11, denom, minx, maxx, miny, maxy,
+                         max(__float2int_rz(minx), 0), min(x1, p.G - 1), __float2int_rz(miny), __float2int_rz(maxy),
+                         p.half);
+          if (T.nx > 0 && T.ny > 0) {
+            ncx = (int)((unsigned)(T.nx + kCellX - 1) / kCellX);
+            ncell = ncx * (int)((unsigned)(T.ny + kCellY - 1) / kCellY);
+          }
+        }
+      }
+      int lim = ncell;
       if (first) {
-        fb_x = __float2int_rz(centroid(__fsub_rn(raw[0].x, sh.dx), __fsub_rn(raw[1].x, sh.dx), __fsub_rn(raw[2].x, sh.dx)));
-        fb_y = __float2int_rz(centroid(__fsub_rn(raw[0].y, sh.dy), __fsub_rn(raw[1].y, sh.dy), __fsub_rn(raw[2].y, sh.dy)));
-        fb_z = centroid(__fsub_rn(raw[0].z, sh.dz), __fsub_rn(raw[1].z, sh.dz), __fsub_rn(raw[2].z, sh.dz));
-        n0 = g.n0;
+        big = __ballot_sync(full, ncell > kLaneCells * L && sub == 0);
+        lim = min(ncell, kLaneCells * L);
       }
-      if (b.ok) {
-        T = mask_setup(g.ax, g.ay, b.e0x, b.e0y, b.e1x, b.e1y, b.d00, b.d01, b.d11, b.denom,
-                       fminf(fminf(g.ax, g.bx), g.cx), fmaxf(fmaxf(g.ax, g.bx), g.cx), fminf(fminf(g.ay, g.by), g.cy),
-                       fmaxf(fmaxf(g.ay, g.by), g.cy), max(g.x0, 0), min(g.x1, p.G - 1), g.y0, g.y1, p.half);
-        if (T.nx > 0 && T.ny > 0) {
-          ncx = (T.nx + kCellX - 1) / kCellX;
-          ncell = ncx * ((T.ny + kCellY - 1) / kCellY);
+      float rc;
+      asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(rc) : "f"((float)max(ncx, 1)));
+      while (__any_sync(full, c < lim)) {
+        unsigned m = 0u;
+        if (c < lim) {
+          // c / ncx: at most 1,024 with ncx <= 512, so the float quotient of c + 1/2 truncates exactly
+          const int cj = __float2int_rz(((float)c + 0.5f) * rc), ci = c - cj * ncx;
+          m = mask_cell(T, ci, cj);
+          R.org[lane] = (unsigned)(T.x0 + kCellX * ci) | ((unsigned)(T.y0 + kCellY * cj) << 16);
         }
-      }
-    }
-    int lim = ncell;
-    if (first) {
-      big = __ballot_sync(full, ncell > kLaneCells * L && sub == 0);
-      lim = min(ncell, kLaneCells * L);
-    }
-    const float rc = __frcp_rn((float)max(ncx, 1));
-    while (__any_sync(full, c < lim)) {
-      unsigned m = 0u;
-      if (c < lim) {
-        // c / ncx: at most 1,024 with ncx <= 512, so the float quotient of c + 1/2 truncates exactly
-        const int cj = __float2int_rz(((float)c + 0.5f) * rc), ci = c - cj * ncx;
-        m = mask_cell(T, ci, cj);
-        R.org[lane] = (unsigned)(T.x0 + kCellX * ci) | ((unsigned)(T.y0 + kCellY * cj) << 16);
-      }
-      c += step;
-      // queue the candidates in lane order
-      const int mine = __popc(m);
-      int at = mine;
-      for (int d = 1; d < 32; d <<= 1) {
-        const int y = __shfl_up_sync(full, at, d);
-        if (lane >= d) at += y;
-      }
-      const int n = __shfl_sync(full, at, 31);
-      at -= mine;
-      while (m) {
-        const int b = __clz(m);
-        m ^= 0x80000000u >> b;
-        R.q[at++] = (unsigned short)(lane << 5 | b);
-      }
-      __syncwarp();
-      for (int i = 0; i < n; i += 32) {
-        const bool valid = i + lane < n;
-        const unsigned item = valid ? R.q[i + lane] : 0u;
-        const int l = (int)(item >> 5), b = (int)(item & 31u);
-        const int w = first ? l & ~(L - 1) : own;
-        const unsigned org = R.org[l];
-        const int x = (int)(org & 0xFFFFu) + (b >> 2), y = (int)(org >> 16) + (b & 3);
-        const float4 A = R.q0[w], B = R.q1[w], C = R.q2[w], D = R.q3[w];
-        // _getBaryCoord (Tomo_types.cpp:86-115), the "+ 0*0" terms of _dot
-        // left out (they only turn -0 into +0, which changes no comparison
-        // and no stored value)
-        const float e0x = __fsub_rn(B.x, A.x), e0y = __fsub_rn(B.y, A.y);
-        const float e1x = __fsub_rn(C.x, A.x), e1y = __fsub_rn(C.y, A.y);
-        const float e2x = __fsub_rn(pix_center(x, p.half), A.x), e2y = __fsub_rn(pix_center(y, p.half), A.y);
-        const float d20 = __fadd_rn(__fmul_rn(e2x, e0x), __fmul_rn(e2y, e0y));
-        const float d21 = __fadd_rn(__fmul_rn(e2x, e1x), __fmul_rn(e2y, e1y));
-        const float v = __fdiv_rn(__fsub_rn(__fmul_rn(D.z, d20), __fmul_rn(D.y, d21)), D.w);
-        const float ww = __fdiv_rn(__fsub_rn(__fmul_rn(D.x, d21), __fmul_rn(D.y, d20)), D.w);
-        const float u = __double2float_rn(__dsub_rn(__dsub_rn(1.0, (double)v), (double)ww));
-        const bool hit = valid && (u >= -0.001f) && (v >= -0.001f) && (v <= p.vmax) && (__fadd_rn(u, v) <= p.vmax);
-        hits |= __reduce_or_sync(full, hit ? 1u << w : 0u);
-        const unsigned who = __ballot_sync(full, hit);
-        if (hit) {
-          const int sx = __float2int_rz(bary3(A.x, B.x, C.x, u, v, ww));
-          const int sy = __float2int_rz(bary3(A.y, B.y, C.y, u, v, ww));
-          const float fz = bary3(A.z, B.z, C.z, u, v, ww), fn = bary3(A.w, B.w, C.w, u, v, ww);
-          const float fz2 = __fadd_rn(fz, (fn >= 0.0f) ? -p.shell_off : p.shell_off);
-          append(p, o, who, sx, sy, make_key(to_i16(fz), to_i16(__fmul_rn(fn, 1000.0f))),
-                 make_key(to_i16(fz2), to_i16(__fmul_rn(-fn, 1000.0f))));
+        c += step;
+        // queue the candidates in lane order
+        const int mine = __popc(m);
+        int at = mine;
+        for (int d = 1; d < 32; d <<= 1) {
+          const int y = __shfl_up_sync(full, at, d);
+          if (lane >= d) at += y;
         }
+        const int n = __shfl_sync(full, at, 31);
+        unsigned short* q = R.q + (at - mine);
+        while (m) {
+          const int b = __clz(m);
+          m ^= 0x80000000u >> b;
+          *q++ = (unsigned short)(lane << 5 | b);
+        }
+        __syncwarp();
+        for (int i = 0; i < n; i += 32) {
+          const bool valid = i + lane < n;
+          const unsigned item = valid ? R.q[i + lane] : 0u;
+          const int l = (int)(item >> 5), b = (int)(item & 31u);
+          const int w = first ? l & ~(L - 1) : own;
+          const unsigned org = R.org[l];
+          const int x = (int)(org & 0xFFFFu) + (b >> 2), y = (int)(org >> 16) + (b & 3);
+          const float4 A = R.q0[w], B = R.q1[w], C = R.q2[w], D = R.q3[w];
+          // _getBaryCoord (Tomo_types.cpp:86-115), the "+ 0*0" terms of _dot
+          // left out (they only turn -0 into +0, which changes no comparison
+          // and no stored value)
+          const F2 a = {A.x, A.y};
+          const F2 e0 = sub2(F2{B.x, B.y}, a), e1 = sub2(F2{C.x, C.y}, a);
+          const F2 e2 = sub2(add2(add2(F2{(float)x, (float)y}, F2{0.001f, 0.001f}), F2{p.half, p.half}), a);
+          const F2 t0 = mul2(e2, e0), t1 = mul2(e2, e1);
+          const float d20 = __fadd_rn(t0.x, t0.y), d21 = __fadd_rn(t1.x, t1.y);
+          const float v = __fdiv_rn(__fsub_rn(__fmul_rn(D.z, d20), __fmul_rn(D.y, d21)), D.w);
+          const float ww = __fdiv_rn(__fsub_rn(__fmul_rn(D.x, d21), __fmul_rn(D.y, d20)), D.w);
+          const float u = __double2float_rn(__dsub_rn(__dsub_rn(1.0, (double)v), (double)ww));
+          const bool hit = valid && (u >= -0.001f) && (v >= -0.001f) && (v <= p.vmax) && (__fadd_rn(u, v) <= p.vmax);
+          hits |= __reduce_or_sync(full, hit ? 1u << w : 0u);
+          const unsigned who = __ballot_sync(full, hit);
+          room();
+          if (hit) {
+            const F2 f = bary3x2(F2{A.x, A.y}, F2{B.x, B.y}, F2{C.x, C.y}, u, v, ww);
+            const F2 g = bary3x2(F2{A.z, A.w}, F2{B.z, B.w}, F2{C.z, C.w}, u, v, ww);
+            const int e = ns + __popc(who & below);
+            R.st[e] = make_uint2(pixel_key(g.x, g.y), slot_xy(p, f.x, f.y));
+            if (kTwin) R.st2[e] = pixel_key(__fadd_rn(g.x, (g.y >= 0.0f) ? -p.shell_off : p.shell_off), -g.y);
+          }
+          ns += __popc(who);
+        }
+        __syncwarp();
       }
+      if (!big) break;
+      own = __ffs(big) - 1;
+      big &= big - 1;
+      tt = __shfl_sync(full, t, own);
+      c = kLaneCells * L + lane;
+      step = 32;
       __syncwarp();
     }
-    if (!big) break;
-    own = __ffs(big) - 1;
-    big &= big - 1;
-    tt = __shfl_sync(full, t, own);
-    c = kLaneCells * L + lane;
-    step = 32;
+    // centroid fallback of triangles without an accepted pixel, with the vertex-0 normal
+    const bool miss = t < p.nT && sub == 0 && !((hits >> lane) & 1u);
+    const unsigned who = __ballot_sync(full, miss);
+    if (who) {
+      room();
+      if (miss) {
+        const int e = ns + __popc(who & below);
+        R.st[e] = make_uint2(pixel_key(fbz, n0), slot_xy(p, fbx, fby));
+        if (kTwin) R.st2[e] = pixel_key(__fadd_rn(fbz, (n0 >= 0.0f) ? -p.shell_off : p.shell_off), -n0);
+      }
+      ns += __popc(who);
+    }
     __syncwarp();
   }
-  // centroid fallback of triangles without an accepted pixel, with the vertex-0 normal
-  const bool miss = t < p.nT && sub == 0 && !((hits >> lane) & 1u);
-  const unsigned who = __ballot_sync(full, miss);
-  if (miss) {
-    const float fz2 = __fadd_rn(fb_z, (n0 >= 0.0f) ? -p.shell_off : p.shell_off);
-    append(p, o, who, fb_x, fb_y, make_key(to_i16(fb_z), to_i16(__fmul_rn(n0, 1000.0f))),
-           make_key(to_i16(fz2), to_i16(__fmul_rn(-n0, 1000.0f))));
-  }
+  flush<kTwin, kStash / 32>(p, o, R, ns);
 }
 
 // ---------------------------------------------------------------- K3 strip
@@ -1978,11 +2097,20 @@ static dim3 tri_grid(const EngineParams& p)
 // kRastFill; then the lanes of a triangle share its cells.
 constexpr int kRastFill = 148 * 16;
 
-int raster_lanes(int nT, int Bo)
+int raster_lanes_log2(int nT, int Bo)
 {
-  int L = 1;
-  while (L < 32 && (long long)Bo * ((nT + 32 / L - 1) / (32 / L)) < kRastFill) L *= 2;
-  return L;
+  int s = 0;
+  while (s < 5 && (long long)Bo * ((nT + (32 >> s) - 1) >> (5 - s)) < kRastFill) s++;
+  return s;
+}
+
+// Blocks per orientation: each warp takes several groups of triangles in turn
+// (its stash then fills whole rounds), while kRastFill warps are left.
+static int raster_blocks(int ngroup, int Bo)
+{
+  int per = kRastGroups;
+  while (per > 1 && (long long)Bo * (ngroup / per) < 4 * kRastFill) per--;
+  return std::min((ngroup + kRastWarps * per - 1) / (kRastWarps * per), 65535);
 }
 
 // Rotation and, for priority and safe strips, the triangle bins' count pass.
@@ -2003,8 +2131,10 @@ cudaError_t launch_bin_count(const EngineParams& p, cudaStream_t main, LaunchLog
 cudaError_t launch_fill(const EngineParams& p, cudaStream_t s, LaunchLog* L)
 {
   if (p.mode == 0) {
-    const int per_block = kRastWarps * (32 / p.rast_lanes);
-    TOMO_LAUNCH(kKRaster, s, (k_raster<<<dim3((p.nT + per_block - 1) / per_block, p.Bo), 32 * kRastWarps, 0, s>>>(p)));
+    const int ngroup = (p.nT + (32 >> p.rast_shift) - 1) >> (5 - p.rast_shift);
+    const dim3 grid(std::min(kRastMix, p.Bo), raster_blocks(ngroup, p.Bo), (p.Bo + kRastMix - 1) / kRastMix);
+    if (p.twin) TOMO_LAUNCH(kKRaster, s, (k_raster<true><<<grid, 32 * kRastWarps, 0, s>>>(p)));
+    else TOMO_LAUNCH(kKRaster, s, (k_raster<false><<<grid, 32 * kRastWarps, 0, s>>>(p)));
   } else {
     TOMO_LAUNCH(kKFill, s, (k_bin_fill<<<tri_grid(p), 256, 2 * sizeof(int) * p.S, s>>>(p)));
   }

@@ -165,21 +165,23 @@ TOMO_HD void span_rows(const SpanTri& T, float px, int y0, int ylen, int& lo, in
 // are affine in the pixel's column and row; a pixel is a candidate when all
 // three are >= 0.  vn, wn are the barycentric numerators above and the bounds
 // are the pre-reject's (0.002, 1.003 of |denom|, twice the exact test's
-// margins) widened by every rounding, in units of the numerators:
+// margins) widened by every rounding, in units of the numerators.  With L the
+// larger extent of the bounding box, q = L + 2 + |half| (no pixel looked at is
+// further from vertex a) and D = d00 + d11 (so |d01| <= D / 2), the terms of
+// both numerators sum to at most S = 3 q L D:
 //   * the exact test's float numerators against the linear form, the float
 //     coefficients, and the evaluation below (at most nine roundings of values
-//     below S per function): less than 2^-19 S together; 2^-17 S is added
-//     (S as in span_setup);
+//     below S per function): less than 2^-19 S together; 2^-18 S is added;
 //   * a pixel centre ((x + 0.001f) + half) - ax is formed in float by the
 //     reference with three roundings, each within 2^-24 of a value below
 //     M = |x| + |half| + |ax| + 2, here for the cell grid's first pixel only
-//     and then stepped by whole numbers: they differ by less than 2^-21 M, and
-//     the functions are widened by slope x 2^-20 M.
+//     and then stepped by whole numbers: they differ by less than 2^-21 M per
+//     axis, and the slopes are below 1.5 D L; 1.5 D L 2^-20 (Mx + My) is added.
 // Only the pixels whose centres lie within the triangle's bounding box widened
-// by d are looked at: with the roundings above at most 0.004 |denom| (else the
-// whole pixel box is used), an accepted pixel has v, w >= -0.0051 and
+// by d are looked at: with 2^-18 S at most 0.002 |denom| (else the whole pixel
+// box is used), an accepted pixel has v, w >= -0.0051 and
 // u >= -0.0102, so its centre is within 0.0205 of the box's extent;
-// d = 0.025 extent + 2^-19 M + 0.001.
+// d = 0.025 L + 2^-19 (Mx + My) + 0.001.
 struct MaskTri {
   float pv, pw, pu;        // change per column of V, W, U
   float bv, bw, bu;        // change per row
@@ -214,36 +216,30 @@ TOMO_HD MaskTri mask_setup(float ax, float ay, float e0x, float e0y, float e1x, 
 {
   MaskTri T;
   const float ad = fabsf(denom), ah = fabsf(half);
-  const float sgn = denom > 0.0f ? 1.0f : -1.0f;
-  T.pv = sgn * fmaf(d11, e0x, -(d01 * e1x));
-  T.bv = sgn * fmaf(d11, e0y, -(d01 * e1y));
-  T.pw = sgn * fmaf(d00, e1x, -(d01 * e0x));
-  T.bw = sgn * fmaf(d00, e1y, -(d01 * e0y));
+  // the numerators' common sign goes into the d's
+  const float f00 = copysignf(d00, denom), f11 = copysignf(d11, denom), f01 = denom < 0.0f ? -d01 : d01;
+  T.pv = fmaf(f11, e0x, -(f01 * e1x));
+  T.bv = fmaf(f11, e0y, -(f01 * e1y));
+  T.pw = fmaf(f00, e1x, -(f01 * e0x));
+  T.bw = fmaf(f00, e1y, -(f01 * e0y));
   T.pu = -(T.pv + T.pw);
   T.bu = -(T.bv + T.bw);
-  const float extx = maxx - minx, exty = maxy - miny;
-  const float mx = extx + (2.0f + ah), my = exty + (2.0f + ah);
-  const float s0 = fmaf(mx, fabsf(e0x), my * fabsf(e0y)), s1 = fmaf(mx, fabsf(e1x), my * fabsf(e1y));
-  const float k = 1.0f / 131072.0f;   // 2^-17
-  const float a01 = fabsf(d01);
-  const float ev = k * fmaf(d11, s0, a01 * s1), ew = k * fmaf(d00, s1, a01 * s0);
-  const float posx = fabsf(maxx) + fabsf(minx) + (2.0f + ah), posy = fabsf(maxy) + fabsf(miny) + (2.0f + ah);
-  const float ex = posx * (1.0f / 1048576.0f), ey = posy * (1.0f / 1048576.0f);   // 2^-20 M
-  T.x0 = x0; T.y0 = y0; T.nx = x1 - x0 + 1; T.ny = y1 - y0 + 1;
-  if (ev + ew <= 0.004f * ad) {
-    const float dx = fmaf(0.025f, extx, fmaf(2.0f, ex, 0.001f)), dy = fmaf(0.025f, exty, fmaf(2.0f, ey, 0.001f));
-    const float c = 0.001f + half;
-    const int cx0 = ceil_int((minx - dx) - c), cx1 = floor_int((maxx + dx) - c);
-    const int cy0 = ceil_int((miny - dy) - c), cy1 = floor_int((maxy + dy) - c);
-    T.x0 = cx0 > x0 ? cx0 : x0; T.y0 = cy0 > y0 ? cy0 : y0;
-    T.nx = (cx1 < x1 ? cx1 : x1) - T.x0 + 1; T.ny = (cy1 < y1 ? cy1 : y1) - T.y0 + 1;
-  }
+  const float L = fmaxf(maxx - minx, maxy - miny);
+  const float m = fmaf(2.0f, fabsf(maxx) + fabsf(maxy), 6.0f + 2.0f * ah);   // Mx + My
+  const float DL = (d00 + d11) * L, es = DL * ((L + (2.0f + ah)) * (3.0f / 262144.0f));
+  const float e = fmaf(DL, m * (1.5f / 1048576.0f), es);
+  const float c = 0.001f + half;
+  // a sliver's numerators are too uncertain: no tighter box than the pixel box
+  const float d = es <= 0.002f * ad ? fmaf(0.025f, L, fmaf(m, 1.0f / 524288.0f, 0.001f)) : 1.0e6f;
+  const float lo = d + c, hi = d - c;
+  const int cx0 = ceil_int(minx - lo), cx1 = floor_int(maxx + hi);
+  const int cy0 = ceil_int(miny - lo), cy1 = floor_int(maxy + hi);
+  T.x0 = cx0 > x0 ? cx0 : x0; T.y0 = cy0 > y0 ? cy0 : y0;
+  T.nx = (cx1 < x1 ? cx1 : x1) - T.x0 + 1; T.ny = (cy1 < y1 ? cy1 : y1) - T.y0 + 1;
   const float cx = (((float)T.x0 + 0.001f) + half) - ax, cy = (((float)T.y0 + 0.001f) + half) - ay;
-  const float lv = fmaf(0.002f, ad, ev) + fmaf(fabsf(T.pv), ex, fabsf(T.bv) * ey);
-  const float lw = fmaf(0.002f, ad, ew) + fmaf(fabsf(T.pw), ex, fabsf(T.bw) * ey);
-  const float lu = fmaf(1.003f, ad, ev + ew) + fmaf(fabsf(T.pu), ex, fabsf(T.bu) * ey) + k * ad;
+  const float lv = fmaf(0.002f, ad, e), lu = fmaf(1.00301f, ad, 2.0f * e);
   T.v0 = fmaf(T.pv, cx, fmaf(T.bv, cy, lv));
-  T.w0 = fmaf(T.pw, cx, fmaf(T.bw, cy, lw));
+  T.w0 = fmaf(T.pw, cx, fmaf(T.bw, cy, lv));
   T.u0 = fmaf(T.pu, cx, fmaf(T.bu, cy, lu));
   return T;
 }
