@@ -93,6 +93,7 @@ struct EngineParams {
   float vmax;           // largest float <= 1.0 + double(0.001f)
   float thr;            // float(-sin(theta_c))
   int explicit_ss;
+  int nz_ex, nz_im;     // of a down face (nz <= -1): nz / 1000 < thr iff nz <= nz_ex, > thr iff nz >= nz_im
 
   // shared-memory layout of the strip kernel
   int ent_cap;          // entries per strip CTA
@@ -106,7 +107,7 @@ struct EngineParams {
   int* bins;            // [Bo][bin_cap]
   int bin_cap;
 
-  // accepted pixels of each strip (normal strips: k_raster -> k_strip)
+  // accepted pixels of each strip (normal strips: k_raster -> k_columns)
   uint2* ents;          // [Bo][S][ent_cap] (z, nz) key; slot within the strip
   int* ent_cnt;         // [Bo][S] pixels appended (may exceed ent_cap: the strip overflowed)
   int hshift;           // log2(H)

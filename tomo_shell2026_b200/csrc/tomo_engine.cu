@@ -30,7 +30,7 @@
 namespace tomo {
 
 size_t strip_smem_bytes(int mode, int H, int G, int ent_cap);
-size_t strip_four_per_sm_budget();
+size_t strip_default_budget();
 int raster_lanes_log2(int nT, int Bo);
 cudaError_t configure_kernels(size_t normal_smem, size_t safe_smem, size_t prio_smem);
 cudaError_t launch_batch(const EngineParams& p, cudaStream_t main, size_t strip_smem, LaunchLog* L);
@@ -401,50 +401,63 @@ struct Engine {
   }
 
   // Strip configurations.
-  //   0 normal     : H0-column strips, ~55 KB of shared memory (four CTAs
-  //                  per SM), entries without priorities; H0 is the tallest
-  //                  strip with room for two entries per slot;
-  //   1 safe       : H0-column strips, whole-box evaluation, priorities,
-  //                  all opt-in shared memory;
+  //   0 normal     : H0-column strips whose columns k_columns resolves from
+  //                  k_raster's pixel lists, five CTAs per SM; H0 is the
+  //                  tallest strip with room for two pixels per slot;
+  //   1 safe       : strips that rasterize their own triangles, whole-box
+  //                  evaluation, priorities, all opt-in shared memory;
   //   2 big normal : configuration 0 semantics with all opt-in shared memory
   //                  (orientations whose strip lists overflowed);
   //   3 narrow safe: safe mode with one-column strips (last resort);
-  //   4 priorities : configuration 0 strips whose entries also carry their
-  //                  first-come priority, all opt-in shared memory, for
-  //                  orientations where a column passed the 63-pixel cap.
+  //   4 priorities : strips that rasterize their own triangles and carry each
+  //                  pixel's first-come priority, all opt-in shared memory,
+  //                  for orientations where a column passed the 63-pixel cap.
   struct StripCfg { int H, S, C; size_t smem; int mode; };
   StripCfg cfg[5];
 
   void plan_strips()
   {
     const size_t optin = smem_optin ? smem_optin : 232448;
-    // default: the largest budget that keeps four CTAs on an SM (~55 KB on B200)
-    const size_t four = strip_four_per_sm_budget();
-    const size_t budget0 = std::min<size_t>(optin - 2048, normal_smem ? (size_t)normal_smem : (four ? four : 73728));
-    // the strip kernel also holds ~0.7 KB of static shared memory
+    // the strip kernels also hold ~0.7 KB of static shared memory
     const size_t budget1 = std::min<size_t>(optin, 227 * 1024) - 2048;
+    const size_t five = strip_default_budget();
+    // Pixels of an h-column normal strip.  By default what the shared memory of
+    // five CTAs per SM holds (82k solid, 256 orientations: 545 us at five, 592
+    // at four, 615 at six with 40 registers); a budget given by
+    // TOMO_OPT_NORMAL_SMEM (or a later one of adapt_after) buys 6 bytes per
+    // pixel beside four bytes and a bit per slot and a 20 KB work area.
+    auto pixels = [&](int h, size_t budget) -> int {
+      const size_t HG = (size_t)h * G;
+      const size_t fixed = budget ? 4 * HG + HG / 8 + 32 + std::max<size_t>(20816, 6 * HG + 2048) : strip_smem_bytes(0, h, G, 0);
+      const size_t all = budget ? std::min(optin - 2048, budget) : (five ? five : 45056), per = budget ? 6 : 4;
+      if (all < fixed + 32 * per) return 16;
+      const size_t most = (budget1 - strip_smem_bytes(0, h, G, 0)) / 4 - 16;
+      return (int)std::min<size_t>(std::min<size_t>((all - fixed) / per - 16, most), 32767);
+    };
     int h0 = 1;
     for (int h : {8, 4, 2, 1}) {
       if (force_h && h != force_h) continue;
-      const size_t fixed = strip_smem_bytes(0, h, G, 0);
-      if (fixed + 6 * 256 >= budget0) continue;
-      const int cap = (int)std::min<size_t>((budget0 - fixed) / 6 - 16, 32767);
+      if (strip_smem_bytes(0, h, G, 256) > budget1) continue;
+      const int cap = pixels(h, (size_t)normal_smem);
+      if (cap < 256) continue;
       if (force_h || cap >= 2 * h * G) { h0 = h; break; }
     }
-    auto make = [&](int mode, int h, size_t budget) {
+    auto make = [&](int mode, int h, int C) {
       StripCfg c;
       c.mode = mode; c.H = h; c.S = (G + h - 1) / h;
-      const size_t per = mode == 0 ? 6 : 15;
-      const size_t fixed = strip_smem_bytes(mode, h, G, 0);
-      c.C = (int)std::min<size_t>(budget > fixed + 32 * per ? (budget - fixed) / per - 16 : 16, 32767);
+      c.C = C;
+      if (mode != 0) {
+        const size_t fixed = strip_smem_bytes(mode, h, G, 0);
+        c.C = (int)std::min<size_t>(budget1 > fixed + 32 * 15 ? (budget1 - fixed) / 15 - 16 : 16, 32767);
+      }
       c.smem = strip_smem_bytes(mode, h, G, c.C);
       return c;
     };
-    cfg[0] = make(0, h0, budget0);
-    cfg[1] = make(1, h0, budget1);
-    cfg[2] = make(0, h0, budget1);
-    cfg[3] = make(1, 1, budget1);
-    cfg[4] = make(2, h0, budget1);
+    cfg[0] = make(0, h0, pixels(h0, (size_t)normal_smem));
+    cfg[1] = make(1, h0, 0);
+    cfg[2] = make(0, h0, (int)std::min<size_t>((budget1 - strip_smem_bytes(0, h0, G, 0)) / 4 - 16, 32767));
+    cfg[3] = make(1, 1, 0);
+    cfg[4] = make(2, h0, 0);
   }
 
   void choose_strips(int c)
@@ -537,6 +550,18 @@ struct Engine {
     p.vmax = largest_float_not_above(1.0 + (double)0.001f);
     p.thr = (float)(-1.0 * (double)sinf(P.theta_c));   // STomoSh_INT3.cpp:756
     p.explicit_ss = P.explicit_ss;
+    // nz / 1000 does not fall as nz grows: the down faces (nz <= -1) on either
+    // side of the threshold by bisection of the reference's own float division
+    auto first_nz = [&](auto above) {
+      int lo = -32768, hi = 0;
+      while (lo < hi) {
+        const int mid = lo + (hi - lo) / 2;
+        if (above((float)mid / 1000.0f)) hi = mid; else lo = mid + 1;
+      }
+      return lo;
+    };
+    p.nz_ex = first_nz([&](float v) { return v >= p.thr; }) - 1;
+    p.nz_im = first_nz([&](float v) { return v > p.thr; });
     p.ent_cap = ent_cap;
     p.out_vo = o_vo.ptr; p.out_vss = o_vss.ptr; p.out_vtc = o_vtc.ptr;
     p.out_vof = o_vof.ptr; p.out_vssf = o_vssf.ptr; p.out_vtcf = o_vtcf.ptr;
@@ -623,7 +648,7 @@ struct Engine {
     // upload adapted to (see adapt_after below)
     const int user_smem = normal_smem, user_h = force_h;
     const bool adapt = adaptive && !ids;
-    if (adapt && adapt_smem) { normal_smem = adapt_smem; force_h = adapt_h; plan_strips(); }
+    if (adapt && adapt_h) { normal_smem = adapt_smem; force_h = adapt_h; plan_strips(); }
     const int rc = sweep_batches(ids, n, adapt);
     if (adapt && (normal_smem != user_smem || force_h != user_h)) {
       normal_smem = user_smem; force_h = user_h; plan_strips();
@@ -632,24 +657,22 @@ struct Engine {
   }
 
   // After an early batch: if more than a fifth of its orientations overflowed
-  // their strip lists, give the rest of the sweep the next larger entry
-  // budget at the same strip height (one host wait per check; the overflowed
-  // orientations are re-run by the ladder as usual).  Returns true when the
-  // configuration changed.
+  // their strip lists, the rest of the sweep gets strips of half the height at
+  // the same occupancy (twice the pixels per column of the strip) or, past
+  // one-column strips, the next larger budget (one host wait per check; the
+  // overflowed orientations are re-run by the ladder as usual).  Returns true
+  // when the configuration changed.
   // A batch where most orientations passed the 63-pixel cap in some column
   // switches the rest of the sweep to the priority-carrying strips
   // (configuration 4), which resolve those columns in one pass.
   int adapt_after(int first, int nb, int* c, bool* changed)
   {
     *changed = false;
-    static const int kBudgets[] = {73728, 101376, 150528, 0};   // 0: everything the SM allows
+    static const int kBudgets[] = {73728, 101376, 150528, 232448};
     int next = -1;
-    if (*c == 0) {
-      const size_t cur = cfg[0].smem;
-      for (int b : kBudgets) {
-        const size_t lim = b ? (size_t)b : (size_t)std::min<size_t>(smem_optin, 227 * 1024) - 2048;
-        if (lim > cur + 4096) { next = b ? b : (int)lim; break; }
-      }
+    if (*c == 0 && H == 1) {
+      for (int b : kBudgets)
+        if (b > normal_smem && next < 0) next = b;
     }
     if (*c != 0) return 0;
     std::vector<int> fl(nb);
@@ -660,9 +683,9 @@ struct Engine {
     if (cap * 2 > nb) {
       *c = 4;
       adapt_cfg = 4;
-    } else if (next >= 0 && over * 5 > nb) {
-      force_h = H;
-      normal_smem = next;
+    } else if ((H > 1 || next >= 0) && over * 5 > nb) {
+      force_h = std::max(H / 2, 1);
+      if (H == 1) normal_smem = next;
       plan_strips();
       adapt_smem = normal_smem; adapt_h = force_h;
     } else {

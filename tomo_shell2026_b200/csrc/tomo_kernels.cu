@@ -1,7 +1,7 @@
 // B200 kernels of the orientation search (sm_100a).
 //
 // One batch of orientations runs as
-//   k_reset -> k_rotate -> k_raster -> k_strip -> k_bed, and k_fold on a
+//   k_reset -> k_rotate -> k_raster -> k_columns -> k_bed, and k_fold on a
 //   second stream;
 // see the launch sequence in tomo_engine.cu.  The work per orientation is the
 // reference INT3 pipeline (Tomo_Shell2026.cpp thread_func:138-156):
@@ -11,11 +11,10 @@
 //  * the slot grid is cut into strips of H x-columns; k_raster rasterizes
 //    every triangle once and appends its accepted pixels to their strips'
 //    lists in global memory;
-//  * one CTA per (orientation, strip) builds per-column linked lists of its
-//    pixels in shared memory, then runs the column stage (dedup, 63-pixel cap,
-//    sort, brief pairing, shadow casting) per column, reduces the column
-//    volumes to int64 and writes the column values in slot order for the
-//    float32 fold (k_strip);
+//  * one CTA per (orientation, strip) groups its pixels by column in shared
+//    memory, runs the column stage (dedup, 63-pixel cap, sort, brief pairing,
+//    shadow casting), reduces the column volumes to int64 and writes the
+//    column values in slot order for the float32 fold (k_columns);
 //  * an orientation whose strip lists overflow, or with a column past the
 //    63-pixel cap (where first-come order decides which pixels stay), is
 //    flagged and re-run by the host in a larger configuration, or in strips
@@ -28,7 +27,6 @@
 
 #include <algorithm>
 #include <climits>
-
 
 namespace tomo {
 
@@ -502,7 +500,7 @@ __global__ void __launch_bounds__(256) k_bin_fill(EngineParams p)
 // Normal strips.  triVoxel (STomoSh_INT3.cpp:1138-1209) of every triangle,
 // each handled once: the accepted pixels are appended to the lists of their
 // strips in global memory (8 bytes each: (z, nz) key and slot in the strip),
-// from which k_strip builds its columns.
+// from which k_columns builds its columns.
 //
 // One warp takes 32 / L triangles, L lanes each (L = 1 unless there are too
 // few triangles to fill the chip; then the lanes of a triangle share its
@@ -804,16 +802,14 @@ __global__ void __launch_bounds__(32 * kRastWarps, 7) k_raster(EngineParams p)
 
 // ---------------------------------------------------------------- K3 strip
 //
-// One CTA per (orientation, strip).  Normal mode keeps per entry only the
-// packed (z, nz) key and the next index (6 bytes) so four CTAs fit on an SM;
-// a column whose distinct keys exceed the 63-pixel cap needs first-come
-// priorities and sends its orientation to safe mode, which also stores the
-// (triangle, pixel, twin) priority of every entry.
+// Priority and safe strips: one CTA per (orientation, strip) rasterizes the
+// strip's binned triangles into per-column linked lists whose entries carry
+// their (triangle, pixel, twin) priority, for the orientations where a column
+// passes the 63-pixel cap (which keys survive depends on first-come order) or
+// a normal strip could not be resolved.
 
 constexpr int kChunk = 256;    // triangles staged per pass (== blockDim.x)
 constexpr int kRegKeys = 11;   // columns with up to this many raw pixels sort in registers
-constexpr int kMaxEnt = 32767; // entry indices are stored as int16
-constexpr int kWarpKeys = 64;  // raw entries a warp sorts in registers (two per lane)
 constexpr int kWalkQueue = 64; // pre-reject survivors queued per warp before the exact test
 
 struct StripSmem {
@@ -833,8 +829,6 @@ struct StripSmem {
   unsigned* wq;        // [warps][kWalkQueue] pixels past the pre-reject, per warp
   short* olist;        // [H*G] occupied local slots in slot order (aliases the chunk area)
   short* longq;        // [H*G] phase B: positions in olist of columns with three or more raw entries
-  short* longq2;       // [H*G] phase B, normal strips: columns of more than kRegKeys raw entries
-  unsigned* wbuf;      // [warps][kWarpKeys] phase B, normal strips: one long column's keys per warp
   unsigned* scr;       // phase B: per-thread key scratch, scr[i * blockDim + thread] (chunk area after longq)
   int scr_cap;         // keys per thread in scr
 };
@@ -848,17 +842,13 @@ __host__ __device__ inline size_t strip_chunk_bytes()
 __host__ __device__ inline size_t round16(size_t b) { return (b + 15) / 16 * 16; }
 
 // Shared-memory bytes of one strip CTA (mirrors the carve-up in k_strip).
-__host__ __device__ inline size_t strip_smem_layout(int mode, int H, int G, int C)
+__host__ __device__ inline size_t strip_smem_layout(int H, int G, int C)
 {
   const size_t HG = (size_t)H * G;
   size_t b = round16(sizeof(int) * HG) + round16(sizeof(unsigned) * ((HG + 31) / 32));
-  b += round16(sizeof(unsigned) * (size_t)C) + round16(sizeof(short) * (size_t)C);
-  if (mode != 0) b += 2 * round16(sizeof(unsigned) * (size_t)C) + round16((size_t)C);
+  b += 3 * round16(sizeof(unsigned) * (size_t)C) + round16(sizeof(short) * (size_t)C) + round16((size_t)C);
   const size_t chunk = strip_chunk_bytes();
-  // phase B: occupied-slot list + long-column queue (+ normal strips: the queue of
-  // columns past kRegKeys raw entries and the per-warp key buffers)
-  const size_t ob = round16(sizeof(short) * HG);
-  const size_t olist = mode == 0 ? 3 * ob + sizeof(unsigned) * kWarpKeys * (kChunk / 32) : 2 * ob;
+  const size_t olist = 2 * round16(sizeof(short) * HG);   // phase B: occupied-slot list + long-column queue
   return b + (chunk > olist ? chunk : olist);
 }
 
@@ -973,69 +963,6 @@ __device__ __forceinline__ bool column_short(const EngineParams& p, const StripS
   if (dump) { dump_key(p, gslot, 0, hi, t0); dump_key(p, gslot, 1, lo, t1); }
   col_result(p, s, 2, r);
   return true;
-}
-
-// Column stage of a normal-strip column of more than kRegKeys and at most
-// kWarpKeys raw entries, by one warp: lane 0 copies the list into the warp's
-// key buffer, every lane ranks its two keys among the distinct keys (first
-// occurrences) with shuffles, the distinct keys are scattered into
-// descending order, and lane 0 runs the column scan (col_step) over them --
-// the per-thread path's result, without its per-key list walks.  More than
-// 63 distinct keys flag the orientation for first-come priorities, as the
-// per-thread path does.  Every lane returns lane 0's result.
-__device__ __forceinline__ void column_warp(const EngineParams& p, const StripSmem& sm, int head, int n,
-                                            unsigned* wbuf, bool dump, int gslot, int* sflag, ColOut& r)
-{
-  const int lane = threadIdx.x & 31;
-  if (lane == 0) {
-    int m = 0;
-    for (int e = head; e >= 0 && m < kWarpKeys; e = sm.enext[e]) wbuf[m++] = sm.ekey[e];
-  }
-  __syncwarp();
-  const bool va = lane < n, vb = lane + 32 < n;
-  const unsigned ka = va ? wbuf[lane] : 0u, kb = vb ? wbuf[lane + 32] : 0u;
-  // first occurrences: no equal key at a smaller list position
-  bool fa = va, fb = vb;
-  for (int j = 0; j < 32; j++) {
-    const unsigned x = __shfl_sync(0xFFFFFFFFu, ka, j), y = __shfl_sync(0xFFFFFFFFu, kb, j);
-    if (j < n) { fa = fa && !(x == ka && j < lane); fb = fb && !(x == kb); }
-    if (j + 32 < n) fb = fb && !(y == kb && j < lane);
-  }
-  // rank among the distinct keys, descending
-  int ra = 0, rb = 0;
-  for (int j = 0; j < 32; j++) {
-    const unsigned x = __shfl_sync(0xFFFFFFFFu, ka, j), y = __shfl_sync(0xFFFFFFFFu, kb, j);
-    const bool fx = __shfl_sync(0xFFFFFFFFu, fa, j), fy = __shfl_sync(0xFFFFFFFFu, fb, j);
-    ra += (fx && x > ka) + (fy && y > ka);
-    rb += (fx && x > kb) + (fy && y > kb);
-  }
-  const int d = __popc(__ballot_sync(0xFFFFFFFFu, fa)) + __popc(__ballot_sync(0xFFFFFFFFu, fb));
-  r.vo = r.vss = r.tc = 0; r.ndist = 0; r.nfin = 0; r.lastz = 0; r.lasttype = 0; r.has10 = 0;
-  if (d > kSlotCap) {   // first-come order decides which keys survive
-    if (lane == 0) atomicOr(sflag, kFlagCap);
-    return;
-  }
-  __syncwarp();
-  if (fa) wbuf[ra] = ka;
-  if (fb) wbuf[rb] = kb;
-  __syncwarp();
-  if (lane == 0) {
-    if (d == 1) {   // duplicates of a single key
-      r.ndist = 1; r.nfin = 1; r.lastz = key_z(wbuf[0]); r.lasttype = 0;
-      r.has10 = (key_z(wbuf[0]) == 1 && key_nz(wbuf[0]) == 0);
-      if (dump) dump_key(p, gslot, 0, wbuf[0], 0);
-    } else {
-      ColState s;
-      col_init(s);
-      for (int i = 0; i < d; i++) {
-        const unsigned key = wbuf[i];
-        const int t = col_step(s, key_z(key), key_nz(key), p.thr, p.explicit_ss);
-        if (dump) dump_key(p, gslot, i, key, t);
-      }
-      col_result(p, s, d, r);
-    }
-  }
-  __syncwarp();
 }
 
 // Column stage of one slot from its shared-memory list.
@@ -1159,7 +1086,6 @@ __device__ ColOut column(const EngineParams& p, const StripSmem& sm, int head, b
   // Past 63 distinct keys the first-come cap decides which survive, which
   // needs priorities: normal strips hand the orientation on; priority strips
   // start the column over with them.
-  if (need_prio && MODE == 0) { atomicOr(sflag, kFlagCap); return r; }
   if (need_prio) {
     col_init(s);
     d = 0;
@@ -1350,10 +1276,10 @@ __device__ __forceinline__ void exact_item(const EngineParams& p, const StripSme
 }
 
 template <int MODE>
-__global__ void __launch_bounds__(256, MODE == 0 ? 4 : 1) k_strip(EngineParams p)
+__global__ void __launch_bounds__(256, 1) k_strip(EngineParams p)
 {
   extern __shared__ __align__(16) unsigned char smem[];
-  __shared__ int nent, sflag, nlong, nlong2, wtot[32];
+  __shared__ int nent, sflag, nlong, wtot[32];
   __shared__ long long red[8][8];
 
   const int s = blockIdx.x, o = blockIdx.y;
@@ -1371,12 +1297,9 @@ __global__ void __launch_bounds__(256, MODE == 0 ? 4 : 1) k_strip(EngineParams p
   sm.occ = (unsigned*)q; q += round16(sizeof(unsigned) * nwords);
   sm.ekey = (unsigned*)q; q += round16(sizeof(unsigned) * C);
   sm.enext = (short*)q; q += round16(sizeof(short) * C);
-  sm.et = sm.elo = nullptr; sm.emark = nullptr;
-  if (MODE != 0) {
-    sm.et = (unsigned*)q; q += round16(sizeof(unsigned) * C);
-    sm.elo = (unsigned*)q; q += round16(sizeof(unsigned) * C);
-    sm.emark = (uint8_t*)q; q += round16((size_t)C);
-  }
+  sm.et = (unsigned*)q; q += round16(sizeof(unsigned) * C);
+  sm.elo = (unsigned*)q; q += round16(sizeof(unsigned) * C);
+  sm.emark = (uint8_t*)q; q += round16((size_t)C);
   unsigned char* chunk = q;
   sm.q0 = (float4*)q; q += sizeof(float4) * kChunk;
   sm.q1 = (float4*)q; q += sizeof(float4) * kChunk;
@@ -1390,17 +1313,10 @@ __global__ void __launch_bounds__(256, MODE == 0 ? 4 : 1) k_strip(EngineParams p
   sm.tkind = (uint8_t*)q; q += kChunk;
   sm.olist = (short*)chunk;
 
-  int nlist;
-  const int* list = nullptr;             // triangles of the strip (priority and safe strips)
-  if (MODE == 0) {
-    nlist = p.ent_cnt[(size_t)o * p.S + s];
-    if (nlist > C) return;               // k_raster flagged the orientation
-  } else {
-    const int* off = p.bin_off + (size_t)o * (p.S + 1);
-    const int lbeg = off[s];
-    nlist = max(min(off[s + 1], p.bin_cap) - lbeg, 0);
-    list = p.bins + (size_t)o * p.bin_cap + lbeg;
-  }
+  const int* off = p.bin_off + (size_t)o * (p.S + 1);
+  const int lbeg = off[s];
+  const int nlist = max(min(off[s + 1], p.bin_cap) - lbeg, 0);
+  const int* list = p.bins + (size_t)o * p.bin_cap + lbeg;
   uint8_t* bedf = p.bedf + (size_t)o * p.G * p.G + (size_t)xs0 * p.G;
 
   // bed flags of empty slots; occupied ones are overwritten in phase B
@@ -1416,15 +1332,6 @@ __global__ void __launch_bounds__(256, MODE == 0 ? 4 : 1) k_strip(EngineParams p
   if (threadIdx.x == 0) { nent = 0; sflag = 0; }
   __syncthreads();
 
-  if constexpr (MODE == 0) {
-  // ---- phase A: the strip's accepted pixels (k_raster) into per-column lists
-    const uint2* ents = p.ents + ((size_t)o * p.S + s) * C;
-    for (int i = threadIdx.x; i < nlist; i += blockDim.x) {
-      const uint2 e = __ldcs(ents + i);
-      sm.ekey[i] = e.x;
-      sm.enext[i] = (short)atomicExch(&sm.heads[e.y], i);
-    }
-  } else {
   const Shift sh = load_shift(p, o);
   const float half = p.half, vmax = p.vmax;
 
@@ -1591,7 +1498,6 @@ __global__ void __launch_bounds__(256, MODE == 0 ? 4 : 1) k_strip(EngineParams p
     prev_n = nchunk;
   }
   if (prev_n) fallback(prev_n, thit_base + ((chunk_no + 1) & 1) * (kChunk / 32));
-  }
   __syncthreads();
 
   // ---- occupied slots in slot order (bitmap from the list heads -> list)
@@ -1622,13 +1528,7 @@ __global__ void __launch_bounds__(256, MODE == 0 ? 4 : 1) k_strip(EngineParams p
     const size_t ob = round16(sizeof(short) * (size_t)HG);
     const size_t cb = strip_chunk_bytes();
     sm.longq = (short*)(chunk + ob);
-    size_t used = 2 * ob;
-    sm.longq2 = nullptr; sm.wbuf = nullptr;
-    if (MODE == 0) {
-      sm.longq2 = (short*)(chunk + 2 * ob);
-      sm.wbuf = (unsigned*)(chunk + 3 * ob);
-      used = 3 * ob + sizeof(unsigned) * kWarpKeys * (blockDim.x >> 5);
-    }
+    const size_t used = 2 * ob;
     sm.scr = (unsigned*)(chunk + used);
     sm.scr_cap = used < cb ? (int)((cb - used) / (sizeof(unsigned) * blockDim.x)) : 0;
   }
@@ -1669,7 +1569,7 @@ __global__ void __launch_bounds__(256, MODE == 0 ? 4 : 1) k_strip(EngineParams p
       d[6] = c.lasttype; d[7] = (p.bed_type != kBedNone) ? bed_flags(p, c) : 0;
     }
   };
-  if (threadIdx.x == 0) { nlong = 0; nlong2 = 0; }
+  if (threadIdx.x == 0) nlong = 0;
   __syncthreads();
   if (!redo) {
     for (int l = threadIdx.x; l < nocc; l += blockDim.x) {
@@ -1690,62 +1590,18 @@ __global__ void __launch_bounds__(256, MODE == 0 ? 4 : 1) k_strip(EngineParams p
     }
   }
   __syncthreads();
-  // B2: columns of three or more raw entries, one per thread; in normal
-  // strips those past kRegKeys raw entries go on to B3 instead
+  // B2: columns of three or more raw entries, one per thread
   if (!redo) {
     for (int q = threadIdx.x; q < nlong; q += blockDim.x) {
       const int l = sm.longq[q];
       const int ls = sm.olist[l];
       const int head = sm.heads[ls];
-      bool later = false;
-      if (MODE == 0) {
-        int n = 0;
-        for (int e = head; e >= 0 && n <= kRegKeys; e = sm.enext[e]) n++;
-        later = n > kRegKeys;
-      }
-      const unsigned want = __ballot_sync(__activemask(), later);
-      if (later) {
-        const int lane = threadIdx.x & 31, leader = __ffs(want) - 1;
-        int base = 0;
-        if (lane == leader) base = atomicAdd(&nlong2, __popc(want));
-        base = __shfl_sync(want, base, leader);
-        sm.longq2[base + __popc(want & ((1u << lane) - 1u))] = (short)l;
-        continue;
-      }
       const int gx = xs0 + ls / p.G, gy = ls % p.G;
       const int gslot = gx * p.G + gy;
       const ColOut c = column<MODE>(p, sm, head, dump, gslot, &sflag);
       store(l, ls, gx, gy, gslot, c);
     }
   }
-  // B3 (normal strips): one warp per column of more than kRegKeys raw entries
-  if (MODE == 0) {
-    __syncthreads();
-    if (!redo) {
-      const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
-      unsigned* wbuf = sm.wbuf + wid * kWarpKeys;
-      for (int q = wid; q < nlong2; q += nw) {
-        const int l = sm.longq2[q];
-        const int ls = sm.olist[l];
-        const int head = sm.heads[ls];
-        const int gx = xs0 + ls / p.G, gy = ls % p.G;
-        const int gslot = gx * p.G + gy;
-        int n = 0;
-        if (lane == 0)
-          for (int e = head; e >= 0 && n <= kWarpKeys; e = sm.enext[e]) n++;
-        n = __shfl_sync(0xFFFFFFFFu, n, 0);
-        ColOut c;
-        if (n <= kWarpKeys) {
-          column_warp(p, sm, head, n, wbuf, dump, gslot, &sflag, c);
-        } else if (lane == 0) {
-          c = column<MODE>(p, sm, head, dump, gslot, &sflag);   // a very long list: one thread
-        }
-        if (lane == 0) store(l, ls, gx, gy, gslot, c);
-        __syncwarp();
-      }
-    }
-  }
-
   // ---- phase C: reductions
   const long long vals[8] = {a_vo, a_vss, a_tc, a_avss, a_atc, a_ent, a_col, 0};
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -1777,6 +1633,492 @@ __global__ void __launch_bounds__(256, MODE == 0 ? 4 : 1) k_strip(EngineParams p
     if (!redo2) p.foldcnt[(size_t)o * p.S + s] = nocc;
     if (sflag) atomicOr(&p.flags[o], sflag);
   }
+}
+
+// ---------------------------------------------------------------- K3 columns
+// Normal strips: one CTA per (orientation, strip) turns the strip's pixel list
+// (k_raster) into columns and runs the column stage: dedup by (z, nz), the
+// 63-pixel cap, sort, splitAlBe / matchAlBePairBriefly
+// (STomoSh_INT3.cpp:493-513,583-611), createShadowBriefly (:749-812),
+// createTCPixels (:734-747) and createVoPixels / createVss_* (:934-1025).
+//
+// The pixels are grouped by slot with a counting sort in shared memory (one
+// 16-bit counter per slot), so a column is a run of keys.  Columns of one or
+// two raw pixels (nine in ten on a solid) have a closed form and take a thread
+// each.  The rest are resolved by pixel: a warp takes as many whole columns as
+// fit its 32 lanes, every lane ranks its key within its column, and the pairing
+// follows from ballots (see pair_pixels).  A column of more than 32 raw pixels
+// takes a warp by itself, 32 sorted keys at a time.
+//
+// Bound by instruction issue and, on strips of a few hundred pixels, by the
+// latency between its barriers.  With linked lists per column, one thread per
+// column of up to 11 pixels and a serial pairing scan the stage took 1,060 us
+// per 256 orientations of the 82k solid at four CTAs per SM, now 545 at five
+// (592 at four); 5k solid 92 -> 53 us; the 87k thin shell's 2-degree sweep
+// (seven pixels to a column) 557 -> 219 ms.
+constexpr int kColThreads = 256;
+constexpr int kColBlocks = 5;    // CTAs per SM
+constexpr int kLongKeys = 128;   // raw pixels of a column that a warp sorts in its scratch
+
+// Shared-memory bytes of one k_columns CTA.
+__host__ __device__ inline size_t columns_smem(int HG, int C)
+{
+  return round16(sizeof(short) * (size_t)(HG + 2)) + round16(sizeof(unsigned) * (size_t)C) +
+         2 * round16(sizeof(short) * (size_t)HG) + sizeof(unsigned) * kLongKeys * (kColThreads / 32);
+}
+
+// What earlier pixels of the same column leave behind for the next 32.
+struct PairCarry {
+  bool al;      // the last pixel with an up or down face was an up face
+  bool s, n;    // the last kept down face casts explicit / implicit support
+  bool first;   // an up face was kept
+};
+
+struct PairOut {
+  int vo, vss, tc;      // this pixel's share of the column's sums
+  int type;             // its type bits
+  unsigned ka, kb, s;   // lanes of kept up faces, kept down faces, down faces with explicit support
+};
+
+// Pairing of up to 32 distinct pixels in column order, one per lane; `seg`:
+// the lanes of this lane's column.  The reference walks a column from the top
+// and keeps an up face when no up face is open, a down face when one is: of the
+// pixels with an up or down face, those whose face differs from the one before
+// (the first only if it is an up face).  A kept down face casts support by its
+// slope, and the next kept up face, which always follows it, receives it.
+// p.nz_ex / p.nz_im: nz at or below / at or above which nz / 1000 is below /
+// above the shadow threshold.
+__device__ __forceinline__ PairOut pair_pixels(const EngineParams& p, unsigned key, bool distinct, unsigned seg,
+                                               const PairCarry& c)
+{
+  const unsigned full = 0xFFFFFFFFu;
+  const unsigned below = seg & ((1u << (threadIdx.x & 31)) - 1u);
+  const int z = key_z(key), nz = key_nz(key);
+  const bool up = distinct && nz >= 1, down = distinct && nz <= -1;
+  const unsigned A = __ballot_sync(full, up), B = __ballot_sync(full, down);
+  const unsigned prev = (A | B) & below;
+  const bool open = prev ? (A >> (31 - __clz(prev))) & 1u : c.al;
+  const bool ka = up && !open, kb = down && open;
+  PairOut r;
+  r.ka = __ballot_sync(full, ka);
+  r.kb = __ballot_sync(full, kb);
+  const bool s = kb && nz <= p.nz_ex, n = kb && nz >= p.nz_im;
+  r.s = __ballot_sync(full, s);
+  const unsigned N = __ballot_sync(full, n);
+  const unsigned pb = r.kb & below;
+  const int last = 31 - __clz(pb);
+  const bool sa = ka && (pb ? (r.s >> last) & 1u : c.s), na = ka && (pb ? (N >> last) & 1u : c.n);
+  const bool tc = !p.explicit_ss && ka && !((r.ka & below) || c.first);
+  r.type = (ka ? kAl : 0) | (kb ? kBe : 0) | (s ? kSSB : 0) | (sa ? kSSA : 0) | (n ? kNVB : 0) | (na ? kNVA : 0) |
+           (tc ? kTC : 0);
+  r.vo = ka ? z : (kb ? -z : 0);
+  r.tc = tc ? z : 0;
+  if (p.explicit_ss) r.vss = s ? z : (sa ? -z : 0);
+  else r.vss = (ka ? r.tc - z + (na ? z : 0) : 0) + (kb ? (n ? 0 : z) : 0);
+  return r;
+}
+
+__global__ void __launch_bounds__(kColThreads, kColBlocks) k_columns(EngineParams p)
+{
+  extern __shared__ __align__(16) unsigned char smem[];
+  __shared__ int nlong, nbig, sflag, wtot[32];
+  __shared__ long long red[kColThreads / 32][6];
+  const unsigned full = 0xFFFFFFFFu;
+  const int s = blockIdx.x, o = blockIdx.y;
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  const int HG = p.H * p.G, C = p.ent_cap;
+  const int xs0 = s * p.H;
+  const int HGs = (min(xs0 + p.H, p.G) - xs0) * p.G;   // the last strip may be narrower than H
+  const int n = p.ent_cnt[(size_t)o * p.S + s];
+  if (n > C) return;                     // k_raster flagged the orientation
+  uint8_t* bedf = p.bedf + (size_t)o * p.G * p.G + (size_t)xs0 * p.G;
+  const bool bed = p.bed_type != kBedNone;
+  // bed flags of empty slots; occupied ones are overwritten below
+  if (bed)
+    for (int i = tid; i < HGs; i += kColThreads) bedf[i] = kBfPoss | kBfLand;
+  if (n == 0) return;                    // strip sums stay zero (k_reset), fold count zero
+
+  unsigned char* q = smem;
+  unsigned* const off2 = (unsigned*)q; q += round16(sizeof(short) * (size_t)(HG + 2));   // two 16-bit slot counters a word
+  unsigned* const keys = (unsigned*)q; q += round16(sizeof(unsigned) * (size_t)C);
+  unsigned short* const olist = (unsigned short*)q; q += round16(sizeof(short) * (size_t)HG);   // occupied slots in order
+  unsigned short* const longq = (unsigned short*)q; q += round16(sizeof(short) * (size_t)HG);   // columns of 3..32 pixels from the front, longer from the back
+  unsigned* const scr = (unsigned*)q + wid * kLongKeys;
+  const unsigned short* const ends = (const unsigned short*)off2;
+
+  // ---- group the pixels by slot
+  const int nw = (HG + 1) >> 1;
+  for (int i = tid; i < nw; i += kColThreads) off2[i] = 0u;
+  if (tid == 0) { nlong = 0; nbig = 0; sflag = 0; }
+  const uint2* const ents = p.ents + ((size_t)o * p.S + s) * C;
+  constexpr int kHold = 8;               // pixels a thread keeps between the two passes
+  uint2 held[kHold];
+#pragma unroll
+  for (int j = 0; j < kHold; j++)
+    if (tid + j * kColThreads < n) held[j] = ents[tid + j * kColThreads];
+  __syncthreads();
+#pragma unroll
+  for (int j = 0; j < kHold; j++)
+    if (tid + j * kColThreads < n) atomicAdd(off2 + (held[j].y >> 1), 1u << (16 * (held[j].y & 1u)));
+  for (int i = tid + kHold * kColThreads; i < n; i += kColThreads) {
+    const unsigned y = ents[i].y;
+    atomicAdd(off2 + (y >> 1), 1u << (16 * (y & 1u)));
+  }
+  __syncthreads();
+  // exclusive scan of the counters (low half) and of the occupied slots (high half)
+  const int wper = (nw + kColThreads - 1) / kColThreads;
+  const int w0 = min(tid * wper, nw), w1 = min(w0 + wper, nw);
+  unsigned mine = 0u;
+  for (int w = w0; w < w1; w++) {
+    const unsigned c = off2[w], a = c & 0xFFFFu, b = c >> 16;
+    mine += a + b + ((a ? 0x10000u : 0u) + (b ? 0x10000u : 0u));
+  }
+  int total;
+  unsigned run = (unsigned)block_excl_scan((int)mine, wtot, total);
+  const int nocc = (int)((unsigned)total >> 16);
+  for (int w = w0; w < w1; w++) {
+    const unsigned c = off2[w], a = c & 0xFFFFu, b = c >> 16;
+    const unsigned at = run & 0xFFFFu;
+    off2[w] = at | (at + a) << 16;
+    if (a) { olist[run >> 16] = (unsigned short)(2 * w); run += 0x10000u; }
+    if (b) { olist[run >> 16] = (unsigned short)(2 * w + 1); run += 0x10000u; }
+    run += a + b;
+  }
+  __syncthreads();
+  auto place = [&](uint2 e) {
+    const unsigned sft = 16 * (e.y & 1u);
+    keys[(atomicAdd(off2 + (e.y >> 1), 1u << sft) >> sft) & 0xFFFFu] = e.x;
+  };
+#pragma unroll
+  for (int j = 0; j < kHold; j++)
+    if (tid + j * kColThreads < n) place(held[j]);
+  for (int i = tid + kHold * kColThreads; i < n; i += kColThreads) place(ents[i]);
+  __syncthreads();
+  // now ends[slot] is one past the slot's last key, and the slot's first key
+  // follows the previous slot's last
+
+  // per-thread sums over at most H*G columns of |value| <= 2 * grid: int32
+  int a_vo = 0, a_vss = 0, a_tc = 0, a_avss = 0, a_atc = 0, a_ent = 0;
+  int bx0 = INT_MAX, by0 = INT_MAX, bx1 = -1, by1 = -1;
+  const bool dump = (o == p.dump_slot) && p.dump_cols != nullptr;
+  const bool last_px = bed || dump;      // someone reads the columns' last pixels
+  unsigned* const fv = p.foldp + (size_t)o * p.G * p.G + (size_t)xs0 * p.G;
+  short* const ftc = p.foldtc ? p.foldtc + (size_t)o * p.G * p.G + (size_t)xs0 * p.G : nullptr;
+  // the fold record, sums and bed flags of column l (occupied slot ls)
+  auto store = [&](int l, int ls, const ColOut& c) {
+    const int lim = p.fold_lim;
+    if (max(max((unsigned)(c.vo + lim), (unsigned)(c.vss + lim)), (unsigned)(c.tc + lim)) <= 2u * (unsigned)lim) {
+      fv[l] = __byte_perm(c.vo, c.vss, 0x5410);
+      if (ftc) ftc[l] = (short)c.tc;   // tc is zero with explicit support
+    } else {
+      fv[l] = kFoldEscaped;
+      if (ftc) ftc[l] = 0;
+      const int k = atomicAdd(p.foldxn, 1);
+      if (k < kFoldEscapes) p.foldx[k] = FoldEscape{o, xs0 * p.G + l, c.vo, c.vss, c.tc, 0, 0, 0};
+      else atomicOr(&p.flags[o], kFlagFoldRange);
+    }
+    a_vo += c.vo; a_vss += c.vss; a_tc += c.tc;
+    a_avss += abs(c.vss); a_atc += abs(c.tc);
+    a_ent += c.ndist;
+    if (last_px) {
+      const int gx = xs0 + ls / p.G, gy = ls % p.G;
+      bx0 = min(bx0, gx); bx1 = max(bx1, gx); by0 = min(by0, gy); by1 = max(by1, gy);
+      const int f = bed ? bed_flags(p, c) : 0;
+      if (bed) bedf[ls] = (uint8_t)f;
+      if (dump) {
+        int* d = p.dump_cols + ((size_t)xs0 * p.G + ls) * 8;
+        d[0] = c.ndist; d[1] = c.nfin; d[2] = c.vo; d[3] = c.vss; d[4] = c.tc; d[5] = c.lastz;
+        d[6] = c.lasttype; d[7] = f;
+      }
+    }
+  };
+  // a column's outcome from its last pixel, and the support still open below it
+  auto finish = [&](ColOut& c, bool ex, bool im) {
+    c.nfin = c.ndist;
+    if (ex && c.nfin < kSlotCap) { c.nfin++; c.lastz = 0; c.lasttype = kSSA; }
+    if (im && c.nfin < kSlotCap) { c.nfin++; c.lastz = 0; c.lasttype = kNVA; }
+  };
+
+  // ---- columns of one or two raw pixels, one per thread
+  for (int l0 = wid * 32; l0 < nocc; l0 += kColThreads) {
+    const int l = l0 + lane;
+    int cnt = 0;
+    if (l < nocc) {
+      const int ls = olist[l];
+      const int end = ends[ls], beg = ls ? ends[ls - 1] : 0;
+      cnt = end - beg;
+      if (cnt <= 2) {
+        const unsigned k0 = keys[beg], k1 = keys[end - 1];
+        const unsigned hi = max(k0, k1), lo = min(k0, k1);
+        const int z0 = key_z(hi), n0 = key_nz(hi), z1 = key_z(lo), n1 = key_nz(lo);
+        ColOut c;
+        c.vo = c.vss = c.tc = 0;
+        c.ndist = 1;
+        bool s1 = false, m1 = false;
+        if (hi != lo) {                  // a single distinct pixel is not paired
+          c.ndist = 2;
+          const bool up0 = n0 >= 1, up1 = !up0 && n1 >= 1, dn1 = up0 && n1 <= -1;
+          s1 = dn1 && n1 <= p.nz_ex; m1 = dn1 && n1 >= p.nz_im;
+          const int al = up0 ? z0 : (up1 ? z1 : 0), be = dn1 ? z1 : 0;
+          c.vo = max(al - be, 0);
+          if (p.explicit_ss) c.vss = s1 ? z1 : 0;
+          else { c.tc = al; c.vss = m1 ? 0 : be; }
+          if (last_px) {
+            const int tc = p.explicit_ss ? 0 : kTC;
+            const int t0 = up0 ? kAl | tc : 0, t1 = up1 ? kAl | tc : (dn1 ? kBe | (s1 ? kSSB : 0) | (m1 ? kNVB : 0) : 0);
+            c.lastz = z1; c.lasttype = t1;
+            c.has10 = (z0 == 1 && n0 == 0) || (z1 == 1 && n1 == 0);
+            if (dump) { dump_key(p, xs0 * p.G + ls, 0, hi, t0); dump_key(p, xs0 * p.G + ls, 1, lo, t1); }
+          }
+        } else if (last_px) {
+          c.lastz = z0; c.lasttype = 0;
+          c.has10 = z0 == 1 && n0 == 0;
+          if (dump) dump_key(p, xs0 * p.G + ls, 0, hi, 0);
+        }
+        if (last_px) finish(c, s1, m1);
+        store(l, ls, c);
+      }
+    }
+    const unsigned some = __ballot_sync(full, cnt > 2 && cnt <= 32);
+    if (some) {
+      int at = 0;
+      if (lane == 0) at = atomicAdd(&nlong, __popc(some));
+      at = __shfl_sync(full, at, 0);
+      if (cnt > 2 && cnt <= 32) longq[at + __popc(some & ((1u << lane) - 1u))] = (unsigned short)l;
+    }
+    if (cnt > 32) longq[HG - 1 - atomicAdd(&nbig, 1)] = (unsigned short)l;
+  }
+  __syncthreads();
+
+  // ---- columns of 3 to 32 raw pixels: whole columns side by side in a warp's lanes
+  {
+    const int share = (nlong + kColThreads / 32 - 1) / (kColThreads / 32);
+    const int q1 = min((wid + 1) * share, nlong);
+    const PairCarry none = {false, false, false, false};
+    for (int q0 = wid * share; q0 < q1; q0 += 32) {
+      // lane i: the i-th column of this batch
+      int l = 0, ls = 0, beg = 0, cnt = 0;
+      if (q0 + lane < q1) {
+        l = longq[q0 + lane];
+        ls = olist[l];
+        beg = ls ? ends[ls - 1] : 0;
+        cnt = ends[ls] - beg;
+      }
+      int cum = cnt;
+      for (int d = 1; d < 32; d <<= 1) {
+        const int y = __shfl_up_sync(full, cum, d);
+        if (lane >= d) cum += y;
+      }
+      const int all = __shfl_sync(full, cum, 31);
+      int base = 0;                      // pixels already resolved
+      while (base < all) {
+        const bool in = cnt > 0 && cum - cnt >= base && cum - base <= 32;
+        const unsigned heads = __reduce_or_sync(full, in ? 1u << (cum - cnt - base) : 0u);
+        const int width = __reduce_max_sync(full, in ? cum - base : 0);
+        const int c0 = __ffs(__ballot_sync(full, in)) - 1;   // its first column
+        const bool active = lane < width;
+        const unsigned upto = heads & (0xFFFFFFFFu >> (31 - lane));
+        const int col = c0 + __popc(upto) - 1;
+        const int hs = 31 - __clz(upto);
+        const int len = __shfl_sync(full, cnt, col);
+        const int src = __shfl_sync(full, beg, col) + lane - hs;
+        const unsigned seg = active ? (len == 32 ? full : ((1u << len) - 1u) << hs) : 0u;
+        const unsigned key = active ? keys[src] : 0u;
+        // rank within the column, equal keys in their present order
+        const int maxlen = __reduce_max_sync(full, active ? len : 0);
+        int rank = 0;
+        for (int k = 0; k < maxlen; k++) {
+          const unsigned x = __shfl_sync(full, key, hs + k);
+          rank += k < len && (x > key || (x == key && hs + k < lane));
+        }
+        if (active) scr[hs + rank] = key;
+        __syncwarp();
+        const unsigned sk = active ? scr[lane] : 0u;
+        const bool distinct = active && (lane == hs || scr[lane - 1] != sk);
+        __syncwarp();
+        const unsigned D = __ballot_sync(full, distinct);
+        const int nd = __popc(D & seg);
+        const PairOut r = pair_pixels(p, sk, distinct && nd > 1, seg, none);
+        // column sums: differences of the running sums at the column's ends
+        int vo = r.vo, vss = r.vss, tc = r.tc;
+        for (int d = 1; d < 32; d <<= 1) {
+          const int y0 = __shfl_up_sync(full, vo, d), y1 = __shfl_up_sync(full, vss, d);
+          if (lane >= d) { vo += y0; vss += y1; }
+        }
+        if (!p.explicit_ss)
+          for (int d = 1; d < 32; d <<= 1) {
+            const int y = __shfl_up_sync(full, tc, d);
+            if (lane >= d) tc += y;
+          }
+        const int hp = max(hs - 1, 0);
+        const int vo0 = __shfl_sync(full, vo, hp), vss0 = __shfl_sync(full, vss, hp), tc0 = __shfl_sync(full, tc, hp);
+        ColOut c;
+        c.vo = hs ? vo - vo0 : vo; c.vss = hs ? vss - vss0 : vss; c.tc = hs ? tc - tc0 : tc;
+        base += width;
+        const int cl = __shfl_sync(full, l, col), cls = __shfl_sync(full, ls, col);
+        c.vo = max(c.vo, 0);
+        c.ndist = nd;
+        if (last_px) {
+          const unsigned ds = D & seg;
+          const int lp = ds ? 31 - __clz(ds) : 0;
+          const int z = key_z(sk);
+          const unsigned ten = __ballot_sync(full, distinct && z == 1 && key_nz(sk) == 0);
+          c.lastz = __shfl_sync(full, z, lp);
+          c.lasttype = __shfl_sync(full, r.type, lp);
+          c.has10 = (ten & seg) != 0u;
+          const unsigned kept = (r.ka | r.kb) & seg;
+          const int lk = kept ? 31 - __clz(kept) : 0;
+          const bool open = kept && ((r.kb >> lk) & 1u);
+          const unsigned im = __ballot_sync(full, (r.type & kNVB) != 0);
+          finish(c, open && ((r.s >> lk) & 1u), open && ((im >> lk) & 1u));
+          if (dump && distinct) dump_key(p, xs0 * p.G + cls, __popc(ds & ((1u << lane) - 1u)), sk, r.type);
+        }
+        if (active && lane == hs + len - 1) store(cl, cls, c);
+        __syncwarp();
+      }
+    }
+  }
+  // ---- longer columns, one per warp
+  for (int b = wid; b < nbig; b += kColThreads / 32) {
+    const int l = longq[HG - 1 - b];
+    const int ls = olist[l];
+    const int beg = ls ? ends[ls - 1] : 0, cnt = ends[ls] - beg;
+    ColOut c;
+    c.vo = c.vss = c.tc = 0; c.nfin = c.lastz = c.lasttype = c.has10 = 0;
+    c.ndist = 0;
+    bool ex = false, im = false;
+    int al = 0, vss = 0, tc = 0;
+    const int gslot = xs0 * p.G + ls;
+    if (cnt <= kLongKeys) {
+      unsigned kk[kLongKeys / 32];
+      int rk[kLongKeys / 32];
+#pragma unroll
+      for (int j = 0; j < kLongKeys / 32; j++) {
+        kk[j] = lane + 32 * j < cnt ? keys[beg + lane + 32 * j] : 0u;
+        rk[j] = 0;
+      }
+      for (int i = 0; i < cnt; i++) {
+        const unsigned x = keys[beg + i];
+#pragma unroll
+        for (int j = 0; j < kLongKeys / 32; j++) rk[j] += x > kk[j] || (x == kk[j] && i < lane + 32 * j);
+      }
+#pragma unroll
+      for (int j = 0; j < kLongKeys / 32; j++)
+        if (lane + 32 * j < cnt) scr[rk[j]] = kk[j];
+      __syncwarp();
+      int nd = 0;
+      for (int i = 0; i < cnt; i += 32) {
+        const int k = i + lane;
+        nd += __popc(__ballot_sync(full, k < cnt && (k == 0 || scr[k - 1] != scr[k])));
+      }
+      c.ndist = nd;
+      if (nd > kSlotCap) {               // first-come order decides which keys survive
+        if (lane == 0) atomicOr(&sflag, kFlagCap);
+        continue;
+      }
+      PairCarry cy = {false, false, false, false};
+      int done = 0;
+      for (int i = 0; i < cnt; i += 32) {
+        const int k = i + lane;
+        const unsigned key = k < cnt ? scr[k] : 0u;
+        const bool distinct = k < cnt && (k == 0 || scr[k - 1] != key);
+        const PairOut r = pair_pixels(p, key, distinct && nd > 1, full, cy);
+        al += __reduce_add_sync(full, r.vo);
+        vss += __reduce_add_sync(full, r.vss);
+        tc += __reduce_add_sync(full, r.tc);
+        const int z = key_z(key), nz = key_nz(key);
+        const unsigned A = __ballot_sync(full, distinct && nz >= 1), B = __ballot_sync(full, distinct && nz <= -1);
+        const unsigned N = __ballot_sync(full, (r.type & kNVB) != 0), D = __ballot_sync(full, distinct);
+        if (A | B) cy.al = A > B;        // the higher lane's face
+        if (r.kb) {
+          const int lb = 31 - __clz(r.kb);
+          cy.s = (r.s >> lb) & 1u; cy.n = (N >> lb) & 1u;
+        }
+        cy.first = cy.first || r.ka;
+        if (r.ka | r.kb) {
+          const bool dn = r.kb > r.ka;
+          ex = dn && cy.s; im = dn && cy.n;
+        }
+        if (last_px) {
+          if (__ballot_sync(full, distinct && z == 1 && nz == 0)) c.has10 = 1;
+          if (D) {
+            const int lp = 31 - __clz(D);
+            c.lastz = __shfl_sync(full, z, lp);
+            c.lasttype = __shfl_sync(full, r.type, lp);
+          }
+          if (dump && distinct) dump_key(p, gslot, done + __popc(D & ((1u << lane) - 1u)), key, r.type);
+          done += __popc(D);
+        }
+      }
+      c.vo = max(al, 0); c.vss = vss; c.tc = tc;
+    } else {
+      // a very long list: its distinct keys in descending order, one at a time
+      ColState st;
+      col_init(st);
+      unsigned long long prev = 0x100000000ull;
+      for (;;) {
+        unsigned best = 0u;
+        bool any = false;
+        for (int i = lane; i < cnt; i += 32) {
+          const unsigned key = keys[beg + i];
+          if ((unsigned long long)key < prev) { any = true; best = max(best, key); }
+        }
+        if (!__any_sync(full, any)) break;
+        best = __reduce_max_sync(full, best);
+        if (c.ndist == kSlotCap) { c.ndist++; break; }
+        const int t = col_step(st, key_z(best), key_nz(best), p.thr, p.explicit_ss);
+        if (dump && lane == 0) dump_key(p, gslot, c.ndist, best, t);
+        prev = best;
+        c.ndist++;
+      }
+      if (c.ndist > kSlotCap) {
+        if (lane == 0) atomicOr(&sflag, kFlagCap);
+        continue;
+      }
+      c.lastz = st.lastz; c.lasttype = st.lasttype; c.has10 = st.has10;
+      if (c.ndist == 1) {                // duplicates of a single key
+        c.lasttype = 0;
+        if (dump && lane == 0 && p.dump_types) p.dump_types[(size_t)gslot * 64] = 0;
+      } else {
+        ex = st.ex; im = st.im;
+        c.vo = max(st.al - st.be, 0);
+        c.vss = p.explicit_ss ? (st.ssb - st.ssa) : (-st.al + st.be + st.tc - st.nvb + st.nva);
+        c.tc = st.tc;
+      }
+    }
+    if (last_px) finish(c, ex, im);
+    if (lane == 0) store(l, ls, c);
+    __syncwarp();
+  }
+
+  // ---- reductions
+  const int vals[6] = {a_vo, a_vss, a_tc, a_avss, a_atc, a_ent};
+#pragma unroll
+  for (int k = 0; k < 6; k++) {
+    const int v = __reduce_add_sync(full, vals[k]);
+    if (lane == 0) red[wid][k] = v;
+  }
+  if (last_px) {
+    bx0 = __reduce_min_sync(full, bx0); by0 = __reduce_min_sync(full, by0);
+    bx1 = __reduce_max_sync(full, bx1); by1 = __reduce_max_sync(full, by1);
+  }
+  __syncthreads();
+  if (tid == 0 && sflag) atomicOr(&p.flags[o], sflag);
+  if (sflag & kFlagRedo) return;
+  if (bed && lane == 0 && bx1 >= 0) {
+    atomicMin(&p.bbox[o * 4 + 0], bx0); atomicMin(&p.bbox[o * 4 + 1], by0);
+    atomicMax(&p.bbox[o * 4 + 2], bx1); atomicMax(&p.bbox[o * 4 + 3], by1);
+  }
+  if (tid < 7) {
+    long long v = 0;
+    if (tid < 6) for (int w = 0; w < kColThreads / 32; w++) v += red[w][tid];
+    else v = nocc;
+    const int to = tid < 5 ? tid : (tid == 5 ? (int)kAccEntries : (int)kAccColumns);
+    if (v != 0) atomicAdd((unsigned long long*)&p.acc[(size_t)o * kAccLanes + to], (unsigned long long)v);
+    // strip sums for the fold: |column value| <= 2 * grid, so a strip sum fits in int32
+    if (tid < 5) p.foldmeta[((size_t)o * p.S + s) * 8 + tid] = (int)v;
+  }
+  if (tid == 0) p.foldcnt[(size_t)o * p.S + s] = nocc;
 }
 
 // ---------------------------------------------------------------- K4 bed
@@ -1845,7 +2187,7 @@ __global__ void __launch_bounds__(256) k_bed(EngineParams p)
 // STomoSh_INT3.cpp:375-392) and Vtc (Calculate, :1237) in float32 over
 // columns in ascending slot order.  A float32 fold of integers is exact while
 // every partial sum stays within 2^24 in magnitude.  The per-strip exact sums
-// and absolute sums written by k_strip bound every partial sum inside a
+// and absolute sums written by k_columns or k_strip bound every partial sum inside a
 // strip, so whole strips are skipped exactly until the first strip where the
 // bound could pass 2^24; from there the fold is replayed value by value in
 // slot order: warps 1-3 unpack the next piece of fold records (and any
@@ -2011,9 +2353,9 @@ __global__ void __launch_bounds__(256) k_dump_gather(const int* cols8, const uns
 
 namespace tomo {
 
-// Largest dynamic shared-memory budget that keeps four normal strip CTAs
-// resident per SM (the kernel's registers are bounded for four), or 0.
-size_t strip_four_per_sm_budget()
+// Largest dynamic shared-memory budget that keeps kColBlocks k_columns CTAs
+// resident per SM (its registers are bounded for as many), or 0.
+size_t strip_default_budget()
 {
   static size_t cache[64];
   int dev = 0, per_sm = 0, reserved = 0;
@@ -2022,16 +2364,16 @@ size_t strip_four_per_sm_budget()
   cudaFuncAttributes fa;
   if (cudaDeviceGetAttribute(&per_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev) != cudaSuccess ||
       cudaDeviceGetAttribute(&reserved, cudaDevAttrReservedSharedMemoryPerBlock, dev) != cudaSuccess ||
-      cudaFuncGetAttributes(&fa, k_strip<0>) != cudaSuccess)
+      cudaFuncGetAttributes(&fa, k_columns) != cudaSuccess)
     return 0;
-  const long long per_cta = per_sm / 4 / 128 * 128 - reserved - (long long)fa.sharedSizeBytes;
+  const long long per_cta = per_sm / kColBlocks / 128 * 128 - reserved - (long long)fa.sharedSizeBytes;
   cache[dev] = per_cta > 0 ? (size_t)per_cta / 128 * 128 : 0;
   return cache[dev];
 }
 
 size_t strip_smem_bytes(int mode, int H, int G, int ent_cap)
 {
-  return strip_smem_layout(mode, H, G, ent_cap);
+  return mode == 0 ? columns_smem(H * G, ent_cap) : strip_smem_layout(H, G, ent_cap);
 }
 
 // The strip kernels' dynamic shared-memory limit only ever rises (per
@@ -2045,7 +2387,7 @@ cudaError_t configure_kernels(size_t normal_smem, size_t safe_smem, size_t prio_
   if (e != cudaSuccess) return e;
   if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
   if (normal_smem > conf[dev][0]) {
-    e = cudaFuncSetAttribute(k_strip<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)normal_smem);
+    e = cudaFuncSetAttribute(k_columns, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)normal_smem);
     if (e != cudaSuccess) return e;
     conf[dev][0] = normal_smem;
   }
@@ -2145,7 +2487,7 @@ cudaError_t launch_fill(const EngineParams& p, cudaStream_t s, LaunchLog* L)
 cudaError_t launch_strip_bed(const EngineParams& p, cudaStream_t main, size_t strip_smem, LaunchLog* L)
 {
   const int kind = p.variant == 0 ? kKStrip : kKStripRedo;
-  if (p.mode == 0) TOMO_LAUNCH(kind, main, (k_strip<0><<<dim3(p.S, p.Bo), 256, strip_smem, main>>>(p)));
+  if (p.mode == 0) TOMO_LAUNCH(kind, main, (k_columns<<<dim3(p.S, p.Bo), kColThreads, strip_smem, main>>>(p)));
   else if (p.mode == 2) TOMO_LAUNCH(kind, main, (k_strip<2><<<dim3(p.S, p.Bo), 256, strip_smem, main>>>(p)));
   else TOMO_LAUNCH(kind, main, (k_strip<1><<<dim3(p.S, p.Bo), 256, strip_smem, main>>>(p)));
   TOMO_LAUNCH(kKBed, main, (k_bed<<<dim3(8, p.Bo), 256, 0, main>>>(p)));
