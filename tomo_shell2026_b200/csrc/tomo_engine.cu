@@ -2423,15 +2423,14 @@ int tomoMlpPredict(const float* x, int n, float* out)
   if (!g_mlp) return set_error(TOMO_ERR_ARG, "tomoMlpInit was not called");
   if (n <= 0 || x == nullptr || out == nullptr) return set_error(TOMO_ERR_ARG, "bad prediction arguments");
   Engine& E = engine();
-  DevBuf<float> dx, dy;
+  DevBuf<float>& dx = E.srch_x;   // the searches' buffers: a call that frees its own waits for the whole device
+  DevBuf<float>& dy = E.srch_y;
   TOMO_CUDA(dx.reserve((size_t)n * kMlpIn));
   TOMO_CUDA(dy.reserve((size_t)n));
   TOMO_CUDA(cudaMemcpyAsync(dx.ptr, x, sizeof(float) * n * kMlpIn, cudaMemcpyHostToDevice, E.main));
   TOMO_CUDA(mlp().predict_device(dx.ptr, n, dy.ptr, E.main));
   TOMO_CUDA(cudaMemcpyAsync(out, dy.ptr, sizeof(float) * n, cudaMemcpyDeviceToHost, E.main));
   TOMO_CUDA(cudaStreamSynchronize(E.main));
-  dx.release();
-  dy.release();
   return 0;
 }
 

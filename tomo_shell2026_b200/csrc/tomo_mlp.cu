@@ -2,15 +2,22 @@
 //
 // The network is small (33,793 parameters, 128-wide), and the training set
 // is a coarse orientation grid (~10^3 samples), so a step is latency-bound,
-// not FLOP-bound.  The design keeps a step to two launches:
+// not FLOP-bound.  A step is two launches:
 //
-//   k_mlp_block    one CTA per 16 samples: forward pass (activations in
-//                  shared memory), loss, backward pass, and that block's
-//                  gradient for every parameter written to its own row of a
-//                  partial-gradient buffer;
-//   k_mlp_reduce   one thread per parameter: the blocks' gradients summed in
-//                  block order (deterministic), optionally followed by the
-//                  Adam update of the parameter and of its transposed copy.
+//   k_mlp_pass     one CTA per 8 samples: forward pass, loss and the whole
+//                  backward pass to the layers' inputs out of shared memory;
+//                  activations and pre-activation gradients go to global
+//                  memory (3 MB for 936 samples);
+//   k_mlp_update   one CTA per 16 x 16 weights (and per 32 of the rest): the
+//                  weight gradient over all samples, then the Adam update of
+//                  the parameter and of its transposed copy.
+//
+// The gradient is summed in a fixed order (deterministic): over each 8 samples
+// in turn, the sums of eights r, r + 8, r + 16, ... of each r in 0..7, then the
+// eight of those.  When each CTA wrote its own gradient of all parameters and a
+// second kernel added them up (16 MB written and read a step), a step of 936
+// samples took 31 us; now 21 (B200, 300 steps replayed as a graph), most of it
+// the latency of four dependent 128-term sums and three activations.
 //
 // Weights are row-major [in][out]; the backward pass reads each matrix
 // through a transposed copy [out][in] kept in step with the parameters, so
@@ -27,232 +34,312 @@ namespace tomo {
 
 namespace {
 
-constexpr int kSB = 8;           // samples per CTA
-constexpr int kQ = kSB / 2;      // samples per thread (two groups of 128 threads)
-constexpr int kThreads = 256;
+constexpr int kSB = 8;           // samples per k_mlp_pass CTA and per partial gradient sum
+constexpr int kFB = 64;          // samples per k_mlp_forward CTA and turn, eight per warp
 constexpr int kH = kMlpHidden;   // 128
-static_assert(kThreads == 2 * kH, "thread mapping assumes two groups of 128");
-static_assert(kSB % 8 == 0 && kSB <= 32, "the output layer gives each of the 8 warps kSB / 8 samples");
+constexpr int kParts = 8;        // partial gradient sums per parameter
 
-// Padded row length of the partial-gradient buffer.
-__host__ __device__ inline int part_stride(int total) { return (total + 31) / 32 * 32; }
+__device__ __forceinline__ void cp16(void* smem, const void* g)
+{
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(smem)), "l"(g));
+}
+__device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;"); }
+template <int N>
+__device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N)); }
 
-struct alignas(16) Shared {
-  float w[kH * kH];          // the 128 x 128 weight matrix in use (W or its transpose)
+// Start copying one 128 x 128 matrix into shared memory (one commit group).
+__device__ __forceinline__ void stage(const float* __restrict__ src, float* dst)
+{
+  for (int k = threadIdx.x; k < kH * kH / 4; k += blockDim.x) cp16(dst + 4 * k, src + 4 * k);
+  cp_commit();
+}
+
+// a * w + c for two samples, each rounded once as __fmaf_rn rounds it.
+__device__ __forceinline__ float2 fma2(float2 a, float2 w, float2 c)
+{
+  float2 r;
+  asm("{.reg .b64 a, w, c, r;\n\tmov.b64 a, {%2, %3};\n\tmov.b64 w, {%4, %5};\n\tmov.b64 c, {%6, %7};\n\t"
+      "fma.rn.f32x2 r, a, w, c;\n\tmov.b64 {%0, %1}, r;}"
+      : "=f"(r.x), "=f"(r.y) : "f"(a.x), "f"(a.y), "f"(w.x), "f"(w.y), "f"(c.x), "f"(c.y));
+  return r;
+}
+
+// out[j][s] = sum over i (in order, from b[j] or zero) of in[i][s] * W[i][j] for
+// eight samples and 128 units, by the first two warps: a thread has four units
+// x four samples, so that eight shared-memory words serve sixteen products (a
+// thread per unit with all eight samples took nine words for eight products,
+// and shared memory returns 32 words a cycle: 36 cycles per i instead of 16).
+// The next rows are read while these are used.
+__device__ __forceinline__ void matmul8(const float (*in)[kSB], const float* W, const float* b, float (*out)[kSB])
+{
+  constexpr int kRows = 8;
+  if (threadIdx.x >= 64) return;
+  const int j0 = (threadIdx.x & 31) * 4, s0 = (threadIdx.x >> 5) * 4;
+  float2 acc[4][2];
+#pragma unroll
+  for (int c = 0; c < 4; c++) {
+    const float v = b ? b[j0 + c] : 0.f;
+    acc[c][0] = acc[c][1] = make_float2(v, v);
+  }
+  float4 w[2][kRows], a[2][kRows];
+  auto load = [&](int i0, float4* pw, float4* pa) {
+#pragma unroll
+    for (int k = 0; k < kRows; k++) {
+      pw[k] = *reinterpret_cast<const float4*>(W + (i0 + k) * kH + j0);
+      pa[k] = *reinterpret_cast<const float4*>(&in[i0 + k][s0]);
+    }
+  };
+  auto use = [&](const float4* pw, const float4* pa) {
+#pragma unroll
+    for (int k = 0; k < kRows; k++) {
+      const float2 x = make_float2(pa[k].x, pa[k].y), y = make_float2(pa[k].z, pa[k].w);
+      const float wc[4] = {pw[k].x, pw[k].y, pw[k].z, pw[k].w};
+#pragma unroll
+      for (int c = 0; c < 4; c++) {
+        const float2 w2 = make_float2(wc[c], wc[c]);
+        acc[c][0] = fma2(x, w2, acc[c][0]);
+        acc[c][1] = fma2(y, w2, acc[c][1]);
+      }
+    }
+  };
+  load(0, w[0], a[0]);
+#pragma unroll 1
+  for (int i0 = 0; i0 < kH; i0 += 2 * kRows) {
+    load(i0 + kRows, w[1], a[1]);
+    use(w[0], a[0]);
+    if (i0 + 2 * kRows < kH) load(i0 + 2 * kRows, w[0], a[0]);
+    use(w[1], a[1]);
+  }
+#pragma unroll
+  for (int c = 0; c < 4; c++)
+    *reinterpret_cast<float4*>(&out[j0 + c][s0]) = make_float4(acc[c][0].x, acc[c][0].y, acc[c][1].x, acc[c][1].y);
+}
+
+struct alignas(16) PassShared {
+  float w[2][kH * kH];       // the two 128 x 128 matrices in use
+  float a[3][kH][kSB];       // tanh outputs of the three hidden layers, samples innermost
+  float dz[2][kH][kSB];      // pre-activation gradients, ping-pong
+  float mm[kH][kSB];         // a product before its activation
   float x[kSB][kMlpIn];
-  float a[3][kSB][kH];       // tanh outputs of the three hidden layers
-  float dz[2][kSB][kH];      // pre-activation gradients, ping-pong
   float yhat[kSB];
   float dz4[kSB];
 };
-constexpr size_t kSmemBytes = sizeof(Shared);   // ~106 KB: dynamic, opted in
+constexpr size_t kPassSmem = sizeof(PassShared);   // ~153 KB: dynamic, opted in
 
-__device__ __forceinline__ Shared& shared_block()
+// What a pass leaves for the weight gradients: [rows][128] each (rows: samples
+// rounded up to eights), outputs of the hidden layers, gradients before their
+// activations, and the output's gradient [rows].
+struct PassOut {
+  float *a[3], *d[3], *d4;
+};
+
+// One thread per hidden unit and eight samples but for the products (matmul8);
+// rows past the last sample hold zero features and a zero output gradient.
+__global__ void __launch_bounds__(kH) k_mlp_pass(MlpLayout L, const float* __restrict__ P, const float* __restrict__ WT,
+                                                 const float* __restrict__ x, const float* __restrict__ y, int n,
+                                                 PassOut O, float* __restrict__ part_loss)
 {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  return *reinterpret_cast<Shared*>(smem_raw);
-}
-
-// Stage one 128 x 128 matrix into S.w (the caller synchronises).
-__device__ __forceinline__ void stage(const float* __restrict__ src, Shared& S)
-{
-  const float4* s4 = reinterpret_cast<const float4*>(src);
-  float4* d4 = reinterpret_cast<float4*>(S.w);
-  for (int k = threadIdx.x; k < kH * kH / 4; k += blockDim.x) d4[k] = s4[k];
-}
-
-// Forward pass of one block of samples; rows s >= ns hold zero features.
-__device__ void forward_block(const MlpLayout& L, const float* __restrict__ P, Shared& S)
-{
-  const int t = threadIdx.x, j = t & (kH - 1), g = t >> 7;
-  {
-    const float* W = P + L.w[0];
-    const float b = P[L.b[0] + j];
-#pragma unroll
-    for (int q = 0; q < kQ; q++) {
-      const int s = g * kQ + q;
-      float acc = b;
-#pragma unroll
-      for (int i = 0; i < kMlpIn; i++) acc = __fmaf_rn(S.x[s][i], W[i * kH + j], acc);
-      S.a[0][s][j] = tanhf(acc);
-    }
-  }
-  __syncthreads();
-  for (int l = 1; l < 3; l++) {
-    stage(P + L.w[l], S);
-    __syncthreads();
-    const float* W = S.w;
-    float acc[kQ];
-    const float b = P[L.b[l] + j];
-#pragma unroll
-    for (int q = 0; q < kQ; q++) acc[q] = b;
-#pragma unroll 4
-    for (int i = 0; i < kH; i += 4) {
-      const float w0 = W[(i + 0) * kH + j], w1 = W[(i + 1) * kH + j];
-      const float w2 = W[(i + 2) * kH + j], w3 = W[(i + 3) * kH + j];
-#pragma unroll
-      for (int q = 0; q < kQ; q++) {
-        const float4 a = *reinterpret_cast<const float4*>(&S.a[l - 1][g * kQ + q][i]);
-        acc[q] = __fmaf_rn(a.x, w0, acc[q]);
-        acc[q] = __fmaf_rn(a.y, w1, acc[q]);
-        acc[q] = __fmaf_rn(a.z, w2, acc[q]);
-        acc[q] = __fmaf_rn(a.w, w3, acc[q]);
-      }
-    }
-#pragma unroll
-    for (int q = 0; q < kQ; q++) S.a[l][g * kQ + q][j] = tanhf(acc[q]);
-    __syncthreads();
-  }
-  {
-    const float* W = P + L.w[3];
-    const int warp = t >> 5, lane = t & 31;
-    for (int s = warp * (kSB / 8); s < (warp + 1) * (kSB / 8); s++) {
-      float acc = 0.f;
-#pragma unroll
-      for (int k = 0; k < kH / 32; k++) acc = __fmaf_rn(S.a[2][s][lane + 32 * k], W[lane + 32 * k], acc);
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xFFFFFFFFu, acc, o);
-      if (lane == 0) S.yhat[s] = acc + P[L.b[3]];
-    }
-  }
-  __syncthreads();
-}
-
-__device__ void load_x(const float* __restrict__ x, int s0, int ns, Shared& S)
-{
-  for (int k = threadIdx.x; k < kSB * kMlpIn; k += blockDim.x) {
-    const int s = k / kMlpIn, i = k % kMlpIn;
+  PassShared& S = *reinterpret_cast<PassShared*>(smem_raw);
+  const int j = threadIdx.x, warp = j >> 5, lane = j & 31;
+  const int s0 = blockIdx.x * kSB, ns = min(kSB, n - s0);
+  stage(P + L.w[1], S.w[0]);
+  stage(P + L.w[2], S.w[1]);
+  if (j < kSB * kMlpIn) {
+    const int s = j / kMlpIn, i = j % kMlpIn;
     S.x[s][i] = s < ns ? x[(size_t)(s0 + s) * kMlpIn + i] : 0.f;
   }
+  const float w4 = P[L.w[3] + j];
+  float w0[kMlpIn];
+#pragma unroll
+  for (int i = 0; i < kMlpIn; i++) w0[i] = P[L.w[0] + i * kH + j];
+  const float b0 = P[L.b[0] + j];
   __syncthreads();
-}
-
-__global__ void __launch_bounds__(kThreads) k_mlp_forward(MlpLayout L, const float* __restrict__ P,
-                                                          const float* __restrict__ x, int n, float* __restrict__ out)
-{
-  Shared& S = shared_block();
-  const int s0 = blockIdx.x * kSB, ns = min(kSB, n - s0);
-  load_x(x, s0, ns, S);
-  forward_block(L, P, S);
-  if (threadIdx.x < ns) out[s0 + threadIdx.x] = S.yhat[threadIdx.x];
-}
-
-// Forward + MSE + backward of one block; gradient row `blockIdx.x` of `part`.
-__global__ void __launch_bounds__(kThreads) k_mlp_block(MlpLayout L, const float* __restrict__ P,
-                                                        const float* __restrict__ WT, const float* __restrict__ x,
-                                                        const float* __restrict__ y, int n, float* __restrict__ part,
-                                                        float* __restrict__ part_loss)
-{
-  Shared& S = shared_block();
-  const int t = threadIdx.x, j = t & (kH - 1), g = t >> 7;
-  const int s0 = blockIdx.x * kSB, ns = min(kSB, n - s0);
-  float* G = part + (size_t)blockIdx.x * part_stride(L.total);
-  load_x(x, s0, ns, S);
-  forward_block(L, P, S);
+  float v[kSB];
+  // outputs of hidden layer l: shared (samples innermost) and global rows
+  auto put = [&](float (*dst)[kSB], float* g) {
+    *reinterpret_cast<float4*>(&dst[j][0]) = make_float4(v[0], v[1], v[2], v[3]);
+    *reinterpret_cast<float4*>(&dst[j][4]) = make_float4(v[4], v[5], v[6], v[7]);
+#pragma unroll
+    for (int s = 0; s < kSB; s++) g[(size_t)(s0 + s) * kH + j] = v[s];
+  };
+#pragma unroll
+  for (int s = 0; s < kSB; s++) {
+    float acc = b0;
+#pragma unroll
+    for (int i = 0; i < kMlpIn; i++) acc = __fmaf_rn(S.x[s][i], w0[i], acc);
+    v[s] = tanhf(acc);
+  }
+  put(S.a[0], O.a[0]);
+  cp_wait<1>();
+  __syncthreads();
+  matmul8(S.a[0], S.w[0], P + L.b[1], S.mm);
+  __syncthreads();
+#pragma unroll
+  for (int s = 0; s < kSB; s++) v[s] = tanhf(S.mm[j][s]);
+  put(S.a[1], O.a[1]);
+  cp_wait<0>();
+  __syncthreads();
+  stage(WT + L.w[2], S.w[0]);            // [out][in], for the backward pass
+  matmul8(S.a[1], S.w[1], P + L.b[2], S.mm);
+  __syncthreads();
+#pragma unroll
+  for (int s = 0; s < kSB; s++) v[s] = tanhf(S.mm[j][s]);
+  put(S.a[2], O.a[2]);
+  __syncthreads();
+  stage(WT + L.w[1], S.w[1]);
+  for (int s = warp * 2; s < warp * 2 + 2; s++) {
+    float acc = 0.f;
+#pragma unroll
+    for (int k = 0; k < kH / 32; k++) acc = __fmaf_rn(S.a[2][lane + 32 * k][s], P[L.w[3] + lane + 32 * k], acc);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xFFFFFFFFu, acc, o);
+    if (lane == 0) S.yhat[s] = acc + P[L.b[3]];
+  }
+  __syncthreads();
   // loss and output-layer gradient
-  if (t < 32) {
+  if (j < 32) {
     float e = 0.f;
-    if (t < kSB) {
-      const float d = t < ns ? S.yhat[t] - y[s0 + t] : 0.f;
-      S.dz4[t] = 2.f * d / (float)n;
+    if (j < kSB) {
+      const float d = j < ns ? S.yhat[j] - y[s0 + j] : 0.f;
+      S.dz4[j] = 2.f * d / (float)n;
+      O.d4[s0 + j] = S.dz4[j];
       e = d * d / (float)n;
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) e += __shfl_xor_sync(0xFFFFFFFFu, e, o);
-    if (t == 0) part_loss[blockIdx.x] = e;
+    if (j == 0) part_loss[blockIdx.x] = e;
   }
   __syncthreads();
-  // layer 4 (128 -> 1): dW4, db4, dZ3
-  if (t < kH) {
-    float acc = 0.f;
 #pragma unroll
-    for (int s = 0; s < kSB; s++) acc = __fmaf_rn(S.a[2][s][t], S.dz4[s], acc);
-    G[L.w[3] + t] = acc;
+  for (int s = 0; s < kSB; s++) {
+    const float a = S.a[2][j][s];
+    v[s] = S.dz4[s] * w4 * (1.f - a * a);
   }
-  if (t == 0) {
-    float acc = 0.f;
-    for (int s = 0; s < kSB; s++) acc += S.dz4[s];
-    G[L.b[3]] = acc;
-  }
-  {
-    const float w = P[L.w[3] + j];
-#pragma unroll
-    for (int q = 0; q < kQ; q++) {
-      const int s = g * kQ + q;
-      const float a = S.a[2][s][j];
-      S.dz[0][s][j] = S.dz4[s] * w * (1.f - a * a);
-    }
-  }
+  put(S.dz[0], O.d[2]);
+  cp_wait<1>();
   __syncthreads();
-  // hidden layers 3 and 2 (128 -> 128): dZ in dz[cur], layer input a[l-1]
-  int cur = 0;
-  for (int l = 2; l >= 1; l--) {
-    stage(WT + L.w[l], S);   // [out][in]
-    __syncthreads();
-    const float (*A)[kH] = S.a[l - 1];
-    const float (*D)[kH] = S.dz[cur];
+  matmul8(S.dz[0], S.w[0], nullptr, S.mm);
+  __syncthreads();
+#pragma unroll
+  for (int s = 0; s < kSB; s++) {
+    const float a = S.a[1][j][s];
+    v[s] = S.mm[j][s] * (1.f - a * a);
+  }
+  put(S.dz[1], O.d[1]);
+  cp_wait<0>();
+  __syncthreads();
+  matmul8(S.dz[1], S.w[1], nullptr, S.mm);
+  __syncthreads();
+#pragma unroll
+  for (int s = 0; s < kSB; s++) {
+    const float a = S.a[0][j][s];
+    O.d[0][(size_t)(s0 + s) * kH + j] = S.mm[j][s] * (1.f - a * a);
+  }
+}
+
+struct alignas(16) ForwardShared {
+  float w[2][kH * kH];       // both 128 x 128 matrices, loaded once per CTA
+  float a[kH][kFB];          // activations, samples innermost
+  float x[kFB][kMlpIn];
+};
+constexpr size_t kForwardSmem = sizeof(ForwardShared);   // ~161 KB: dynamic, opted in
+
+// Prediction: persistent CTAs, tiles of 64 samples; a thread has four units
+// x eight samples (twelve shared-memory words for 32 products, which bound this
+// kernel too).  Every output is summed in the order of the training pass.
+// 87,120 samples in 195 us (a CTA per 8 samples, loading both matrices each
+// time, and nine words for eight products: about 400).
+__global__ void __launch_bounds__(256) k_mlp_forward(MlpLayout L, const float* __restrict__ P,
+                                                     const float* __restrict__ x, int n, float* __restrict__ out)
+{
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  ForwardShared& S = *reinterpret_cast<ForwardShared*>(smem_raw);
+  const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
+  const int j0 = lane * 4, g = warp * 8;   // units j0 .. j0 + 3, samples g .. g + 7
+  stage(P + L.w[1], S.w[0]);
+  stage(P + L.w[2], S.w[1]);
+  float4 w0[kMlpIn], b[3];
+#pragma unroll
+  for (int i = 0; i < kMlpIn; i++) w0[i] = *reinterpret_cast<const float4*>(P + L.w[0] + i * kH + j0);
+#pragma unroll
+  for (int l = 0; l < 3; l++) b[l] = *reinterpret_cast<const float4*>(P + L.b[l] + j0);
+  float w3[kH / 32];
+#pragma unroll
+  for (int k = 0; k < kH / 32; k++) w3[k] = P[L.w[3] + lane + 32 * k];
+  const float b3 = P[L.b[3]];
+  cp_wait<0>();
+  __syncthreads();
+  // a warp's eight samples never leave it: no barrier from here on
+  for (int s0 = (blockIdx.x * (kFB / 8) + warp) * 8; s0 < n; s0 += gridDim.x * kFB) {
+    const int ns = min(8, n - s0);
     {
-      float d[kSB];
+      const int s = lane / kMlpIn, i = lane % kMlpIn;
+      S.x[g + s][i] = s < ns ? x[(size_t)(s0 + s) * kMlpIn + i] : 0.f;
+    }
+    __syncwarp();
+    float v[4][8];
+    auto put = [&](float (*to)[kFB]) {
 #pragma unroll
-      for (int s = 0; s < kSB; s++) d[s] = D[s][j];
-#pragma unroll 4
-      for (int k = 0; k < kH / 2; k++) {
-        const int i = g + 2 * k;
-        float acc = 0.f;
+      for (int c = 0; c < 4; c++)
 #pragma unroll
-        for (int s = 0; s < kSB; s++) acc = __fmaf_rn(A[s][i], d[s], acc);
-        G[L.w[l] + i * kH + j] = acc;
+        for (int q = 0; q < 2; q++)
+          *reinterpret_cast<float4*>(&to[j0 + c][g + 4 * q]) =
+              make_float4(tanhf(v[c][4 * q]), tanhf(v[c][4 * q + 1]), tanhf(v[c][4 * q + 2]), tanhf(v[c][4 * q + 3]));
+    };
+#pragma unroll
+    for (int s = 0; s < 8; s++) {
+      float4 acc = b[0];
+#pragma unroll
+      for (int i = 0; i < kMlpIn; i++) {
+        const float xi = S.x[g + s][i];
+        acc.x = __fmaf_rn(xi, w0[i].x, acc.x); acc.y = __fmaf_rn(xi, w0[i].y, acc.y);
+        acc.z = __fmaf_rn(xi, w0[i].z, acc.z); acc.w = __fmaf_rn(xi, w0[i].w, acc.w);
       }
+      v[0][s] = acc.x; v[1][s] = acc.y; v[2][s] = acc.z; v[3][s] = acc.w;
     }
-    if (t < kH) {
-      float acc = 0.f;
+    put(S.a);
+    __syncwarp();
 #pragma unroll
-      for (int s = 0; s < kSB; s++) acc += D[s][t];
-      G[L.b[l] + t] = acc;
-    }
-    {
-      const float* Wt = S.w;
-      const int i = j;
-      float acc[kQ];
+    for (int l = 1; l < 3; l++) {
+      const float* W = S.w[l - 1];
+      const float bb[4] = {b[l].x, b[l].y, b[l].z, b[l].w};
+      float2 acc[4][4];
 #pragma unroll
-      for (int q = 0; q < kQ; q++) acc[q] = 0.f;
+      for (int c = 0; c < 4; c++)
+#pragma unroll
+        for (int q = 0; q < 4; q++) acc[c][q] = make_float2(bb[c], bb[c]);
 #pragma unroll 4
-      for (int o = 0; o < kH; o += 4) {
-        const float w0 = Wt[(o + 0) * kH + i], w1 = Wt[(o + 1) * kH + i];
-        const float w2 = Wt[(o + 2) * kH + i], w3 = Wt[(o + 3) * kH + i];
+      for (int i = 0; i < kH; i++) {
+        const float4 w = *reinterpret_cast<const float4*>(W + i * kH + j0);
+        const float4 a0 = *reinterpret_cast<const float4*>(&S.a[i][g]), a1 = *reinterpret_cast<const float4*>(&S.a[i][g + 4]);
+        const float wc[4] = {w.x, w.y, w.z, w.w};
 #pragma unroll
-        for (int q = 0; q < kQ; q++) {
-          const float4 d = *reinterpret_cast<const float4*>(&D[g * kQ + q][o]);
-          acc[q] = __fmaf_rn(d.x, w0, acc[q]);
-          acc[q] = __fmaf_rn(d.y, w1, acc[q]);
-          acc[q] = __fmaf_rn(d.z, w2, acc[q]);
-          acc[q] = __fmaf_rn(d.w, w3, acc[q]);
+        for (int c = 0; c < 4; c++) {
+          const float2 w2 = make_float2(wc[c], wc[c]);
+          acc[c][0] = fma2(make_float2(a0.x, a0.y), w2, acc[c][0]);
+          acc[c][1] = fma2(make_float2(a0.z, a0.w), w2, acc[c][1]);
+          acc[c][2] = fma2(make_float2(a1.x, a1.y), w2, acc[c][2]);
+          acc[c][3] = fma2(make_float2(a1.z, a1.w), w2, acc[c][3]);
         }
       }
 #pragma unroll
-      for (int q = 0; q < kQ; q++) {
-        const float a = A[g * kQ + q][i];
-        S.dz[cur ^ 1][g * kQ + q][i] = acc[q] * (1.f - a * a);
-      }
+      for (int c = 0; c < 4; c++)
+#pragma unroll
+        for (int q = 0; q < 4; q++) { v[c][2 * q] = acc[c][q].x; v[c][2 * q + 1] = acc[c][q].y; }
+      __syncwarp();
+      put(S.a);
+      __syncwarp();
     }
-    __syncthreads();
-    cur ^= 1;
-  }
-  // layer 1 (4 -> 128)
-  {
-    const float (*D)[kH] = S.dz[cur];
-    for (int i = g; i < kMlpIn; i += 2) {
+    for (int s = 0; s < 8; s++) {
       float acc = 0.f;
 #pragma unroll
-      for (int s = 0; s < kSB; s++) acc = __fmaf_rn(S.x[s][i], D[s][j], acc);
-      G[L.w[0] + i * kH + j] = acc;
-    }
-    if (t < kH) {
-      float acc = 0.f;
+      for (int k = 0; k < kH / 32; k++) acc = __fmaf_rn(S.a[lane + 32 * k][g + s], w3[k], acc);
 #pragma unroll
-      for (int s = 0; s < kSB; s++) acc += D[s][t];
-      G[L.b[0] + t] = acc;
+      for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xFFFFFFFFu, acc, o);
+      if (lane == 0 && s < ns) out[s0 + s] = acc + b3;
     }
+    __syncwarp();
   }
 }
 
@@ -281,37 +368,133 @@ __device__ __forceinline__ void adam_update(const MlpLayout& L, int p, float gi,
   if (q >= 0) WT[q] = np;
 }
 
-// grad[p] = sum over blocks (fixed order); loss likewise; optional Adam.
-// Block (32 parameters) x (8 lanes over the partial rows): lane r sums rows
-// r, r + 8, ...; the 8 lane sums are then added in lane order.
-__global__ void __launch_bounds__(256) k_mlp_reduce(MlpLayout L, const float* __restrict__ part,
-                                                    const float* __restrict__ part_loss, int nblk,
-                                                    float* __restrict__ grad, float* __restrict__ loss, int update,
-                                                    float* P, float* WT, float* m, float* v, float lr, float bc1,
-                                                    float bc2)
+constexpr int kTile = 16;                                       // 16 x 16 weights per CTA
+constexpr int kTilesPerLayer = (kH / kTile) * (kH / kTile);     // 64
+constexpr int kSmallPer = 32;                                   // other parameters per CTA
+
+// The parameters outside the two 128 x 128 matrices, numbered 0 .. kSmall - 1:
+// W1, b1, b2, b3, W4, b4.
+constexpr int kSmall = kMlpIn * kH + 3 * kH + kH + 1;
+
+// Weight gradients and (update) the Adam step.  Warp r of a CTA sums the
+// partial gradients of the eights r, r + 8, ... (each eight in sample order);
+// the eight sums are then added in order.  nblk: eights of samples.
+__global__ void __launch_bounds__(32 * kParts) k_mlp_update(MlpLayout L, const float* __restrict__ x, PassOut O,
+                                                            const float* __restrict__ part_loss, int nblk,
+                                                            float* __restrict__ grad, float* __restrict__ loss,
+                                                            int update, float* P, float* WT, float* m, float* v,
+                                                            float lr, float bc1, float bc2)
 {
-  __shared__ float red[8][33];
-  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-  const int p = blockIdx.x * 32 + tx;
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
+  __shared__ float red[kParts][kTile * kTile + 1];
+  const int lane = threadIdx.x & 31, r = threadIdx.x >> 5;
+  const int tile = blockIdx.x;
+  if (tile < 2 * kTilesPerLayer) {
+    // 16 x 16 weights of layer l: a thread has 2 inputs x 4 outputs
+    const int l = 1 + tile / kTilesPerLayer, q = tile % kTilesPerLayer;
+    const int i0 = q / (kH / kTile) * kTile + (lane >> 2) * 2, j0 = q % (kH / kTile) * kTile + (lane & 3) * 4;
+    const float* A = O.a[l - 1] + i0;
+    const float* D = O.d[l] + j0;
+    float acc[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
+    float2 a[kSB], an[kSB];
+    float4 d[kSB], dn[kSB];
+    auto load = [&](int b, float2* pa, float4* pd) {
+#pragma unroll
+      for (int s = 0; s < kSB; s++) {
+        pa[s] = *reinterpret_cast<const float2*>(A + (size_t)(b * kSB + s) * kH);
+        pd[s] = *reinterpret_cast<const float4*>(D + (size_t)(b * kSB + s) * kH);
+      }
+    };
+    if (r < nblk) load(r, a, d);
+    for (int b = r; b < nblk; b += kParts) {
+      if (b + kParts < nblk) load(b + kParts, an, dn);   // the next eight, while this one is summed
+      float p[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
+#pragma unroll
+      for (int s = 0; s < kSB; s++) {
+        p[0][0] = __fmaf_rn(a[s].x, d[s].x, p[0][0]); p[0][1] = __fmaf_rn(a[s].x, d[s].y, p[0][1]);
+        p[0][2] = __fmaf_rn(a[s].x, d[s].z, p[0][2]); p[0][3] = __fmaf_rn(a[s].x, d[s].w, p[0][3]);
+        p[1][0] = __fmaf_rn(a[s].y, d[s].x, p[1][0]); p[1][1] = __fmaf_rn(a[s].y, d[s].y, p[1][1]);
+        p[1][2] = __fmaf_rn(a[s].y, d[s].z, p[1][2]); p[1][3] = __fmaf_rn(a[s].y, d[s].w, p[1][3]);
+      }
+#pragma unroll
+      for (int h = 0; h < 2; h++)
+#pragma unroll
+        for (int c = 0; c < 4; c++) acc[h][c] += p[h][c];
+#pragma unroll
+      for (int s = 0; s < kSB; s++) { a[s] = an[s]; d[s] = dn[s]; }
+    }
+#pragma unroll
+    for (int h = 0; h < 2; h++)
+#pragma unroll
+      for (int c = 0; c < 4; c++) red[r][((lane >> 2) * 2 + h) * kTile + (lane & 3) * 4 + c] = acc[h][c];
+    __syncthreads();
+    const int t = threadIdx.x;   // one weight per thread
+    float gi = 0.f;
+#pragma unroll
+    for (int k = 0; k < kParts; k++) gi += red[k][t];
+    const int w = L.w[l] + (q / (kH / kTile) * kTile + t / kTile) * kH + q % (kH / kTile) * kTile + t % kTile;
+    grad[w] = gi;
+    if (update) adam_update(L, w, gi, P, WT, m, v, lr, bc1, bc2);
+    return;
+  }
+  // the rest: lane = parameter, warp = partial sum
+  const int k = (tile - 2 * kTilesPerLayer) * kSmallPer + lane;
+  int par = -1;
+  float acc = 0.f;
+  if (k < kSmall) {
+    int e = k;
+    if (e < kMlpIn * kH) {
+      par = L.w[0] + e;
+      const int i = e / kH, j = e % kH;
+      for (int b = r; b < nblk; b += kParts) {
+        float p = 0.f;
+#pragma unroll
+        for (int s = 0; s < kSB; s++)
+          p = __fmaf_rn(x[(size_t)(b * kSB + s) * kMlpIn + i], O.d[0][(size_t)(b * kSB + s) * kH + j], p);
+        acc += p;
+      }
+    } else if ((e -= kMlpIn * kH) < 3 * kH) {
+      const int l = e / kH, j = e % kH;
+      par = L.b[l] + j;
+      for (int b = r; b < nblk; b += kParts) {
+        float p = 0.f;
+#pragma unroll
+        for (int s = 0; s < kSB; s++) p += O.d[l][(size_t)(b * kSB + s) * kH + j];
+        acc += p;
+      }
+    } else if ((e -= 3 * kH) < kH) {
+      par = L.w[3] + e;
+      for (int b = r; b < nblk; b += kParts) {
+        float p = 0.f;
+#pragma unroll
+        for (int s = 0; s < kSB; s++) p = __fmaf_rn(O.a[2][(size_t)(b * kSB + s) * kH + e], O.d4[b * kSB + s], p);
+        acc += p;
+      }
+    } else {
+      par = L.b[3];
+      for (int b = r; b < nblk; b += kParts) {
+        float p = 0.f;
+#pragma unroll
+        for (int s = 0; s < kSB; s++) p += O.d4[b * kSB + s];
+        acc += p;
+      }
+    }
+  }
+  red[r][lane] = acc;
+  __syncthreads();
+  if (r == 0 && par >= 0) {
+    float gi = 0.f;
+#pragma unroll
+    for (int q = 0; q < kParts; q++) gi += red[q][lane];
+    grad[par] = gi;
+    if (update) adam_update(L, par, gi, P, WT, m, v, lr, bc1, bc2);
+  }
+  // the loss: the eights' losses in order
+  if (tile == 2 * kTilesPerLayer && r == 1 && lane == 0) {
     float e = 0.f;
+#pragma unroll 8
     for (int b = 0; b < nblk; b++) e += part_loss[b];
     *loss = e;
   }
-  const int stride = part_stride(L.total);
-  float gi = 0.f;
-  if (p < L.total) {
-#pragma unroll 4
-    for (int b = ty; b < nblk; b += 8) gi += part[(size_t)b * stride + p];
-  }
-  red[ty][tx] = gi;
-  __syncthreads();
-  if (ty != 0 || p >= L.total) return;
-  gi = 0.f;
-#pragma unroll
-  for (int r = 0; r < 8; r++) gi += red[r][tx];
-  grad[p] = gi;
-  if (update) adam_update(L, p, gi, P, WT, m, v, lr, bc1, bc2);
 }
 
 __global__ void __launch_bounds__(256) k_mlp_adam(MlpLayout L, const float* __restrict__ grad, float* P, float* WT,
@@ -346,8 +529,8 @@ cudaError_t configure()
   MLP_TRY(cudaGetDevice(&dev));
   if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
   if (done[dev]) return cudaSuccess;
-  MLP_TRY(cudaFuncSetAttribute(k_mlp_block, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes));
-  MLP_TRY(cudaFuncSetAttribute(k_mlp_forward, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes));
+  MLP_TRY(cudaFuncSetAttribute(k_mlp_pass, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPassSmem));
+  MLP_TRY(cudaFuncSetAttribute(k_mlp_forward, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kForwardSmem));
   done[dev] = true;
   return cudaSuccess;
 }
@@ -441,13 +624,21 @@ cudaError_t Mlp::reserve(int n)
   for (float** p : {&x_, &y_, &part_, &part_loss_})
     if (*p) { cudaFree(*p); *p = nullptr; }
   cap_ = 0;
-  const size_t c = (size_t)n, nblk = (c + kSB - 1) / kSB;
-  MLP_TRY(cudaMalloc(&x_, sizeof(float) * c * kMlpIn));
-  MLP_TRY(cudaMalloc(&y_, sizeof(float) * c));
-  MLP_TRY(cudaMalloc(&part_, sizeof(float) * nblk * part_stride(L.total)));
+  const size_t nblk = ((size_t)n + kSB - 1) / kSB, rows = nblk * kSB;
+  MLP_TRY(cudaMalloc(&x_, sizeof(float) * rows * kMlpIn));
+  MLP_TRY(cudaMalloc(&y_, sizeof(float) * rows));
+  MLP_TRY(cudaMalloc(&part_, sizeof(float) * rows * (6 * kH + 1)));
   MLP_TRY(cudaMalloc(&part_loss_, sizeof(float) * nblk));
   cap_ = n;
   return cudaSuccess;
+}
+
+// The features' rows past the last sample (the weight gradients read whole eights).
+cudaError_t Mlp::zero_tail(int n, cudaStream_t s)
+{
+  const size_t rows = ((size_t)n + kSB - 1) / kSB * kSB;
+  if (rows == (size_t)n) return cudaSuccess;
+  return cudaMemsetAsync(x_ + (size_t)n * kMlpIn, 0, sizeof(float) * (rows - n) * kMlpIn, s);
 }
 
 cudaError_t Mlp::set_data(const float* host_x, const float* host_y, int n, cudaStream_t s)
@@ -456,6 +647,7 @@ cudaError_t Mlp::set_data(const float* host_x, const float* host_y, int n, cudaS
   MLP_TRY(reserve(n));
   MLP_TRY(cudaMemcpyAsync(x_, host_x, sizeof(float) * n * kMlpIn, cudaMemcpyHostToDevice, s));
   MLP_TRY(cudaMemcpyAsync(y_, host_y, sizeof(float) * n, cudaMemcpyHostToDevice, s));
+  MLP_TRY(zero_tail(n, s));
   n_ = n;
   return cudaStreamSynchronize(s);
 }
@@ -466,6 +658,7 @@ cudaError_t Mlp::set_data_device(const float* dev_x, const float* dev_y, int n, 
   MLP_TRY(reserve(n));
   MLP_TRY(cudaMemcpyAsync(x_, dev_x, sizeof(float) * n * kMlpIn, cudaMemcpyDeviceToDevice, s));
   MLP_TRY(cudaMemcpyAsync(y_, dev_y, sizeof(float) * n, cudaMemcpyDeviceToDevice, s));
+  MLP_TRY(zero_tail(n, s));
   n_ = n;
   return cudaSuccess;
 }
@@ -475,8 +668,12 @@ cudaError_t Mlp::step(float lr, bool update, cudaStream_t s)
   const int n = n_;
   if (n <= 0 || !params_) return cudaErrorInvalidValue;
   const int nblk = (n + kSB - 1) / kSB;
+  const size_t rows = (size_t)nblk * kSB;
+  PassOut O;
+  for (int l = 0; l < 3; l++) { O.a[l] = part_ + l * rows * kH; O.d[l] = part_ + (3 + l) * rows * kH; }
+  O.d4 = part_ + 6 * rows * kH;
   MLP_TRY(configure());
-  k_mlp_block<<<nblk, kThreads, kSmemBytes, s>>>(L, params_, wt_, x_, y_, n, part_, part_loss_);
+  k_mlp_pass<<<nblk, kH, kPassSmem, s>>>(L, params_, wt_, x_, y_, n, O, part_loss_);
   MLP_TRY(cudaGetLastError());
   float bc1 = 1.f, bc2 = 1.f;
   if (update) {
@@ -484,8 +681,9 @@ cudaError_t Mlp::step(float lr, bool update, cudaStream_t s)
     bc1 = 1.f - std::pow(0.9f, (float)t);
     bc2 = 1.f - std::pow(0.999f, (float)t);
   }
-  k_mlp_reduce<<<(L.total + 31) / 32, 256, 0, s>>>(L, part_, part_loss_, nblk, grads_, loss_, update ? 1 : 0,
-                                                      params_, wt_, m_, v_, lr, bc1, bc2);
+  const int grid = 2 * kTilesPerLayer + (kSmall + kSmallPer - 1) / kSmallPer;
+  k_mlp_update<<<grid, 32 * kParts, 0, s>>>(L, x_, O, part_loss_, nblk, grads_, loss_, update ? 1 : 0, params_, wt_,
+                                            m_, v_, lr, bc1, bc2);
   MLP_TRY(cudaGetLastError());
   if (update) steps_done_++;
   return cudaSuccess;
@@ -550,7 +748,11 @@ cudaError_t Mlp::predict_device(const float* dev_x, int n, float* dev_out, cudaS
 {
   if (!params_ || n <= 0) return cudaErrorInvalidValue;
   MLP_TRY(configure());
-  k_mlp_forward<<<(n + kSB - 1) / kSB, kThreads, kSmemBytes, s>>>(L, params_, dev_x, n, dev_out);
+  int dev = 0, sms = 0;
+  MLP_TRY(cudaGetDevice(&dev));
+  MLP_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  const int tiles = (n + kFB - 1) / kFB;
+  k_mlp_forward<<<tiles < sms ? tiles : sms, 256, kForwardSmem, s>>>(L, params_, dev_x, n, dev_out);
   return cudaGetLastError();
 }
 

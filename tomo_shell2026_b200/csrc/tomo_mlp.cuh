@@ -1,10 +1,10 @@
 // Surrogate network of the learned-proposal orientation search: an FP32 MLP
 // [sin yaw, cos yaw, sin pitch, cos pitch] -> 128 -> 128 -> 128 -> Vss with
 // tanh hidden units and a linear output, trained full-batch with Adam by the
-// hand-written kernels of tomo_mlp.cu: one fused kernel per block of 16
-// samples runs the forward pass, the loss and the whole backward pass out of
-// shared memory and writes that block's gradient; a second kernel sums the
-// blocks' gradients in a fixed order (deterministic) and applies Adam.
+// hand-written kernels of tomo_mlp.cu: one fused kernel per eight samples runs
+// the forward pass, the loss and the backward pass to the layers' inputs out of
+// shared memory; a second kernel forms the weight gradients in a fixed order
+// (deterministic) and applies Adam.
 // Nothing here is a dense contraction large enough for tensor cores: one
 // training step on 936 samples is ~60 MFLOP.
 #pragma once
@@ -59,13 +59,14 @@ class Mlp {
 
  private:
   cudaError_t reserve(int n);
+  cudaError_t zero_tail(int n, cudaStream_t s);
   cudaError_t step(float lr, bool update, cudaStream_t s);
   void free_all();
 
   float *params_ = nullptr, *wt_ = nullptr;   // parameters, and each weight matrix transposed ([out][in])
   float *grads_ = nullptr, *m_ = nullptr, *v_ = nullptr;
   float *x_ = nullptr, *y_ = nullptr, *loss_ = nullptr;
-  float *part_ = nullptr, *part_loss_ = nullptr;   // per-block gradients [blocks][total], losses [blocks]
+  float *part_ = nullptr, *part_loss_ = nullptr;   // a pass's activations and gradients before them, losses per eight
   int cap_ = 0, n_ = 0, steps_done_ = 0;
   cudaGraphExec_t fit_exec_ = nullptr;     // the last captured fit and what it was captured for
   int fit_n_ = 0, fit_steps_ = 0, fit_start_ = -1;
