@@ -39,7 +39,10 @@ cudaError_t launch_bin_count(const EngineParams& p, cudaStream_t main, LaunchLog
 cudaError_t launch_after_count(const EngineParams& p, cudaStream_t main, size_t strip_smem, LaunchLog* L);
 cudaError_t launch_fill(const EngineParams& p, cudaStream_t s, LaunchLog* L);
 cudaError_t launch_strip_bed(const EngineParams& p, cudaStream_t main, size_t strip_smem, LaunchLog* L);
-cudaError_t launch_dump_scan(const int* cols8, int GG, int* off, int* totals, cudaStream_t s);
+int export_blocks(int G);
+cudaError_t launch_export_count(const EngineParams& p, uint8_t* bedpx, int* blocks, int* head, cudaStream_t s);
+cudaError_t launch_export_write(const EngineParams& p, const uint8_t* bedpx, const int* blocks, const int* head,
+                                short* pix, int4* sums, cudaStream_t s);
 cudaError_t launch_zero_ids(int* out, const int* ids, int n, cudaStream_t s);
 cudaError_t launch_read_probe(const void* buf, long long bytes, int reps, int blocks, cudaStream_t s);
 cudaError_t launch_gather_outputs(const long long* vo, const long long* vss, const long long* vtc, const long long* ent,
@@ -47,8 +50,6 @@ cudaError_t launch_gather_outputs(const long long* vo, const long long* vss, con
                                   const int* nbed, const int* flags, const int* ids, int n, long long* stage,
                                   cudaStream_t s);
 cudaError_t launch_scatter_rot(float* rot, const float* compact, const int* ids, int n, cudaStream_t s);
-cudaError_t launch_dump_gather(const int* cols8, const unsigned* keys64, const short* types64, int GG, const int* off,
-                               int* cols9, unsigned* keys, short* types, cudaStream_t s);
 
 namespace {
 
@@ -245,9 +246,10 @@ struct Workspace {
   DevBuf<int> dump_cols;
   DevBuf<unsigned> dump_keys;
   DevBuf<short> dump_types;
-  DevBuf<int> dump_off, dump_tot, dump_ccols;
-  DevBuf<unsigned> dump_ckeys;
-  DevBuf<short> dump_ctypes;
+  DevBuf<uint8_t> exp_bed;   // pixel export: bed pixels, block counts, totals, pixels, column sums
+  DevBuf<int> exp_blocks, exp_head;
+  DevBuf<short> exp_pix;
+  DevBuf<int4> exp_sums;
   LaunchLog log;
 
   int init()
@@ -273,7 +275,7 @@ struct Workspace {
     for (auto& q : prep) q.release();
     for (auto& s : set) { s.acc.release(); s.flags.release(); s.foldcnt.release(); s.foldp.release(); s.foldtc.release(); s.foldx.release(); s.foldxn.release(); s.foldmeta.release(); }
     dump_cols.release(); dump_keys.release(); dump_types.release();
-    dump_off.release(); dump_tot.release(); dump_ccols.release(); dump_ckeys.release(); dump_ctypes.release();
+    exp_bed.release(); exp_blocks.release(); exp_head.release(); exp_pix.release(); exp_sums.release();
     log.destroy();
     if (main) { cudaStreamDestroy(main); main = nullptr; }
     if (side) { cudaStreamDestroy(side); side = nullptr; }
@@ -306,11 +308,6 @@ struct Engine {
   DevBuf<int>& dump_cols;
   DevBuf<unsigned>& dump_keys;
   DevBuf<short>& dump_types;
-  DevBuf<int>& dump_off;
-  DevBuf<int>& dump_tot;
-  DevBuf<int>& dump_ccols;
-  DevBuf<unsigned>& dump_ckeys;
-  DevBuf<short>& dump_ctypes;
   LaunchLog& log;
 
   explicit Engine(Workspace& w, bool owns = false)
@@ -318,8 +315,7 @@ struct Engine {
         smem_optin(w.smem_optin), xf(w.prep[0].xf), minkey(w.prep[0].minkey), trange(w.prep[0].trange),
         bin_off(w.prep[0].bin_off), bin_cur(w.prep[0].bin_cur), bins(w.prep[0].bins), bbox(w.prep[0].bbox),
         bedf(w.prep[0].bedf), set(w.set), dump_cols(w.dump_cols),
-        dump_keys(w.dump_keys), dump_types(w.dump_types), dump_off(w.dump_off), dump_tot(w.dump_tot),
-        dump_ccols(w.dump_ccols), dump_ckeys(w.dump_ckeys), dump_ctypes(w.dump_ctypes), log(w.log)
+        dump_keys(w.dump_keys), dump_types(w.dump_types), log(w.log)
   {
   }
   Engine(const Engine&) = delete;
@@ -970,9 +966,11 @@ struct Engine {
   // One orientation with the dense per-column dump enabled (parity tests).
   int dump(int id, int c, int* cols8, unsigned* keys64, short* types64)
   {
-    const int fl = dump_device(id, c);
-    if (fl < 0) return fl;
+    EngineParams p;
+    TOMO_TRY(dump_device(id, c, true, &p));
+    int fl = 0;
     const size_t GG = (size_t)G * G;
+    TOMO_CUDA(cudaMemcpyAsync(&fl, o_flags.ptr + id, sizeof(int), cudaMemcpyDeviceToHost, main));
     if (cols8) TOMO_CUDA(cudaMemcpyAsync(cols8, dump_cols.ptr, sizeof(int) * GG * 8, cudaMemcpyDeviceToHost, main));
     if (keys64) TOMO_CUDA(cudaMemcpyAsync(keys64, dump_keys.ptr, sizeof(unsigned) * GG * 64, cudaMemcpyDeviceToHost, main));
     if (types64) TOMO_CUDA(cudaMemcpyAsync(types64, dump_types.ptr, sizeof(short) * GG * 64, cudaMemcpyDeviceToHost, main));
@@ -980,40 +978,10 @@ struct Engine {
     return fl;
   }
 
-  // The same dump compacted on the device to the occupied columns:
-  // cols9[n_occ][9] = slot id + the 8 dump fields, keys/types = each occupied
-  // column's kept keys and types, concatenated in slot order.
-  int dump_compact(int id, int c, std::vector<int>& cols9, std::vector<unsigned>& keys, std::vector<short>& types)
-  {
-    const int fl = dump_device(id, c);
-    if (fl < 0) return fl;
-    const int GG = G * G;
-    TOMO_CUDA(dump_off.reserve((size_t)GG * 2));
-    TOMO_CUDA(dump_tot.reserve(2));
-    TOMO_CUDA(launch_dump_scan(dump_cols.ptr, GG, dump_off.ptr, dump_tot.ptr, main));
-    int tot[2] = {0, 0};
-    TOMO_CUDA(cudaMemcpyAsync(tot, dump_tot.ptr, sizeof(tot), cudaMemcpyDeviceToHost, main));
-    TOMO_CUDA(cudaStreamSynchronize(main));
-    TOMO_CUDA(dump_ccols.reserve((size_t)tot[0] * 9));
-    TOMO_CUDA(dump_ckeys.reserve((size_t)tot[1]));
-    TOMO_CUDA(dump_ctypes.reserve((size_t)tot[1]));
-    TOMO_CUDA(launch_dump_gather(dump_cols.ptr, dump_keys.ptr, dump_types.ptr, GG, dump_off.ptr, dump_ccols.ptr,
-                                 dump_ckeys.ptr, dump_ctypes.ptr, main));
-    cols9.resize((size_t)tot[0] * 9);
-    keys.resize((size_t)tot[1]);
-    types.resize((size_t)tot[1]);
-    if (tot[0]) TOMO_CUDA(cudaMemcpyAsync(cols9.data(), dump_ccols.ptr, sizeof(int) * cols9.size(), cudaMemcpyDeviceToHost, main));
-    if (tot[1]) {
-      TOMO_CUDA(cudaMemcpyAsync(keys.data(), dump_ckeys.ptr, sizeof(unsigned) * keys.size(), cudaMemcpyDeviceToHost, main));
-      TOMO_CUDA(cudaMemcpyAsync(types.data(), dump_ctypes.ptr, sizeof(short) * types.size(), cudaMemcpyDeviceToHost, main));
-    }
-    TOMO_CUDA(cudaStreamSynchronize(main));
-    return fl;
-  }
-
-  // Runs one orientation in strip configuration c with the dense dump on;
-  // returns its status flags.
-  int dump_device(int id, int c)
+  // Runs one orientation in strip configuration c with the dense dump on (the
+  // keys and types past each column's count are zero with `clean`, else
+  // whatever was there); *out: the launch's parameters.
+  int dump_device(int id, int c, bool clean, EngineParams* out)
   {
     if (id < 0 || id >= nYPR) return set_error(TOMO_ERR_ARG, "orientation index out of range");
     if (P.n_tri == 0) return set_error(TOMO_ERR_ARG, "empty mesh");
@@ -1026,8 +994,10 @@ struct Engine {
     const size_t GG = (size_t)G * G;
     TOMO_CUDA(dump_cols.reserve(GG * 8)); TOMO_CUDA(dump_keys.reserve(GG * 64)); TOMO_CUDA(dump_types.reserve(GG * 64));
     TOMO_CUDA(cudaMemsetAsync(dump_cols.ptr, 0, sizeof(int) * GG * 8, main));
-    TOMO_CUDA(cudaMemsetAsync(dump_keys.ptr, 0, sizeof(unsigned) * GG * 64, main));
-    TOMO_CUDA(cudaMemsetAsync(dump_types.ptr, 0, sizeof(short) * GG * 64, main));
+    if (clean) {
+      TOMO_CUDA(cudaMemsetAsync(dump_keys.ptr, 0, sizeof(unsigned) * GG * 64, main));
+      TOMO_CUDA(cudaMemsetAsync(dump_types.ptr, 0, sizeof(short) * GG * 64, main));
+    }
     TOMO_CUDA(cudaMemsetAsync(o_nbed.ptr + id, 0, sizeof(int), main));
     EngineParams p = base_params(mode);
     p.dump_slot = 0; p.dump_cols = dump_cols.ptr; p.dump_keys = dump_keys.ptr; p.dump_types = dump_types.ptr;
@@ -1047,10 +1017,8 @@ struct Engine {
       TOMO_CUDA(launch_after_count(p, main, smem, &log));
     }
     TOMO_CUDA(launch_fold(p, main, &log));
-    int fl = 0;
-    TOMO_CUDA(cudaMemcpyAsync(&fl, o_flags.ptr + id, sizeof(int), cudaMemcpyDeviceToHost, main));
-    TOMO_CUDA(cudaStreamSynchronize(main));
-    return fl;
+    *out = p;
+    return 0;
   }
 
   // Autotuner: times the device sweep of an evenly strided sample of up to
@@ -1178,7 +1146,7 @@ std::vector<float> g_Mss, g_Mo, g_Vtc;
 std::vector<long long> g_Vo64, g_Vss64, g_Vtc64;
 float g_volmass[22] = {0};
 float g_mat4x4[16] = {0};
-std::vector<short> g_pix[11];
+short* g_pix[11] = {nullptr};   // into g_export
 int g_npix[11] = {0};
 
 Engine& engine()
@@ -1212,142 +1180,71 @@ void host_mat4x4(const Engine& E, const float* vtx, int nV, int id, float* m16)
   m16[7] = -dy + R[3] * m + R[4] * n + R[5] * o;
   m16[11] = -dz + R[6] * m + R[7] * n + R[8] * o;
 }
-// Final slot rows of one orientation rebuilt on the host from its column
-// dump: kept pixels in column order with their paired types, the floor
-// sentinels (STomoSh_INT3.cpp:790-810) and the bed pixels (GenerateBed,
-// :1375-1443) -- the reference's slot buffer after thread_func.  From them:
-// the render pixels of slotsToPxls (:1103-1135) and GetSSPixels
-// (:1257-1318, brief branch) and the vm_info of Calculate (:1211-1255).
-struct SlotRow { short type, z, nz; };
+// Library-owned pinned host memory of the exported pixels and column sums: it
+// grows to the largest export and is given back by OnDestroy.
+struct PinnedBuf {
+  unsigned char* ptr = nullptr;
+  size_t n = 0;
+  cudaError_t reserve(size_t bytes)
+  {
+    if (bytes <= n && ptr) return cudaSuccess;
+    release();
+    const size_t want = std::max<size_t>(bytes + bytes / 4, size_t(1) << 20);
+    const cudaError_t e = cudaHostAlloc((void**)&ptr, want, cudaHostAllocDefault);
+    if (e == cudaSuccess) n = want; else ptr = nullptr;
+    return e;
+  }
+  void release() { if (ptr) cudaFreeHost(ptr); ptr = nullptr; n = 0; }
+};
+PinnedBuf g_export;
 
-bool host_bed_candidate(const Engine& E, const std::vector<uint8_t>& bf, int X, int Y)
-{
-  const int G = E.G, r = (int)E.P.bed_outer;
-  const int xa = std::max(X - r, 0), xb = std::min(X + r, G), ya = std::max(Y - r, 0), yb = std::min(Y + r, G);
-  const int qid = X * G + Y;
-  float md = 1e5f;
-  for (int sx = xa; sx < xb; sx++)
-    for (int sy = ya; sy < yb; sy++) {
-      const int sid = sx * G + sy;
-      const uint8_t f = bf[sid];
-      if (!(f & kBfTouch)) continue;
-      if ((f & kBfSelfR) && sid < qid) continue;
-      const float dx = (float)X - (float)sx, dy = (float)Y - (float)sy;
-      const float dist = sqrtf(dx * dx + dy * dy);
-      md = (md < dist) ? md : dist;
-    }
-  if (md > E.P.bed_outer) return false;
-  if (E.P.bed_type == kBedBrim || E.P.bed_type == kBedRaft) return true;
-  if (E.P.bed_type == kBedSkirt && md > E.P.bed_inner) return true;
-  return false;
-}
-
-int export_best(Engine& E, int id, std::vector<short>* pix, int* npix, float* vm)
+// The render pixels of orientation `id` (pix[k], npix[k]: pointers into the
+// export buffer) and the vm_info folds of Calculate, from the device's export
+// kernels.  The float folds run here, over the occupied slots in order.
+int export_best(Engine& E, int id, short** pix, int* npix, float* vm)
 {
   const int G = E.G;
   const size_t GG = (size_t)G * G;
-  std::vector<int> cols;
-  std::vector<unsigned> keys;
-  std::vector<short> types;
-  int fl = -1;
+  const int nblk = export_blocks(G);
+  Workspace& W = E.W;
+  TOMO_CUDA(W.exp_bed.reserve(GG));
+  TOMO_CUDA(W.exp_blocks.reserve((size_t)nblk * 12));
+  TOMO_CUDA(W.exp_head.reserve(13));
+  int head[13] = {0};
+  EngineParams p;
   for (int c : {0, 4, 1, 3}) {
-    fl = E.dump_compact(id, c, cols, keys, types);
-    if (fl < 0) return fl;
-    if (!(fl & (kFlagRedo | kFlagSafeOverflow))) break;
+    TOMO_TRY(E.dump_device(id, c, false, &p));
+    TOMO_CUDA(launch_export_count(p, W.exp_bed.ptr, W.exp_blocks.ptr, W.exp_head.ptr, E.main));
+    TOMO_CUDA(cudaMemcpyAsync(head, W.exp_head.ptr, sizeof(head), cudaMemcpyDeviceToHost, E.main));
+    TOMO_CUDA(cudaStreamSynchronize(E.main));
+    if (!(head[12] & (kFlagRedo | kFlagSafeOverflow))) break;
   }
-  if (fl & (kFlagRedo | kFlagSafeOverflow | kFlagGrid))
+  if (head[12] & (kFlagRedo | kFlagSafeOverflow | kFlagGrid))
     return set_error(TOMO_ERR_CAPACITY, "best orientation could not be exported");
-  // occupied columns in slot order: rows[rbeg[j] .. rbeg[j+1]) plus an
-  // optional bed row (bed_row[j]); bed-only columns listed separately
-  const int nocc = (int)(cols.size() / 9);
-  std::vector<SlotRow> rows;
-  rows.reserve(keys.size() + 2 * (size_t)nocc);
-  std::vector<int> rbeg((size_t)nocc + 1, 0);
-  std::vector<int> colidx(GG, -1);
-  std::vector<uint8_t> bed_row((size_t)nocc, 0);
-  std::vector<uint8_t> bf(GG, (uint8_t)(kBfPoss | kBfLand));
-  int minX = G, minY = G, maxX = -1, maxY = -1;
-  size_t k0 = 0;
-  for (int j = 0; j < nocc; j++) {
-    const int* c = &cols[(size_t)j * 9];
-    const int sl = c[0], nd = c[1], nfin = c[2];
-    const int x = sl / G, y = sl % G;
-    minX = std::min(minX, x); maxX = std::max(maxX, x); minY = std::min(minY, y); maxY = std::max(maxY, y);
-    rbeg[j] = (int)rows.size();
-    const int n = std::min(nd, 64);
-    for (int i = 0; i < n; i++) {
-      const unsigned k = keys[k0 + i];
-      rows.push_back({nd > 1 ? types[k0 + i] : (short)0, (short)((int)(k >> 16) - 32768), (short)((int)(k & 0xFFFFu) - 32768)});
-    }
-    k0 += (size_t)n;
-    const int extra = nfin - nd;
-    if (extra == 2) { rows.push_back({(short)kSSA, 0, 0}); rows.push_back({(short)kNVA, 0, 0}); }
-    else if (extra == 1) rows.push_back({(short)c[7], 0, 0});
-    bf[sl] = (uint8_t)c[8];
-    colidx[sl] = j;
+  size_t total = 0;
+  for (int k = 0; k < 11; k++) total += (size_t)head[k];
+  const size_t nocc = (size_t)head[11];
+  const size_t sums_at = (total * 12 + 15) / 16 * 16;
+  TOMO_CUDA(W.exp_pix.reserve(std::max<size_t>(total, 1) * 6));
+  TOMO_CUDA(W.exp_sums.reserve(std::max<size_t>(nocc, 1)));
+  TOMO_CUDA(g_export.reserve(sums_at + nocc * sizeof(int4)));
+  TOMO_CUDA(launch_export_write(p, W.exp_bed.ptr, W.exp_blocks.ptr, W.exp_head.ptr, W.exp_pix.ptr, W.exp_sums.ptr, E.main));
+  if (total) TOMO_CUDA(cudaMemcpyAsync(g_export.ptr, W.exp_pix.ptr, total * 12, cudaMemcpyDeviceToHost, E.main));
+  if (nocc)
+    TOMO_CUDA(cudaMemcpyAsync(g_export.ptr + sums_at, W.exp_sums.ptr, nocc * sizeof(int4), cudaMemcpyDeviceToHost, E.main));
+  TOMO_CUDA(cudaStreamSynchronize(E.main));
+  short* at = (short*)g_export.ptr;
+  for (int k = 0; k < 11; k++) {
+    pix[k] = head[k] ? at : nullptr;
+    npix[k] = head[k];
+    at += (size_t)head[k] * 6;
   }
-  rbeg[nocc] = (int)rows.size();
-  // bed pixels, in the reference's scan order
-  std::vector<int> bed_only;
-  if (E.P.bed_type != kBedNone && maxX >= 0 && (int)E.P.bed_outer > 0) {
-    const int m = (int)E.P.bed_outer + 1;
-    const int bx0 = std::max(minX - m, 0), bx1 = std::min(maxX + m + 1, G);
-    const int by0 = std::max(minY - m, 0), by1 = std::min(maxY + m + 1, G);
-    for (int X = bx0; X < bx1; X++)
-      for (int Y = by0; Y < by1; Y++) {
-        const size_t sl = (size_t)X * G + Y;
-        const uint8_t f = bf[sl];
-        if (!((f & kBfPoss) && (f & kBfLand)) || !host_bed_candidate(E, bf, X, Y)) continue;
-        const int j = colidx[sl];
-        if (j < 0) { bed_only.push_back((int)sl); continue; }
-        bool merged = false;
-        for (int r = rbeg[j]; r < rbeg[j + 1]; r++)
-          if (rows[r].z == 1 && rows[r].nz == 0) { rows[r].type |= (short)kBed; merged = true; break; }
-        if (!merged) bed_row[j] = 1;
-      }
-  }
-  // render pixels per type (slotsToPxls), the support pixels (GetSSPixels)
-  // and the float folds of Calculate, over the final slots in ascending order
-  for (int k = 0; k < 11; k++) pix[k].clear();
-  float va = 0.f, vb = 0.f, vnv = 0.f, vtc = 0.f, vbed = 0.f;
-  const SlotRow bed_px = {(short)kBed, 1, 0};
-  auto column = [&](int sl, const SlotRow* r, int n, bool extra_bed) {
-    const short x = (short)(sl / G), y = (short)(sl % G);
-    int sa = 0, sb = 0, snvb = 0, snva = 0, stc = 0, sbed = 0;
-    int ss0 = -1, ss1 = -1;
-    for (int i = 0; i < n + (extra_bed ? 1 : 0); i++) {
-      const SlotRow& q = i < n ? r[i] : bed_px;
-      for (int k = 0; k < 11; k++)
-        if (k != 4 && (q.type & (1 << k))) {
-          const short px[6] = {x, y, q.z, 0, 0, q.nz};
-          pix[k].insert(pix[k].end(), px, px + 6);
-        }
-      if (q.type & kSSB) ss0 = q.z;
-      if (q.type & kSSA) ss1 = q.z;
-      if (ss0 > -1 && ss1 > -1) {
-        for (int zz = ss0; zz >= ss1; zz--) {
-          const short px[6] = {x, y, (short)zz, 0, 0, 0};
-          pix[4].insert(pix[4].end(), px, px + 6);
-        }
-        ss0 = ss1 = -1;
-      }
-      if (q.type & kAl) sa += q.z;
-      if (q.type & kBe) sb += q.z;
-      if (q.type & kNVB) snvb += q.z;
-      if (q.type & kNVA) snva += q.z;
-      if (q.type & kTC) stc += q.z;
-      if (q.type & kBed) sbed += q.z;
-    }
-    va += (float)sa; vb += (float)sb; vnv += (float)(snvb - snva); vtc += (float)stc;
-    vbed += (float)sbed * E.P.bed_thickness;
-  };
-  size_t b = 0;
-  for (int j = 0; j <= nocc; j++) {
-    const int sl = j < nocc ? cols[(size_t)j * 9] : INT_MAX;
-    while (b < bed_only.size() && bed_only[b] < sl) { column(bed_only[b], nullptr, 0, true); b++; }
-    if (j < nocc) column(sl, rows.data() + rbeg[j], rbeg[j + 1] - rbeg[j], bed_row[j] != 0);
-  }
-  for (int k = 0; k < 11; k++) npix[k] = (int)(pix[k].size() / 6);
+  float va = 0.f, vb = 0.f, vnv = 0.f, vtc = 0.f;
+  const int4* q = (const int4*)(g_export.ptr + sums_at);
+  for (size_t j = 0; j < nocc; j++) { va += (float)q[j].x; vb += (float)q[j].y; vnv += (float)q[j].z; vtc += (float)q[j].w; }
+  // each bed slot adds its one bed pixel at z = 1, every other occupied slot nothing
+  float vbed = nocc ? 0.f + (float)0 * E.P.bed_thickness : 0.f;
+  for (int j = 0; j < head[5]; j++) vbed += (float)1 * E.P.bed_thickness;
   vm[0] = va; vm[1] = vb; vm[2] = vtc; vm[3] = vnv; vm[11] = vbed;
   return 0;
 }
@@ -1384,7 +1281,7 @@ int TomoSh_CUDA(float* f32info, int* i32info, float* YPR, int* tri, float* vtx, 
   g_Vo64 = E.vo64; g_Vss64 = E.vss64; g_Vtc64 = E.vtc64;
   const int opt = first_optimal(n, g_Mss.data());
   std::memset(g_volmass, 0, sizeof(g_volmass));
-  for (int k = 0; k < 11; k++) { g_pix[k].clear(); g_npix[k] = 0; }
+  for (int k = 0; k < 11; k++) { g_pix[k] = nullptr; g_npix[k] = 0; }
   if (n > 0) {
     if (E.P.n_tri > 0 && E.export_pixels) {
       rc = export_best(E, opt, g_pix, g_npix, g_volmass);
@@ -1415,8 +1312,7 @@ float* getMat4x4(void) { return g_mat4x4; }
 int getnData2i(short type) { return (type >= 0 && type < 11) ? g_npix[type] : 0; }
 short* getpData2i(short type)
 {
-  if (type < 0 || type >= 11 || g_pix[type].empty()) return nullptr;
-  return g_pix[type].data();
+  return (type >= 0 && type < 11) ? g_pix[type] : nullptr;
 }
 const long long* getVo64(void) { return g_Vo64.empty() ? nullptr : g_Vo64.data(); }
 const long long* getVss64(void) { return g_Vss64.empty() ? nullptr : g_Vss64.data(); }
@@ -1427,7 +1323,8 @@ void OnDestroy(void)
   std::lock_guard<std::mutex> lock(g_mutex);
   g_Mss.clear(); g_Mo.clear(); g_Vtc.clear(); g_Vo64.clear(); g_Vss64.clear(); g_Vtc64.clear();
   g_Mss.shrink_to_fit(); g_Mo.shrink_to_fit(); g_Vtc.shrink_to_fit();
-  for (auto& v : g_pix) { v.clear(); v.shrink_to_fit(); }
+  for (short*& q : g_pix) q = nullptr;
+  g_export.release();
   std::memset(g_npix, 0, sizeof(g_npix));
   if (g_engine) {
     Workspace* w = &g_engine->W;
@@ -2281,7 +2178,7 @@ int tomoBatchExport(int mesh)
   g_Vo64 = E.vo64; g_Vss64 = E.vss64; g_Vtc64 = E.vtc64;
   const int opt = first_optimal(n, g_Mss.data());
   std::memset(g_volmass, 0, sizeof(g_volmass));
-  for (int k = 0; k < 11; k++) { g_pix[k].clear(); g_npix[k] = 0; }
+  for (int k = 0; k < 11; k++) { g_pix[k] = nullptr; g_npix[k] = 0; }
   if (n > 0) {
     if (E.P.n_tri > 0) {
       const int rc = export_best(E, opt, g_pix, g_npix, g_volmass);

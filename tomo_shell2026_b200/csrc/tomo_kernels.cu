@@ -2288,63 +2288,172 @@ __global__ void __launch_bounds__(128) k_fold(EngineParams p)
   }
 }
 
-// ---------------------------------------------------------------- dump compaction
-// The dense per-column dump ([G*G][8] fields, [G*G][64] keys and types) is
-// mostly empty; these two kernels compact it to the occupied columns before
-// it crosses PCIe.  off[2*sl] / off[2*sl+1] = exclusive offsets of column
-// sl among the occupied columns / the kept keys; totals = both counts.
+// ---------------------------------------------------------------- pixel export
+// The render pixels of one orientation from its column dump: every slot's final
+// rows -- kept pixels in column order with their paired types, the floor
+// sentinels (STomoSh_INT3.cpp:790-810) and the bed pixel (GenerateBed,
+// :1375-1443) -- as the reference's slot buffer holds them after thread_func,
+// listed per type in slot order (slotsToPxls, :1103-1135), with one pixel per
+// voxel of explicit support (GetSSPixels, :1257-1318, brief branch), and each
+// occupied slot's sums for the float folds of Calculate (:1211-1255).
+//
+// One thread per slot: a counting pass, a scan of the blocks' counts (channels:
+// the 11 pixel types and the occupied slots) and a writing pass.  A one-CTA scan
+// of the dump and a host loop over its rows took 188 + 360 us on a 5k-triangle
+// part and 18.6 ms on the 87k shell (1.9 M pixels); the three kernels take 15 us
+// and 80 us.
+constexpr int kExportThreads = 256;
+constexpr int kChannels = 12;
 
-__global__ void __launch_bounds__(1024) k_dump_scan(const int* cols8, int GG, int* off, int* totals)
+// f(type, z, nz) for every final row of a slot.
+template <typename F>
+__device__ __forceinline__ void slot_rows(const EngineParams& p, int sl, bool bed, F f)
 {
-  __shared__ long long wt[32];
-  const int per = (GG + blockDim.x - 1) / blockDim.x;
-  const int b = threadIdx.x * per;
-  auto item = [&](int sl) -> long long {
-    const int nd = cols8[(size_t)sl * 8];
-    return nd > 0 ? (1ll << 32) + (nd < 64 ? nd : 64) : 0ll;
-  };
-  long long local = 0;
-  for (int i = 0; i < per; i++) if (b + i < GG) local += item(b + i);
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  long long x = local;
-  for (int d = 1; d < 32; d <<= 1) { const long long y = __shfl_up_sync(0xFFFFFFFFu, x, d); if (lane >= d) x += y; }
-  if (lane == 31) wt[wid] = x;
-  __syncthreads();
-  if (wid == 0) {
-    long long t = wt[lane];
-    for (int d = 1; d < 32; d <<= 1) { const long long y = __shfl_up_sync(0xFFFFFFFFu, t, d); if (lane >= d) t += y; }
-    wt[lane] = t;
+  const int* c = p.dump_cols + (size_t)sl * 8;
+  const int nd = c[0], n = min(nd, 64);
+  bool merged = !bed;   // the bed pixel goes into the first pixel equal to it, else behind the column
+  for (int i = 0; i < n; i++) {
+    const unsigned key = p.dump_keys[(size_t)sl * 64 + i];
+    int t = nd > 1 ? p.dump_types[(size_t)sl * 64 + i] : 0;
+    const int z = key_z(key), nz = key_nz(key);
+    if (!merged && z == 1 && nz == 0) { t |= kBed; merged = true; }
+    f(t, z, nz);
   }
-  __syncthreads();
-  long long run = ((wid > 0) ? wt[wid - 1] : 0ll) + x - local;
-  for (int i = 0; i < per; i++) {
-    const int sl = b + i;
-    if (sl >= GG) break;
-    off[2 * sl] = (int)(run >> 32);
-    off[2 * sl + 1] = (int)(run & 0xFFFFFFFFll);
-    run += item(sl);
+  if (nd > 0) {
+    const int extra = c[1] - nd;
+    if (extra == 2) { f((int)kSSA, 0, 0); f((int)kNVA, 0, 0); }
+    else if (extra == 1) f(c[6], 0, 0);
   }
-  if (threadIdx.x == 0) {
-    totals[0] = (int)(wt[31] >> 32);
-    totals[1] = (int)(wt[31] & 0xFFFFFFFFll);
-  }
+  if (!merged) f((int)kBed, 1, 0);
 }
 
-__global__ void __launch_bounds__(256) k_dump_gather(const int* cols8, const unsigned* keys64, const short* types64,
-                                                     int GG, const int* off, int* cols9, unsigned* keys, short* types)
+// Rows of a slot counted per channel.
+__device__ __forceinline__ void count_slot(const EngineParams& p, int sl, bool bed, int* cnt)
 {
-  for (int sl = blockIdx.x * blockDim.x + threadIdx.x; sl < GG; sl += gridDim.x * blockDim.x) {
-    const int nd = cols8[(size_t)sl * 8];
-    if (nd <= 0) continue;
-    const int c = off[2 * sl], k = off[2 * sl + 1];
-    cols9[(size_t)c * 9] = sl;
-    for (int f = 0; f < 8; f++) cols9[(size_t)c * 9 + 1 + f] = cols8[(size_t)sl * 8 + f];
-    const int n = nd < 64 ? nd : 64;
-    for (int i = 0; i < n; i++) {
-      keys[(size_t)k + i] = keys64[(size_t)sl * 64 + i];
-      types[(size_t)k + i] = types64[(size_t)sl * 64 + i];
+  int ss0 = -1, ss1 = -1;
+  slot_rows(p, sl, bed, [&](int t, int z, int) {
+#pragma unroll
+    for (int k = 0; k < 11; k++)
+      if (k != 4) cnt[k] += (t >> k) & 1;
+    if (t & kSSB) ss0 = z;
+    if (t & kSSA) ss1 = z;
+    if (ss0 > -1 && ss1 > -1) {
+      cnt[4] += max(ss0 - ss1 + 1, 0);
+      ss0 = ss1 = -1;
     }
+  });
+  cnt[11] = p.dump_cols[(size_t)sl * 8] > 0;
+}
+
+__global__ void __launch_bounds__(kExportThreads) k_export_count(EngineParams p, uint8_t* bedpx, int* blocks)
+{
+  __shared__ int tot[kChannels];
+  const int sl = blockIdx.x * kExportThreads + threadIdx.x;
+  if (threadIdx.x < kChannels) tot[threadIdx.x] = 0;
+  __syncthreads();
+  int cnt[kChannels];
+#pragma unroll
+  for (int k = 0; k < kChannels; k++) cnt[k] = 0;
+  if (sl < p.G * p.G) {
+    bool bed = false;
+    if (p.bed_type != kBedNone && p.bed_r > 0 && p.bbox[2] >= 0) {
+      const int m = (int)p.bed_outer + 1, X = sl / p.G, Y = sl % p.G;
+      const uint8_t f = p.bedf[sl];
+      bed = X >= p.bbox[0] - m && X <= p.bbox[2] + m && Y >= p.bbox[1] - m && Y <= p.bbox[3] + m && (f & kBfPoss) &&
+            (f & kBfLand) && bed_candidate(p, p.bedf, X, Y);
+    }
+    bedpx[sl] = bed;
+    count_slot(p, sl, bed, cnt);
   }
+#pragma unroll
+  for (int k = 0; k < kChannels; k++) {
+    const int v = __reduce_add_sync(0xFFFFFFFFu, cnt[k]);
+    if ((threadIdx.x & 31) == 0 && v) atomicAdd(&tot[k], v);
+  }
+  __syncthreads();
+  if (threadIdx.x < kChannels) blocks[(size_t)threadIdx.x * gridDim.x + blockIdx.x] = tot[threadIdx.x];
+}
+
+// Exclusive scan of the blocks' counts, one warp per channel, in place; the
+// totals, then the flags of the orientation, go to `head`.
+__global__ void __launch_bounds__(32 * kChannels) k_export_scan(int* blocks, int nblk, const int* flags, int* head)
+{
+  const int k = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  int* row = blocks + (size_t)k * nblk;
+  int run = 0;
+  for (int b0 = 0; b0 < nblk; b0 += 32) {
+    const int v = b0 + lane < nblk ? row[b0 + lane] : 0;
+    int x = v;
+    for (int d = 1; d < 32; d <<= 1) {
+      const int y = __shfl_up_sync(0xFFFFFFFFu, x, d);
+      if (lane >= d) x += y;
+    }
+    if (b0 + lane < nblk) row[b0 + lane] = run + x - v;
+    run += __shfl_sync(0xFFFFFFFFu, x, 31);
+  }
+  if (lane == 0) head[k] = run;
+  if (threadIdx.x == 0) head[kChannels] = *flags;
+}
+
+// pix: the types' pixels one type after another (x, y, z, 0, 0, nz); sums: per
+// occupied slot its sums of up faces, down faces, implicit support (below minus
+// above) and cavity pixels.
+__global__ void __launch_bounds__(kExportThreads) k_export_write(EngineParams p, const uint8_t* bedpx, const int* blocks,
+                                                                 const int* head, short* pix, int4* sums)
+{
+  __shared__ int wtot[kChannels][kExportThreads / 32];
+  const int sl = blockIdx.x * kExportThreads + threadIdx.x;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const bool in = sl < p.G * p.G;
+  int cnt[kChannels], at[kChannels];
+#pragma unroll
+  for (int k = 0; k < kChannels; k++) cnt[k] = 0;
+  const bool bed = in && bedpx[sl];
+  if (in) count_slot(p, sl, bed, cnt);
+#pragma unroll
+  for (int k = 0; k < kChannels; k++) {
+    int x = cnt[k];
+    for (int d = 1; d < 32; d <<= 1) {
+      const int y = __shfl_up_sync(0xFFFFFFFFu, x, d);
+      if (lane >= d) x += y;
+    }
+    if (lane == 31) wtot[k][wid] = x;
+    at[k] = x - cnt[k];
+  }
+  __syncthreads();
+  if (!in) return;
+  int base = 0;
+#pragma unroll
+  for (int k = 0; k < kChannels; k++) {
+    for (int w = 0; w < wid; w++) at[k] += wtot[k][w];
+    at[k] += blocks[(size_t)k * gridDim.x + blockIdx.x];
+    if (k < 11) { at[k] += base; base += head[k]; }
+  }
+  const unsigned xy = (unsigned)(sl / p.G) | (unsigned)(sl % p.G) << 16;
+  unsigned* const out = (unsigned*)pix;   // 12 bytes a pixel
+  auto put = [&](int e, int z, int nz) {
+    unsigned* d = out + (size_t)e * 3;
+    d[0] = xy; d[1] = (unsigned)z & 0xFFFFu; d[2] = (unsigned)nz << 16;
+  };
+  int ss0 = -1, ss1 = -1;
+  int4 sum = make_int4(0, 0, 0, 0);
+  slot_rows(p, sl, bed, [&](int t, int z, int nz) {
+#pragma unroll
+    for (int k = 0; k < 11; k++)
+      if (k != 4 && ((t >> k) & 1)) put(at[k]++, z, nz);
+    if (t & kSSB) ss0 = z;
+    if (t & kSSA) ss1 = z;
+    if (ss0 > -1 && ss1 > -1) {
+      for (int zz = ss0; zz >= ss1; zz--) put(at[4]++, zz, 0);
+      ss0 = ss1 = -1;
+    }
+    if (t & kAl) sum.x += z;
+    if (t & kBe) sum.y += z;
+    if (t & kNVB) sum.z += z;
+    if (t & kNVA) sum.z -= z;
+    if (t & kTC) sum.w += z;
+  });
+  if (cnt[11]) sums[at[11]] = sum;
 }
 
 }  // namespace tomo
@@ -2507,17 +2616,21 @@ cudaError_t launch_batch(const EngineParams& p, cudaStream_t main, size_t strip_
   return e != cudaSuccess ? e : launch_after_count(p, main, strip_smem, L);
 }
 
-cudaError_t launch_dump_scan(const int* cols8, int GG, int* off, int* totals, cudaStream_t s)
+int export_blocks(int G) { return (G * G + kExportThreads - 1) / kExportThreads; }
+
+// blocks: [12][export_blocks]; head: 12 totals and the flags.
+cudaError_t launch_export_count(const EngineParams& p, uint8_t* bedpx, int* blocks, int* head, cudaStream_t s)
 {
-  k_dump_scan<<<1, 1024, 0, s>>>(cols8, GG, off, totals);
+  const int n = export_blocks(p.G);
+  k_export_count<<<n, kExportThreads, 0, s>>>(p, bedpx, blocks);
+  k_export_scan<<<1, 32 * kChannels, 0, s>>>(blocks, n, p.flags, head);
   return cudaGetLastError();
 }
 
-cudaError_t launch_dump_gather(const int* cols8, const unsigned* keys64, const short* types64, int GG, const int* off,
-                               int* cols9, unsigned* keys, short* types, cudaStream_t s)
+cudaError_t launch_export_write(const EngineParams& p, const uint8_t* bedpx, const int* blocks, const int* head,
+                                short* pix, int4* sums, cudaStream_t s)
 {
-  const int blocks = (GG + 255) / 256 < 148 * 8 ? (GG + 255) / 256 : 148 * 8;
-  k_dump_gather<<<blocks > 0 ? blocks : 1, 256, 0, s>>>(cols8, keys64, types64, GG, off, cols9, keys, types);
+  k_export_write<<<export_blocks(p.G), kExportThreads, 0, s>>>(p, bedpx, blocks, head, pix, sums);
   return cudaGetLastError();
 }
 
