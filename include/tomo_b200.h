@@ -236,7 +236,7 @@ int tomoSurrogateSearch(const float* f32info, const int* i32info, const float* Y
  * host arrays of nYPR floats that receive what getMo/getMss/getVtc return
  * after TomoSh_CUDA, and the return value is optID (or a negative error).
  * The render pixels, vm_info and mat4x4 are not produced.
- *   - allocates nothing: device scratch is one file-scope 16 MiB __device__
+ *   - allocates nothing: device scratch is one file-scope 32 MiB __device__
  *     array per device, host staging is file-scope arrays; no cudaMalloc,
  *     cudaFree or allocating library routine is called;
  *   - limits: at most 16384 triangles and 16384 vertices, and a footprint
@@ -259,7 +259,7 @@ int tomoSurrogateSearch(const float* f32info, const int* i32info, const float* Y
  *     configurations as TomoSh_CUDA (large capacity, first-come priorities,
  *     safe mode); tomoGetStats out[9..11] counts them for the last call;
  *   - work is issued on `stream` (a cudaStream_t; null = the legacy default
- *     stream), orientations four at a time. */
+ *     stream), up to sixteen orientations at a time. */
 int tomoSweepStatic(const float* f32info, const int* i32info, const float* YPR, const int* tri, const float* vtx,
                     const float* vtx_nrm, float* Mo, float* Mss, float* Vtc, void* stream);
 

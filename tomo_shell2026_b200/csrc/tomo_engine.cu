@@ -1536,11 +1536,14 @@ int tomoFinish(float* Mo, float* Mss, float* Vtc)
 
 namespace tomo {
 
-constexpr size_t kStaticArenaBytes = size_t(16) << 20;  // 16 MiB of device scratch per device
-constexpr size_t kStaticListBytes = size_t(8) << 20;    // of which the strips' pixel lists
+constexpr size_t kStaticArenaBytes = size_t(32) << 20;  // 32 MiB of device scratch per device
+constexpr size_t kStaticListBytes = size_t(16) << 20;   // of which the strips' pixel lists
 constexpr int kStaticMaxTri = 16384;
 constexpr int kStaticMaxVtx = 16384;
-constexpr int kStaticBatch = 4;
+// Orientations per batch at most (fewer for the largest meshes).  A batch is a
+// chain of launches and one wait, so it costs the same for 4 orientations as for
+// 16: the 5k solid's 684 orientations took 17.6 ms four at a time.
+constexpr int kStaticBatch = 16;
 constexpr int kStaticGrid = 256;                        // the reference's slot grid
 constexpr int kStaticMaxDevices = 64;
 
@@ -1550,21 +1553,30 @@ namespace {
 
 constexpr size_t static_round(size_t b) { return (b + 255) & ~size_t(255); }
 
-// Bytes of the arena layout below for nV vertices and nT triangles.
-constexpr size_t static_bytes(size_t nV, size_t nT)
+// Bytes of the arena layout below for nV vertices, nT triangles and batches of
+// B orientations.  The triangle bins serve the re-runs of single orientations
+// only; safe mode may use more of them than a batch slot's worth.
+constexpr size_t static_bytes(size_t nV, size_t nT, size_t B)
 {
-  const size_t B = kStaticBatch, GG = (size_t)kStaticGrid * kStaticGrid, S = kStaticGrid;  // S bound: 1-column strips
+  const size_t GG = (size_t)kStaticGrid * kStaticGrid, S = kStaticGrid;  // S bound: 1-column strips
   return static_round(16 * nV) * 2 + static_round(16 * nT) + static_round(4 * 9 * B) + static_round(4 * B) +
-         static_round(16 * B * nV) + static_round(4 * 4 * B) + static_round(4 * B * nT) +
-         static_round(4 * B * (S + 1)) + static_round(4 * B * S) + static_round(4 * B * (4 * nT + 4096)) +
+         static_round(16 * B * nV) + static_round(4 * 4 * B) + static_round(4 * nT) +
+         static_round(4 * (S + 1)) + static_round(4 * S) + static_round(4 * 4 * (4 * nT + 4096)) +
          static_round(4 * B * S) + static_round(kStaticListBytes) +
          static_round(4 * 4 * B) + static_round(B * GG) + static_round(8 * B * kAccLanes) + static_round(4 * B) +
          static_round(4 * B * S) + static_round(4 * B * GG) + static_round(2 * B * GG) + static_round(sizeof(FoldEscape) * kFoldEscapes) +
-         static_round(4) + static_round(4 * B * S * 8) +
-         5 * static_round(8 * B) + 3 * static_round(4 * B) + 2 * static_round(4 * B);
+         static_round(4) + static_round(4 * B * S * 8) + 5 * static_round(8 * B) + static_round(5 * 4 * B);
 }
-static_assert(static_bytes(kStaticMaxVtx, kStaticMaxTri) <= kStaticArenaBytes,
+static_assert(static_bytes(kStaticMaxVtx, kStaticMaxTri, 8) <= kStaticArenaBytes,
               "the static scratch must hold the largest accepted mesh");
+
+// Orientations per batch for a mesh.
+int static_batch(int nV, int nT)
+{
+  int B = kStaticBatch;
+  while (B > 1 && static_bytes((size_t)nV, (size_t)nT, (size_t)B) > kStaticArenaBytes) B--;
+  return B;
+}
 
 struct StaticLayout {
   float4 *vpos, *vnrm, *xf;
@@ -1579,14 +1591,14 @@ struct StaticLayout {
   short* foldtc;
   FoldEscape* foldx;
   int* foldxn;
-  float *o_vof, *o_vssf, *o_vtcf;
+  float *o_vof, *o_vssf, *o_vtcf;   // with o_nbed and o_flags: five arrays of B words side by side
   long long bins_total;   // entries of the bins region
 };
 
 // Same order and sizes as static_bytes().
-StaticLayout static_layout(unsigned char* base, int nV, int nT)
+StaticLayout static_layout(unsigned char* base, int nV, int nT, int nB)
 {
-  const size_t B = kStaticBatch, GG = (size_t)kStaticGrid * kStaticGrid, S = kStaticGrid;
+  const size_t B = nB, GG = (size_t)kStaticGrid * kStaticGrid, S = kStaticGrid;
   size_t off = 0;
   auto take = [&](size_t bytes) { unsigned char* q = base + off; off += static_round(bytes); return (void*)q; };
   StaticLayout L;
@@ -1597,10 +1609,10 @@ StaticLayout static_layout(unsigned char* base, int nV, int nT)
   L.ori = (int*)take(4 * B);
   L.xf = (float4*)take(16 * B * nV);
   L.minkey = (unsigned*)take(4 * 4 * B);
-  L.trange = (unsigned*)take(4 * B * nT);
-  L.bin_off = (int*)take(4 * B * (S + 1));
-  L.bin_cur = (int*)take(4 * B * S);
-  L.bins_total = (long long)B * (4 * (long long)nT + 4096);
+  L.trange = (unsigned*)take(4 * (size_t)nT);
+  L.bin_off = (int*)take(4 * (S + 1));
+  L.bin_cur = (int*)take(4 * S);
+  L.bins_total = 4 * (4 * (long long)nT + 4096);
   L.bins = (int*)take(4 * (size_t)L.bins_total);
   L.ent_cnt = (int*)take(4 * B * S);
   L.ents = (uint2*)take(kStaticListBytes);
@@ -1616,8 +1628,9 @@ StaticLayout static_layout(unsigned char* base, int nV, int nT)
   L.foldmeta = (int*)take(4 * B * S * 8);
   L.o_vo = (long long*)take(8 * B); L.o_vss = (long long*)take(8 * B); L.o_vtc = (long long*)take(8 * B);
   L.o_ent = (long long*)take(8 * B); L.o_col = (long long*)take(8 * B);
-  L.o_vof = (float*)take(4 * B); L.o_vssf = (float*)take(4 * B); L.o_vtcf = (float*)take(4 * B);
-  L.o_nbed = (int*)take(4 * B); L.o_flags = (int*)take(4 * B);
+  L.o_flags = (int*)take(5 * 4 * B);
+  L.o_nbed = L.o_flags + B;
+  L.o_vof = (float*)(L.o_nbed + B); L.o_vssf = L.o_vof + B; L.o_vtcf = L.o_vssf + B;
   return L;
 }
 
@@ -1625,12 +1638,11 @@ StaticLayout static_layout(unsigned char* base, int nV, int nT)
 float4 g_static_hpos[kStaticMaxVtx], g_static_hnrm[kStaticMaxVtx];
 int4 g_static_htri[kStaticMaxTri];
 float g_static_hrot[kStaticBatch * 9];
-int g_static_hori[kStaticBatch] = {0, 1, 2, 3};
-int g_static_hflags[kStaticBatch], g_static_hnbed[kStaticBatch];
-float g_static_hvof[kStaticBatch], g_static_hvssf[kStaticBatch], g_static_hvtcf[kStaticBatch];
+int g_static_hori[kStaticBatch] = {0, 1, 2, 3, 4, 5, 6, 7, 8, 9, 10, 11, 12, 13, 14, 15};
+int g_static_hout[5 * kStaticBatch];   // flags, bed pixels, Vo, Vss, Vtc (float bits)
 float g_static_bedfold[kStaticGrid * kStaticGrid + 1];
 void* g_static_addr[kStaticMaxDevices];
-static_assert(kStaticBatch == 4, "g_static_hori lists the batch slots");
+static_assert(kStaticBatch == 16, "g_static_hori lists the batch slots");
 
 // Device address of g_static_arena on the current device, looked up once per
 // device (with that device current).
@@ -1781,7 +1793,8 @@ extern "C" int tomoSweepStatic(const float* f32info, const int* i32info, const f
   StreamDrain drain{st};   // declared after the lock: runs before it is released
   void* base = nullptr;
   TOMO_TRY(static_arena(&base));
-  const StaticLayout L = static_layout((unsigned char*)base, P.n_vtx, P.n_tri);
+  const int B = static_batch(P.n_vtx, P.n_tri);
+  const StaticLayout L = static_layout((unsigned char*)base, P.n_vtx, P.n_tri, B);
   int dev = 0, optin = 0;
   TOMO_CUDA(cudaGetDevice(&dev));
   TOMO_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
@@ -1801,8 +1814,8 @@ extern "C" int tomoSweepStatic(const float* f32info, const int* i32info, const f
   TOMO_CUDA(cudaMemcpyAsync(L.ori, g_static_hori, sizeof(g_static_hori), cudaMemcpyHostToDevice, st));
 
   const int normal_cap = 4 * P.n_tri + 4096;
-  for (int first = 0; first < P.n_ypr; first += kStaticBatch) {
-    const int nb = std::min(kStaticBatch, P.n_ypr - first);
+  for (int first = 0; first < P.n_ypr; first += B) {
+    const int nb = std::min(B, P.n_ypr - first);
     for (int o = 0; o < nb; o++)
       rotation(YPR[(first + o) * 3 + 0], YPR[(first + o) * 3 + 1], YPR[(first + o) * 3 + 2], &g_static_hrot[o * 9]);
     TOMO_CUDA(cudaMemcpyAsync(L.rot, g_static_hrot, sizeof(float) * 9 * nb, cudaMemcpyHostToDevice, st));
@@ -1814,11 +1827,13 @@ extern "C" int tomoSweepStatic(const float* f32info, const int* i32info, const f
     static_bind(p, L, nb, 0, normal_cap);
     TOMO_CUDA(launch_batch(p, st, X.cfg[0].smem, nullptr));
     TOMO_CUDA(launch_fold(p, st, nullptr));
-    TOMO_CUDA(cudaMemcpyAsync(g_static_hflags, L.o_flags, sizeof(int) * nb, cudaMemcpyDeviceToHost, st));
+    TOMO_CUDA(cudaMemcpyAsync(g_static_hout, L.o_flags, sizeof(int) * 5 * B, cudaMemcpyDeviceToHost, st));
     TOMO_CUDA(cudaStreamSynchronize(st));
+    bool rerun = false;
     // the re-run ladder of Engine::resolve_ids, per flagged slot
     for (int o = 0; o < nb; o++) {
-      int fl = g_static_hflags[o];
+      int fl = g_static_hout[o];
+      rerun = rerun || (fl & kFlagRedo);
       if (fl & kFlagGrid) return set_error(TOMO_ERR_CAPACITY, "slot index outside the grid");
       bool safe = (fl & (kFlagStray | kFlagBinCap)) != 0;
       if (!safe && (fl & kFlagOverflow)) {
@@ -1849,15 +1864,16 @@ extern "C" int tomoSweepStatic(const float* f32info, const int* i32info, const f
       if (fl & kFlagFoldRange)
         return set_error(TOMO_ERR_CAPACITY, "column values past 16 bits overflowed the fold escape table");
     }
-    TOMO_CUDA(cudaMemcpyAsync(g_static_hvof, L.o_vof, sizeof(float) * nb, cudaMemcpyDeviceToHost, st));
-    TOMO_CUDA(cudaMemcpyAsync(g_static_hvssf, L.o_vssf, sizeof(float) * nb, cudaMemcpyDeviceToHost, st));
-    TOMO_CUDA(cudaMemcpyAsync(g_static_hvtcf, L.o_vtcf, sizeof(float) * nb, cudaMemcpyDeviceToHost, st));
-    TOMO_CUDA(cudaMemcpyAsync(g_static_hnbed, L.o_nbed, sizeof(int) * nb, cudaMemcpyDeviceToHost, st));
-    TOMO_CUDA(cudaStreamSynchronize(st));
+    if (rerun) {
+      TOMO_CUDA(cudaMemcpyAsync(g_static_hout, L.o_flags, sizeof(int) * 5 * B, cudaMemcpyDeviceToHost, st));
+      TOMO_CUDA(cudaStreamSynchronize(st));
+    }
+    const int* nbed = g_static_hout + B;
+    const float *vof = (const float*)(nbed + B), *vssf = vof + B, *vtcf = vssf + B;
     for (int o = 0; o < nb; o++) {
-      if (g_static_hnbed[o] < 0 || g_static_hnbed[o] > kStaticGrid * kStaticGrid)
+      if (nbed[o] < 0 || nbed[o] > kStaticGrid * kStaticGrid)
         return set_error(TOMO_ERR_CAPACITY, "bed pixel count outside the slot grid");
-      finish(first + o, g_static_hvof[o], g_static_hvssf[o], g_static_hvtcf[o], g_static_hnbed[o]);
+      finish(first + o, vof[o], vssf[o], vtcf[o], nbed[o]);
     }
   }
   return first_optimal(P.n_ypr, Mss);
