@@ -508,9 +508,11 @@ __global__ void __launch_bounds__(256) k_bin_fill(EngineParams p)
 // may pass the exact test (tomo_span.cuh); the set bits go to the warp's
 // queue, and 32 at a time every lane runs the reference's barycentric test on
 // one of them, so that the divisions, the double-precision u and the append
-// run on full warps.  A triangle whose box holds more than kLaneCells cells
-// per lane is finished by the whole warp, 32 cells at a time, so that a few
-// large triangles among small ones do not hold up a warp.  The warps of a
+// run on full warps.  When at most kFewLanes lanes are left with cells, one of
+// them with more than kManyCells, their triangles are finished by the whole
+// warp, 32 cells at a time, so that a few large triangles among small ones do
+// not hold up a warp (a fixed share of 8 cells per lane sent half the triangles
+// of a uniform 2,000-triangle mesh that way: 943 us per 256 orientations).  The warps of a
 // block share nothing: no barrier.  Accepted pixels collect in the warp's stash
 // and are appended in full rounds of 32, and consecutive blocks belong to
 // different orientations: with appends straight from the exact test and whole
@@ -532,7 +534,7 @@ __global__ void __launch_bounds__(256) k_bin_fill(EngineParams p)
 constexpr int kRastWarps = 4;
 constexpr int kRastGroups = 4;  // groups of triangles a warp takes in turn
 constexpr int kRastMix = 16;   // orientations whose blocks run side by side
-constexpr int kLaneCells = 8;
+constexpr int kFewLanes = 4, kManyCells = 6;
 constexpr int kStash = 128;
 
 struct RastWarp {
@@ -669,6 +671,7 @@ __global__ void __launch_bounds__(32 * kRastWarps, 7) k_raster(EngineParams p)
     float fbx = 0.f, fby = 0.f, fbz = 0.f, n0 = 0.f;   // centroid fallback (STomoSh_INT3.cpp:1190-1206)
     unsigned hits = 0u;                   // lanes whose triangle has an accepted pixel (warp-uniform)
     unsigned big = 0u;                    // triangles left to the whole warp
+    int from = 0;                         // their first cell left
     int tt = t, c = sub, step = L;        // cells c, c + step, ... of triangle tt
     for (bool first = true;; first = false) {
       int ncx = 0, ncell = 0;
@@ -710,16 +713,20 @@ __global__ void __launch_bounds__(32 * kRastWarps, 7) k_raster(EngineParams p)
           }
         }
       }
-      int lim = ncell;
-      if (first) {
-        big = __ballot_sync(full, ncell > kLaneCells * L && sub == 0);
-        lim = min(ncell, kLaneCells * L);
-      }
       float rc;
       asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(rc) : "f"((float)max(ncx, 1)));
-      while (__any_sync(full, c < lim)) {
+      for (int turn = 0;; turn++) {
+        const unsigned todo = __ballot_sync(full, c < ncell);
+        if (!todo) break;
+        // few lanes still at work, one of them for long: their triangles, cell by
+        // cell from here on, to the whole warp
+        if (first && __popc(todo) <= kFewLanes && __reduce_max_sync(full, (ncell - c) >> lsh) > kManyCells) {
+          big = __ballot_sync(full, sub == 0 && turn * L < ncell);
+          from = turn * L;
+          break;
+        }
         unsigned m = 0u;
-        if (c < lim) {
+        if (c < ncell) {
           // c / ncx: at most 1,024 with ncx <= 512, so the float quotient of c + 1/2 truncates exactly
           const int cj = __float2int_rz(((float)c + 0.5f) * rc), ci = c - cj * ncx;
           m = mask_cell(T, ci, cj);
@@ -779,7 +786,7 @@ __global__ void __launch_bounds__(32 * kRastWarps, 7) k_raster(EngineParams p)
       own = __ffs(big) - 1;
       big &= big - 1;
       tt = __shfl_sync(full, t, own);
-      c = kLaneCells * L + lane;
+      c = from + lane;
       step = 32;
       __syncwarp();
     }
@@ -2545,8 +2552,10 @@ static dim3 tri_grid(const EngineParams& p)
 }
 
 // Lanes per triangle in k_raster: one, unless that gives fewer warps than
-// kRastFill; then the lanes of a triangle share its cells.
-constexpr int kRastFill = 148 * 16;
+// kRastFill; then the lanes of a triangle share its cells (256 orientations of a
+// 320-triangle solid 330 pixels across: 1,112 us with a quarter of this, 943
+// with half, 732).
+constexpr int kRastFill = 148 * 64;
 
 int raster_lanes_log2(int nT, int Bo)
 {
@@ -2560,7 +2569,7 @@ int raster_lanes_log2(int nT, int Bo)
 static int raster_blocks(int ngroup, int Bo)
 {
   int per = kRastGroups;
-  while (per > 1 && (long long)Bo * (ngroup / per) < 4 * kRastFill) per--;
+  while (per > 1 && (long long)Bo * (ngroup / per) < kRastFill) per--;
   return std::min((ngroup + kRastWarps * per - 1) / (kRastWarps * per), 65535);
 }
 
