@@ -90,7 +90,7 @@ void tomoVolToMass(const float* f32info, const int* i32info, float* vm22);
 #define TOMO_OPT_STRIP_H 2      /* force strip height 1, 2, 4 or 8 (0 = automatic) */
 #define TOMO_OPT_FORCE_SAFE 3   /* 1 = evaluate every orientation in safe mode */
 #define TOMO_OPT_NORMAL_SMEM 4  /* shared-memory budget of a normal strip, in bytes: its pixel capacity is what is left beside four
-                                   bytes and a bit per slot and a 20 KB work area, at 6 bytes a pixel (0 = what five CTAs per SM hold) */
+                                   bytes and a bit per slot and a 20 KB work area, at 6 bytes a pixel (0 = what four CTAs per SM hold) */
 #define TOMO_OPT_EXPORT 5       /* 0 = skip the best orientation's pixel export (default 1) */
 #define TOMO_OPT_ADAPTIVE 6     /* 0 = keep the planned strip budget even when early batches overflow (default 1) */
 #define TOMO_OPT_PROPOSAL 7     /* tomoSurrogateSearch proposals: 0 = the trained network (default), 1 = bilinear

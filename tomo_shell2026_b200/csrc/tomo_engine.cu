@@ -398,7 +398,7 @@ struct Engine {
 
   // Strip configurations.
   //   0 normal     : H0-column strips whose columns k_columns resolves from
-  //                  k_raster's pixel lists, five CTAs per SM; H0 is the
+  //                  k_raster's pixel lists, four CTAs per SM; H0 is the
   //                  tallest strip with room for two pixels per slot;
   //   1 safe       : strips that rasterize their own triangles, whole-box
   //                  evaluation, priorities, all opt-in shared memory;
@@ -416,16 +416,15 @@ struct Engine {
     const size_t optin = smem_optin ? smem_optin : 232448;
     // the strip kernels also hold ~0.7 KB of static shared memory
     const size_t budget1 = std::min<size_t>(optin, 227 * 1024) - 2048;
-    const size_t five = strip_default_budget();
+    const size_t shared = strip_default_budget();
     // Pixels of an h-column normal strip.  By default what the shared memory of
-    // five CTAs per SM holds (82k solid, 256 orientations: 545 us at five, 592
-    // at four, 615 at six with 40 registers); a budget given by
+    // four CTAs per SM holds (k_columns needs its 64 registers); a budget given by
     // TOMO_OPT_NORMAL_SMEM (or a later one of adapt_after) buys 6 bytes per
     // pixel beside four bytes and a bit per slot and a 20 KB work area.
     auto pixels = [&](int h, size_t budget) -> int {
       const size_t HG = (size_t)h * G;
       const size_t fixed = budget ? 4 * HG + HG / 8 + 32 + std::max<size_t>(20816, 6 * HG + 2048) : strip_smem_bytes(0, h, G, 0);
-      const size_t all = budget ? std::min(optin - 2048, budget) : (five ? five : 45056), per = budget ? 6 : 4;
+      const size_t all = budget ? std::min(optin - 2048, budget) : (shared ? shared : 55296), per = budget ? 6 : 4;
       if (all < fixed + 32 * per) return 16;
       const size_t most = (budget1 - strip_smem_bytes(0, h, G, 0)) / 4 - 16;
       return (int)std::min<size_t>(std::min<size_t>((all - fixed) / per - 16, most), 32767);

@@ -1652,26 +1652,32 @@ __global__ void __launch_bounds__(256, 1) k_strip(EngineParams p)
 // The pixels are grouped by slot with a counting sort in shared memory (one
 // 16-bit counter per slot), so a column is a run of keys.  Columns of one or
 // two raw pixels (nine in ten on a solid) have a closed form and take a thread
-// each.  The rest are resolved by pixel: a warp takes as many whole columns as
-// fit its 32 lanes, every lane ranks its key within its column, and the pairing
-// follows from ballots (see pair_pixels).  A column of more than 32 raw pixels
-// takes a warp by itself, 32 sorted keys at a time.
+// each.  Longer ones are queued by length -- 3-4, 5-8, 9-16, 17-32 -- so that a
+// warp's 32 threads take 32 columns of like length, each sorted in place in
+// shared memory and paired by one walk over its sorted keys (see ColWalk).  A
+// column of more than 32 raw pixels takes a warp, 32 sorted keys at a time (see
+// pair_pixels).
 //
 // Bound by instruction issue and, on strips of a few hundred pixels, by the
-// latency between its barriers.  With linked lists per column, one thread per
-// column of up to 11 pixels and a serial pairing scan the stage took 1,060 us
-// per 256 orientations of the 82k solid at four CTAs per SM, now 545 at five
-// (592 at four); 5k solid 92 -> 53 us; the 87k thin shell's 2-degree sweep
-// (seven pixels to a column) 557 -> 219 ms.
+// latency between its barriers.  Per 256 orientations of the 82k solid: 1,060 us
+// with linked lists per column, a thread per column of up to 11 pixels and a
+// serial scan of longer ones; 545 with the counting sort and whole columns side
+// by side in a warp's lanes, ranked by shuffles and paired by ballots; 521 now.
+// The thin shell (seven pixels to a column) gains more: its 2-degree sweep took
+// 557, 220 and now 169 ms.  Sorting networks in registers for 4, 8 and 16 keys
+// were slower than the insertion sort (555 with the first two, 669 with all): the
+// unrolled walks do not fit the instruction cache.  Five CTAs per SM with 48
+// registers spill: 548.  Other class limits (8 / 16, 6 / 12 / 20, 5 / 9, 3 / 6 /
+// 12) are within 1 %.
 constexpr int kColThreads = 256;
-constexpr int kColBlocks = 5;    // CTAs per SM
+constexpr int kColBlocks = 4;    // CTAs per SM
 constexpr int kLongKeys = 128;   // raw pixels of a column that a warp sorts in its scratch
 
 // Shared-memory bytes of one k_columns CTA.
 __host__ __device__ inline size_t columns_smem(int HG, int C)
 {
   return round16(sizeof(short) * (size_t)(HG + 2)) + round16(sizeof(unsigned) * (size_t)C) +
-         2 * round16(sizeof(short) * (size_t)HG) + sizeof(unsigned) * kLongKeys * (kColThreads / 32);
+         3 * round16(sizeof(short) * (size_t)HG) + sizeof(unsigned) * kLongKeys * (kColThreads / 32);
 }
 
 // What earlier pixels of the same column leave behind for the next 32.
@@ -1725,10 +1731,63 @@ __device__ __forceinline__ PairOut pair_pixels(const EngineParams& p, unsigned k
   return r;
 }
 
+// The pairing of one column as a walk over its sorted keys (see pair_pixels).
+// Keys equal to the one before change nothing: an up face is kept only when
+// none is open, a down face only when one is.
+struct ColWalk {
+  int vo = 0, vss = 0, tc = 0, nd = 0;
+  int lastz = 0, lasttype = 0, has10 = 0;
+  unsigned prev = 0u;
+  bool open = false;            // the last pixel with a face was an up face
+  bool ex = false, im = false;  // the last kept down face casts explicit / implicit support
+  bool first = false;           // an up face was kept
+  bool down = false;            // the last kept face is a down face
+
+  __device__ __forceinline__ void step(const EngineParams& p, unsigned key, int i, bool last_px, int dump_slot)
+  {
+    const bool dup = i > 0 && key == prev;
+    prev = key;
+    nd += !dup;
+    const int z = key_z(key), nz = key_nz(key);
+    const bool up = nz >= 1, dn = nz <= -1;
+    const bool ka = up && !open, kb = dn && open;
+    open = up || (open && !dn);
+    const bool s = kb && nz <= p.nz_ex, n = kb && nz >= p.nz_im;
+    const bool sa = ka && ex, na = ka && im;
+    const bool t = !p.explicit_ss && ka && !first;
+    vo += ka ? z : (kb ? -z : 0);
+    if (p.explicit_ss) {
+      vss += s ? z : (sa ? -z : 0);
+    } else {
+      tc += t ? z : 0;
+      vss += (ka ? (t ? 0 : -z) + (na ? z : 0) : 0) + ((kb && !n) ? z : 0);
+    }
+    ex = kb ? s : ex;
+    im = kb ? n : im;
+    first = first || ka;
+    down = kb || (down && !ka);
+    if (last_px && !dup) {
+      lastz = z;
+      lasttype = (ka ? kAl : 0) | (kb ? kBe : 0) | (s ? kSSB : 0) | (sa ? kSSA : 0) | (n ? kNVB : 0) | (na ? kNVA : 0) |
+                 (t ? kTC : 0);
+      has10 |= z == 1 && nz == 0;
+      if (dump_slot >= 0) dump_key(p, dump_slot, nd - 1, key, lasttype);
+    }
+  }
+  // a single distinct pixel is not paired
+  __device__ __forceinline__ void result(ColOut& c) const
+  {
+    const bool pair = nd > 1;
+    c.vo = pair ? max(vo, 0) : 0; c.vss = pair ? vss : 0; c.tc = pair ? tc : 0;
+    c.ndist = nd;
+    c.lastz = lastz; c.lasttype = pair ? lasttype : 0; c.has10 = has10;
+  }
+};
+
 __global__ void __launch_bounds__(kColThreads, kColBlocks) k_columns(EngineParams p)
 {
   extern __shared__ __align__(16) unsigned char smem[];
-  __shared__ int nlong, nbig, sflag, wtot[32];
+  __shared__ int nq[4], sflag, wtot[32];   // queue lengths
   __shared__ long long red[kColThreads / 32][6];
   const unsigned full = 0xFFFFFFFFu;
   const int s = blockIdx.x, o = blockIdx.y;
@@ -1749,14 +1808,18 @@ __global__ void __launch_bounds__(kColThreads, kColBlocks) k_columns(EngineParam
   unsigned* const off2 = (unsigned*)q; q += round16(sizeof(short) * (size_t)(HG + 2));   // two 16-bit slot counters a word
   unsigned* const keys = (unsigned*)q; q += round16(sizeof(unsigned) * (size_t)C);
   unsigned short* const olist = (unsigned short*)q; q += round16(sizeof(short) * (size_t)HG);   // occupied slots in order
-  unsigned short* const longq = (unsigned short*)q; q += round16(sizeof(short) * (size_t)HG);   // columns of 3..32 pixels from the front, longer from the back
+  // queues of longer columns, two growing towards each other in each array:
+  // 3-4 and 5-8 raw pixels, 9-16 and more
+  unsigned short* const queue = (unsigned short*)q; q += round16(sizeof(short) * (size_t)HG);
+  unsigned short* const queue2 = (unsigned short*)q; q += round16(sizeof(short) * (size_t)HG);
   unsigned* const scr = (unsigned*)q + wid * kLongKeys;
   const unsigned short* const ends = (const unsigned short*)off2;
 
   // ---- group the pixels by slot
   const int nw = (HG + 1) >> 1;
   for (int i = tid; i < nw; i += kColThreads) off2[i] = 0u;
-  if (tid == 0) { nlong = 0; nbig = 0; sflag = 0; }
+  if (tid < 4) nq[tid] = 0;
+  if (tid == 0) sflag = 0;
   const uint2* const ents = p.ents + ((size_t)o * p.S + s) * C;
   constexpr int kHold = 8;               // pixels a thread keeps between the two passes
   uint2 held[kHold];
@@ -1813,8 +1876,8 @@ __global__ void __launch_bounds__(kColThreads, kColBlocks) k_columns(EngineParam
   short* const ftc = p.foldtc ? p.foldtc + (size_t)o * p.G * p.G + (size_t)xs0 * p.G : nullptr;
   // the fold record, sums and bed flags of column l (occupied slot ls)
   auto store = [&](int l, int ls, const ColOut& c) {
-    const int lim = p.fold_lim;
-    if (max(max((unsigned)(c.vo + lim), (unsigned)(c.vss + lim)), (unsigned)(c.tc + lim)) <= 2u * (unsigned)lim) {
+    const int avss = abs(c.vss), atc = abs(c.tc);
+    if (max(max(c.vo, avss), atc) <= p.fold_lim) {   // vo >= 0
       fv[l] = __byte_perm(c.vo, c.vss, 0x5410);
       if (ftc) ftc[l] = (short)c.tc;   // tc is zero with explicit support
     } else {
@@ -1825,7 +1888,7 @@ __global__ void __launch_bounds__(kColThreads, kColBlocks) k_columns(EngineParam
       else atomicOr(&p.flags[o], kFlagFoldRange);
     }
     a_vo += c.vo; a_vss += c.vss; a_tc += c.tc;
-    a_avss += abs(c.vss); a_atc += abs(c.tc);
+    a_avss += avss; a_atc += atc;
     a_ent += c.ndist;
     if (last_px) {
       const int gx = xs0 + ls / p.G, gy = ls % p.G;
@@ -1846,150 +1909,8 @@ __global__ void __launch_bounds__(kColThreads, kColBlocks) k_columns(EngineParam
     if (im && c.nfin < kSlotCap) { c.nfin++; c.lastz = 0; c.lasttype = kNVA; }
   };
 
-  // ---- columns of one or two raw pixels, one per thread
-  for (int l0 = wid * 32; l0 < nocc; l0 += kColThreads) {
-    const int l = l0 + lane;
-    int cnt = 0;
-    if (l < nocc) {
-      const int ls = olist[l];
-      const int end = ends[ls], beg = ls ? ends[ls - 1] : 0;
-      cnt = end - beg;
-      if (cnt <= 2) {
-        const unsigned k0 = keys[beg], k1 = keys[end - 1];
-        const unsigned hi = max(k0, k1), lo = min(k0, k1);
-        const int z0 = key_z(hi), n0 = key_nz(hi), z1 = key_z(lo), n1 = key_nz(lo);
-        ColOut c;
-        c.vo = c.vss = c.tc = 0;
-        c.ndist = 1;
-        bool s1 = false, m1 = false;
-        if (hi != lo) {                  // a single distinct pixel is not paired
-          c.ndist = 2;
-          const bool up0 = n0 >= 1, up1 = !up0 && n1 >= 1, dn1 = up0 && n1 <= -1;
-          s1 = dn1 && n1 <= p.nz_ex; m1 = dn1 && n1 >= p.nz_im;
-          const int al = up0 ? z0 : (up1 ? z1 : 0), be = dn1 ? z1 : 0;
-          c.vo = max(al - be, 0);
-          if (p.explicit_ss) c.vss = s1 ? z1 : 0;
-          else { c.tc = al; c.vss = m1 ? 0 : be; }
-          if (last_px) {
-            const int tc = p.explicit_ss ? 0 : kTC;
-            const int t0 = up0 ? kAl | tc : 0, t1 = up1 ? kAl | tc : (dn1 ? kBe | (s1 ? kSSB : 0) | (m1 ? kNVB : 0) : 0);
-            c.lastz = z1; c.lasttype = t1;
-            c.has10 = (z0 == 1 && n0 == 0) || (z1 == 1 && n1 == 0);
-            if (dump) { dump_key(p, xs0 * p.G + ls, 0, hi, t0); dump_key(p, xs0 * p.G + ls, 1, lo, t1); }
-          }
-        } else if (last_px) {
-          c.lastz = z0; c.lasttype = 0;
-          c.has10 = z0 == 1 && n0 == 0;
-          if (dump) dump_key(p, xs0 * p.G + ls, 0, hi, 0);
-        }
-        if (last_px) finish(c, s1, m1);
-        store(l, ls, c);
-      }
-    }
-    const unsigned some = __ballot_sync(full, cnt > 2 && cnt <= 32);
-    if (some) {
-      int at = 0;
-      if (lane == 0) at = atomicAdd(&nlong, __popc(some));
-      at = __shfl_sync(full, at, 0);
-      if (cnt > 2 && cnt <= 32) longq[at + __popc(some & ((1u << lane) - 1u))] = (unsigned short)l;
-    }
-    if (cnt > 32) longq[HG - 1 - atomicAdd(&nbig, 1)] = (unsigned short)l;
-  }
-  __syncthreads();
-
-  // ---- columns of 3 to 32 raw pixels: whole columns side by side in a warp's lanes
-  {
-    const int share = (nlong + kColThreads / 32 - 1) / (kColThreads / 32);
-    const int q1 = min((wid + 1) * share, nlong);
-    const PairCarry none = {false, false, false, false};
-    for (int q0 = wid * share; q0 < q1; q0 += 32) {
-      // lane i: the i-th column of this batch
-      int l = 0, ls = 0, beg = 0, cnt = 0;
-      if (q0 + lane < q1) {
-        l = longq[q0 + lane];
-        ls = olist[l];
-        beg = ls ? ends[ls - 1] : 0;
-        cnt = ends[ls] - beg;
-      }
-      int cum = cnt;
-      for (int d = 1; d < 32; d <<= 1) {
-        const int y = __shfl_up_sync(full, cum, d);
-        if (lane >= d) cum += y;
-      }
-      const int all = __shfl_sync(full, cum, 31);
-      int base = 0;                      // pixels already resolved
-      while (base < all) {
-        const bool in = cnt > 0 && cum - cnt >= base && cum - base <= 32;
-        const unsigned heads = __reduce_or_sync(full, in ? 1u << (cum - cnt - base) : 0u);
-        const int width = __reduce_max_sync(full, in ? cum - base : 0);
-        const int c0 = __ffs(__ballot_sync(full, in)) - 1;   // its first column
-        const bool active = lane < width;
-        const unsigned upto = heads & (0xFFFFFFFFu >> (31 - lane));
-        const int col = c0 + __popc(upto) - 1;
-        const int hs = 31 - __clz(upto);
-        const int len = __shfl_sync(full, cnt, col);
-        const int src = __shfl_sync(full, beg, col) + lane - hs;
-        const unsigned seg = active ? (len == 32 ? full : ((1u << len) - 1u) << hs) : 0u;
-        const unsigned key = active ? keys[src] : 0u;
-        // rank within the column, equal keys in their present order
-        const int maxlen = __reduce_max_sync(full, active ? len : 0);
-        int rank = 0;
-        for (int k = 0; k < maxlen; k++) {
-          const unsigned x = __shfl_sync(full, key, hs + k);
-          rank += k < len && (x > key || (x == key && hs + k < lane));
-        }
-        if (active) scr[hs + rank] = key;
-        __syncwarp();
-        const unsigned sk = active ? scr[lane] : 0u;
-        const bool distinct = active && (lane == hs || scr[lane - 1] != sk);
-        __syncwarp();
-        const unsigned D = __ballot_sync(full, distinct);
-        const int nd = __popc(D & seg);
-        const PairOut r = pair_pixels(p, sk, distinct && nd > 1, seg, none);
-        // column sums: differences of the running sums at the column's ends
-        int vo = r.vo, vss = r.vss, tc = r.tc;
-        for (int d = 1; d < 32; d <<= 1) {
-          const int y0 = __shfl_up_sync(full, vo, d), y1 = __shfl_up_sync(full, vss, d);
-          if (lane >= d) { vo += y0; vss += y1; }
-        }
-        if (!p.explicit_ss)
-          for (int d = 1; d < 32; d <<= 1) {
-            const int y = __shfl_up_sync(full, tc, d);
-            if (lane >= d) tc += y;
-          }
-        const int hp = max(hs - 1, 0);
-        const int vo0 = __shfl_sync(full, vo, hp), vss0 = __shfl_sync(full, vss, hp), tc0 = __shfl_sync(full, tc, hp);
-        ColOut c;
-        c.vo = hs ? vo - vo0 : vo; c.vss = hs ? vss - vss0 : vss; c.tc = hs ? tc - tc0 : tc;
-        base += width;
-        const int cl = __shfl_sync(full, l, col), cls = __shfl_sync(full, ls, col);
-        c.vo = max(c.vo, 0);
-        c.ndist = nd;
-        if (last_px) {
-          const unsigned ds = D & seg;
-          const int lp = ds ? 31 - __clz(ds) : 0;
-          const int z = key_z(sk);
-          const unsigned ten = __ballot_sync(full, distinct && z == 1 && key_nz(sk) == 0);
-          c.lastz = __shfl_sync(full, z, lp);
-          c.lasttype = __shfl_sync(full, r.type, lp);
-          c.has10 = (ten & seg) != 0u;
-          const unsigned kept = (r.ka | r.kb) & seg;
-          const int lk = kept ? 31 - __clz(kept) : 0;
-          const bool open = kept && ((r.kb >> lk) & 1u);
-          const unsigned im = __ballot_sync(full, (r.type & kNVB) != 0);
-          finish(c, open && ((r.s >> lk) & 1u), open && ((im >> lk) & 1u));
-          if (dump && distinct) dump_key(p, xs0 * p.G + cls, __popc(ds & ((1u << lane) - 1u)), sk, r.type);
-        }
-        if (active && lane == hs + len - 1) store(cl, cls, c);
-        __syncwarp();
-      }
-    }
-  }
-  // ---- longer columns, one per warp
-  for (int b = wid; b < nbig; b += kColThreads / 32) {
-    const int l = longq[HG - 1 - b];
-    const int ls = olist[l];
-    const int beg = ls ? ends[ls - 1] : 0, cnt = ends[ls] - beg;
+  // ---- one long column by the whole warp
+  auto long_column = [&](int l, int ls, int beg, int cnt) {
     ColOut c;
     c.vo = c.vss = c.tc = 0; c.nfin = c.lastz = c.lasttype = c.has10 = 0;
     c.ndist = 0;
@@ -2021,7 +1942,7 @@ __global__ void __launch_bounds__(kColThreads, kColBlocks) k_columns(EngineParam
       c.ndist = nd;
       if (nd > kSlotCap) {               // first-come order decides which keys survive
         if (lane == 0) atomicOr(&sflag, kFlagCap);
-        continue;
+        return;
       }
       PairCarry cy = {false, false, false, false};
       int done = 0;
@@ -2080,7 +2001,7 @@ __global__ void __launch_bounds__(kColThreads, kColBlocks) k_columns(EngineParam
       }
       if (c.ndist > kSlotCap) {
         if (lane == 0) atomicOr(&sflag, kFlagCap);
-        continue;
+        return;
       }
       c.lastz = st.lastz; c.lasttype = st.lasttype; c.has10 = st.has10;
       if (c.ndist == 1) {                // duplicates of a single key
@@ -2096,6 +2017,99 @@ __global__ void __launch_bounds__(kColThreads, kColBlocks) k_columns(EngineParam
     if (last_px) finish(c, ex, im);
     if (lane == 0) store(l, ls, c);
     __syncwarp();
+  };
+
+  // ---- columns of one or two raw pixels, one per thread
+  for (int l0 = wid * 32; l0 < nocc; l0 += kColThreads) {
+    const int l = l0 + lane;
+    int cnt = 0;
+    if (l < nocc) {
+      const int ls = olist[l];
+      const int end = ends[ls], beg = ls ? ends[ls - 1] : 0;
+      cnt = end - beg;
+      if (cnt <= 2) {
+        const unsigned k0 = keys[beg], k1 = keys[end - 1];
+        const unsigned hi = max(k0, k1), lo = min(k0, k1);
+        const int z0 = key_z(hi), n0 = key_nz(hi), z1 = key_z(lo), n1 = key_nz(lo);
+        ColOut c;
+        c.vo = c.vss = c.tc = 0;
+        c.ndist = 1;
+        bool s1 = false, m1 = false;
+        if (hi != lo) {                  // a single distinct pixel is not paired
+          c.ndist = 2;
+          const bool up0 = n0 >= 1, up1 = !up0 && n1 >= 1, dn1 = up0 && n1 <= -1;
+          s1 = dn1 && n1 <= p.nz_ex; m1 = dn1 && n1 >= p.nz_im;
+          const int al = up0 ? z0 : (up1 ? z1 : 0), be = dn1 ? z1 : 0;
+          c.vo = max(al - be, 0);
+          if (p.explicit_ss) c.vss = s1 ? z1 : 0;
+          else { c.tc = al; c.vss = m1 ? 0 : be; }
+          if (last_px) {
+            const int tc = p.explicit_ss ? 0 : kTC;
+            const int t0 = up0 ? kAl | tc : 0, t1 = up1 ? kAl | tc : (dn1 ? kBe | (s1 ? kSSB : 0) | (m1 ? kNVB : 0) : 0);
+            c.lastz = z1; c.lasttype = t1;
+            c.has10 = (z0 == 1 && n0 == 0) || (z1 == 1 && n1 == 0);
+            if (dump) { dump_key(p, xs0 * p.G + ls, 0, hi, t0); dump_key(p, xs0 * p.G + ls, 1, lo, t1); }
+          }
+        } else if (last_px) {
+          c.lastz = z0; c.lasttype = 0;
+          c.has10 = z0 == 1 && n0 == 0;
+          if (dump) dump_key(p, xs0 * p.G + ls, 0, hi, 0);
+        }
+        if (last_px) finish(c, s1, m1);
+        store(l, ls, c);
+      }
+    }
+    // longer columns to their queues
+    if (cnt > 2) {
+      const int cls = cnt <= 4 ? 0 : (cnt <= 8 ? 1 : (cnt <= 16 ? 2 : 3));
+      const int at = atomicAdd(&nq[cls], 1);
+      (cls < 2 ? queue : queue2)[cls & 1 ? HG - 1 - at : at] = (unsigned short)l;
+    }
+  }
+  __syncthreads();
+
+  // ---- longer columns: chunks of 32 of one class, in turn to the warps
+  int c0 = 0;
+  for (int cls = 0; cls < 4; cls++) {
+    const int nc = nq[cls], chunks = (nc + 31) >> 5;
+    const unsigned short* const qu = cls < 2 ? queue : queue2;
+    for (int ch = (wid - c0) & (kColThreads / 32 - 1); ch < chunks; ch += kColThreads / 32) {
+      const int at = ch * 32 + lane;
+      int l = 0, ls = 0, beg = 0, cnt = 0;
+      if (at < nc) {
+        l = qu[cls & 1 ? HG - 1 - at : at];
+        ls = olist[l];
+        beg = ls ? ends[ls - 1] : 0;
+        cnt = ends[ls] - beg;
+      }
+      ColWalk w;
+      auto step = [&](unsigned key, int i) { w.step(p, key, i, last_px, dump ? xs0 * p.G + ls : -1); };
+      if (cnt <= 32) {
+        unsigned* const k = keys + beg;
+        for (int i = 1; i < cnt; i++) {   // insertion sort in place, descending
+          const unsigned key = k[i];
+          int j = i;
+          while (j > 0 && k[j - 1] < key) { k[j] = k[j - 1]; j--; }
+          k[j] = key;
+        }
+        for (int i = 0; i < cnt; i++) step(k[i], i);
+      }
+      if (cnt > 0 && cnt <= 32) {
+        ColOut c;
+        w.result(c);
+        if (last_px) finish(c, w.down && w.ex && w.nd > 1, w.down && w.im && w.nd > 1);
+        if (dump && w.nd == 1 && p.dump_types) p.dump_types[(size_t)(xs0 * p.G + ls) * 64] = 0;
+        store(l, ls, c);
+      }
+      unsigned longer = __ballot_sync(full, cnt > 32);
+      while (longer) {
+        const int from = __ffs(longer) - 1;
+        longer &= longer - 1;
+        long_column(__shfl_sync(full, l, from), __shfl_sync(full, ls, from), __shfl_sync(full, beg, from),
+                    __shfl_sync(full, cnt, from));
+      }
+    }
+    c0 = (c0 + chunks) & (kColThreads / 32 - 1);
   }
 
   // ---- reductions
