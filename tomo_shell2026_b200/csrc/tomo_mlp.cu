@@ -8,7 +8,7 @@
 //                  backward pass to the layers' inputs out of shared memory;
 //                  activations and pre-activation gradients go to global
 //                  memory (3 MB for 936 samples);
-//   k_mlp_update   one CTA per 16 x 16 weights (and per 32 of the rest): the
+//   k_mlp_update   one CTA per 16 x 16 weights (and per 16 of the rest): the
 //                  weight gradient over all samples, then the Adam update of
 //                  the parameter and of its transposed copy.
 //
@@ -16,8 +16,9 @@
 // in turn, the sums of eights r, r + 8, r + 16, ... of each r in 0..7, then the
 // eight of those.  When each CTA wrote its own gradient of all parameters and a
 // second kernel added them up (16 MB written and read a step), a step of 936
-// samples took 31 us; now 21 (B200, 300 steps replayed as a graph), most of it
-// the latency of four dependent 128-term sums and three activations.
+// samples took 31 us; now 21 (B200, 300 steps replayed as a graph): 12 of it four
+// dependent 128-term products and three activations on one warp per scheduler,
+// bound by shared-memory words, 5 the weight gradients, the rest launches.
 //
 // Weights are row-major [in][out]; the backward pass reads each matrix
 // through a transposed copy [out][in] kept in step with the parameters, so
@@ -47,10 +48,12 @@ __device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_grou
 template <int N>
 __device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N)); }
 
-// Start copying one 128 x 128 matrix into shared memory (one commit group).
-__device__ __forceinline__ void stage(const float* __restrict__ src, float* dst)
+// Start copying one 128 x 128 matrix into shared memory (one commit group), by
+// the threads from `first` on.
+__device__ __forceinline__ void stage(const float* __restrict__ src, float* dst, int first = 0)
 {
-  for (int k = threadIdx.x; k < kH * kH / 4; k += blockDim.x) cp16(dst + 4 * k, src + 4 * k);
+  if ((int)threadIdx.x < first) return;
+  for (int k = threadIdx.x - first; k < kH * kH / 4; k += blockDim.x - first) cp16(dst + 4 * k, src + 4 * k);
   cp_commit();
 }
 
@@ -69,7 +72,9 @@ __device__ __forceinline__ float2 fma2(float2 a, float2 w, float2 c)
 // x four samples, so that eight shared-memory words serve sixteen products (a
 // thread per unit with all eight samples took nine words for eight products,
 // and shared memory returns 32 words a cycle: 36 cycles per i instead of 16).
-// The next rows are read while these are used.
+// The next rows are read while these are used; the other warps stage the next
+// matrix meanwhile.  3,650 cycles (single products 4,300: a warp by itself on its
+// scheduler issues one every other cycle, packed or not).
 __device__ __forceinline__ void matmul8(const float (*in)[kSB], const float* W, const float* b, float (*out)[kSB])
 {
   constexpr int kRows = 8;
@@ -143,17 +148,20 @@ __global__ void __launch_bounds__(kH) k_mlp_pass(MlpLayout L, const float* __res
   PassShared& S = *reinterpret_cast<PassShared*>(smem_raw);
   const int j = threadIdx.x, warp = j >> 5, lane = j & 31;
   const int s0 = blockIdx.x * kSB, ns = min(kSB, n - s0);
-  stage(P + L.w[1], S.w[0]);
-  stage(P + L.w[2], S.w[1]);
+  // everything small that is read from global memory, before the matrices
   if (j < kSB * kMlpIn) {
     const int s = j / kMlpIn, i = j % kMlpIn;
     S.x[s][i] = s < ns ? x[(size_t)(s0 + s) * kMlpIn + i] : 0.f;
   }
   const float w4 = P[L.w[3] + j];
-  float w0[kMlpIn];
+  float w0[kMlpIn], w3[kH / 32];
 #pragma unroll
   for (int i = 0; i < kMlpIn; i++) w0[i] = P[L.w[0] + i * kH + j];
-  const float b0 = P[L.b[0] + j];
+#pragma unroll
+  for (int k = 0; k < kH / 32; k++) w3[k] = P[L.w[3] + lane + 32 * k];
+  const float b0 = P[L.b[0] + j], b3 = P[L.b[3]];
+  const float target = j < ns ? y[s0 + j] : 0.f;
+  stage(P + L.w[1], S.w[0]);
   __syncthreads();
   float v[kSB];
   // outputs of hidden layer l: shared (samples innermost) and global rows
@@ -171,8 +179,9 @@ __global__ void __launch_bounds__(kH) k_mlp_pass(MlpLayout L, const float* __res
     v[s] = tanhf(acc);
   }
   put(S.a[0], O.a[0]);
-  cp_wait<1>();
+  cp_wait<0>();
   __syncthreads();
+  stage(P + L.w[2], S.w[1], 64);
   matmul8(S.a[0], S.w[0], P + L.b[1], S.mm);
   __syncthreads();
 #pragma unroll
@@ -180,28 +189,28 @@ __global__ void __launch_bounds__(kH) k_mlp_pass(MlpLayout L, const float* __res
   put(S.a[1], O.a[1]);
   cp_wait<0>();
   __syncthreads();
-  stage(WT + L.w[2], S.w[0]);            // [out][in], for the backward pass
+  stage(WT + L.w[2], S.w[0], 64);        // [out][in], for the backward pass
   matmul8(S.a[1], S.w[1], P + L.b[2], S.mm);
   __syncthreads();
 #pragma unroll
   for (int s = 0; s < kSB; s++) v[s] = tanhf(S.mm[j][s]);
   put(S.a[2], O.a[2]);
+  cp_wait<0>();
   __syncthreads();
-  stage(WT + L.w[1], S.w[1]);
   for (int s = warp * 2; s < warp * 2 + 2; s++) {
     float acc = 0.f;
 #pragma unroll
-    for (int k = 0; k < kH / 32; k++) acc = __fmaf_rn(S.a[2][lane + 32 * k][s], P[L.w[3] + lane + 32 * k], acc);
+    for (int k = 0; k < kH / 32; k++) acc = __fmaf_rn(S.a[2][lane + 32 * k][s], w3[k], acc);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xFFFFFFFFu, acc, o);
-    if (lane == 0) S.yhat[s] = acc + P[L.b[3]];
+    if (lane == 0) S.yhat[s] = acc + b3;
   }
   __syncthreads();
   // loss and output-layer gradient
   if (j < 32) {
     float e = 0.f;
     if (j < kSB) {
-      const float d = j < ns ? S.yhat[j] - y[s0 + j] : 0.f;
+      const float d = j < ns ? S.yhat[j] - target : 0.f;
       S.dz4[j] = 2.f * d / (float)n;
       O.d4[s0 + j] = S.dz4[j];
       e = d * d / (float)n;
@@ -217,8 +226,8 @@ __global__ void __launch_bounds__(kH) k_mlp_pass(MlpLayout L, const float* __res
     v[s] = S.dz4[s] * w4 * (1.f - a * a);
   }
   put(S.dz[0], O.d[2]);
-  cp_wait<1>();
   __syncthreads();
+  stage(WT + L.w[1], S.w[1], 64);
   matmul8(S.dz[0], S.w[0], nullptr, S.mm);
   __syncthreads();
 #pragma unroll
@@ -370,130 +379,165 @@ __device__ __forceinline__ void adam_update(const MlpLayout& L, int p, float gi,
 
 constexpr int kTile = 16;                                       // 16 x 16 weights per CTA
 constexpr int kTilesPerLayer = (kH / kTile) * (kH / kTile);     // 64
-constexpr int kSmallPer = 32;                                   // other parameters per CTA
+constexpr int kUpdateThreads = 16 * kParts;                      // sixteen per partial sum
+constexpr int kSmallPer = 16;                                   // other parameters per CTA
+constexpr int kStages = 4;                                      // eights in flight per warp
 
 // The parameters outside the two 128 x 128 matrices, numbered 0 .. kSmall - 1:
 // W1, b1, b2, b3, W4, b4.
 constexpr int kSmall = kMlpIn * kH + 3 * kH + kH + 1;
 
-// Weight gradients and (update) the Adam step.  Warp r of a CTA sums the
-// partial gradients of the eights r, r + 8, ... (each eight in sample order);
+// Weight gradients and (update) the Adam step.  Sixteen threads r of a CTA sum
+// the partial gradients of the eights r, r + 8, ... (each eight in sample order);
 // the eight sums are then added in order.  nblk: eights of samples.
-__global__ void __launch_bounds__(32 * kParts) k_mlp_update(MlpLayout L, const float* __restrict__ x, PassOut O,
+__global__ void __launch_bounds__(kUpdateThreads) k_mlp_update(MlpLayout L, const float* __restrict__ x, PassOut O,
                                                             const float* __restrict__ part_loss, int nblk,
                                                             float* __restrict__ grad, float* __restrict__ loss,
                                                             int update, float* P, float* WT, float* m, float* v,
                                                             float lr, float bc1, float bc2)
 {
   __shared__ float red[kParts][kTile * kTile + 1];
-  const int lane = threadIdx.x & 31, r = threadIdx.x >> 5;
+  __shared__ __align__(16) float ring[kParts][kStages][2][kSB][kTile];   // activations, gradients
+  const int lane = threadIdx.x & 31;
   const int tile = blockIdx.x;
   if (tile < 2 * kTilesPerLayer) {
-    // 16 x 16 weights of layer l: a thread has 2 inputs x 4 outputs
+    // 16 x 16 weights of layer l: sixteen threads with 4 inputs x 4 outputs each,
+    // so a warp has two of the partial sums r.  Their eights arrive kStages - 1
+    // ahead (a row's 16 inputs and 16 outputs are four 16-byte pieces each, two of
+    // either per thread and eight).
     const int l = 1 + tile / kTilesPerLayer, q = tile % kTilesPerLayer;
-    const int i0 = q / (kH / kTile) * kTile + (lane >> 2) * 2, j0 = q % (kH / kTile) * kTile + (lane & 3) * 4;
-    const float* A = O.a[l - 1] + i0;
-    const float* D = O.d[l] + j0;
-    float acc[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
-    float2 a[kSB], an[kSB];
-    float4 d[kSB], dn[kSB];
-    auto load = [&](int b, float2* pa, float4* pd) {
+    const int t = lane & 15, r = threadIdx.x >> 4;
+    const int ti = (t >> 2) * 4, tj = (t & 3) * 4;
+    const float* A = O.a[l - 1] + q / (kH / kTile) * kTile + (t >> 2) * kH + tj;
+    const float* D = O.d[l] + q % (kH / kTile) * kTile + (t >> 2) * kH + tj;
+    float acc[4][4];
 #pragma unroll
-      for (int s = 0; s < kSB; s++) {
-        pa[s] = *reinterpret_cast<const float2*>(A + (size_t)(b * kSB + s) * kH);
-        pd[s] = *reinterpret_cast<const float4*>(D + (size_t)(b * kSB + s) * kH);
+    for (int h = 0; h < 4; h++)
+#pragma unroll
+      for (int c = 0; c < 4; c++) acc[h][c] = 0.f;
+    auto fetch = [&](int b, int k) {
+      if (b < nblk) {
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+          cp16(&ring[r][k % kStages][0][(t >> 2) + 4 * h][tj], A + ((size_t)b * kSB + 4 * h) * kH);
+          cp16(&ring[r][k % kStages][1][(t >> 2) + 4 * h][tj], D + ((size_t)b * kSB + 4 * h) * kH);
+        }
       }
+      cp_commit();
     };
-    if (r < nblk) load(r, a, d);
-    for (int b = r; b < nblk; b += kParts) {
-      if (b + kParts < nblk) load(b + kParts, an, dn);   // the next eight, while this one is summed
-      float p[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
 #pragma unroll
-      for (int s = 0; s < kSB; s++) {
-        p[0][0] = __fmaf_rn(a[s].x, d[s].x, p[0][0]); p[0][1] = __fmaf_rn(a[s].x, d[s].y, p[0][1]);
-        p[0][2] = __fmaf_rn(a[s].x, d[s].z, p[0][2]); p[0][3] = __fmaf_rn(a[s].x, d[s].w, p[0][3]);
-        p[1][0] = __fmaf_rn(a[s].y, d[s].x, p[1][0]); p[1][1] = __fmaf_rn(a[s].y, d[s].y, p[1][1]);
-        p[1][2] = __fmaf_rn(a[s].y, d[s].z, p[1][2]); p[1][3] = __fmaf_rn(a[s].y, d[s].w, p[1][3]);
+    for (int k = 0; k < kStages - 1; k++) fetch(r + k * kParts, k);
+    const int turns = (nblk + kParts - 1) / kParts;   // the same for both halves of a warp
+    for (int k = 0; k < turns; k++) {
+      const int b = r + k * kParts;
+      cp_wait<kStages - 2>();
+      __syncwarp();
+      fetch(b + (kStages - 1) * kParts, k + kStages - 1);   // into the stage read one turn ago
+      if (b < nblk) {
+        float p[4][4];
+#pragma unroll
+        for (int h = 0; h < 4; h++)
+#pragma unroll
+          for (int c = 0; c < 4; c++) p[h][c] = 0.f;
+#pragma unroll
+        for (int s = 0; s < kSB; s++) {
+          const float4 a = *reinterpret_cast<const float4*>(&ring[r][k % kStages][0][s][ti]);
+          const float4 d = *reinterpret_cast<const float4*>(&ring[r][k % kStages][1][s][tj]);
+          const float av[4] = {a.x, a.y, a.z, a.w}, dv[4] = {d.x, d.y, d.z, d.w};
+#pragma unroll
+          for (int h = 0; h < 4; h++)
+#pragma unroll
+            for (int c = 0; c < 4; c++) p[h][c] = __fmaf_rn(av[h], dv[c], p[h][c]);
+        }
+#pragma unroll
+        for (int h = 0; h < 4; h++)
+#pragma unroll
+          for (int c = 0; c < 4; c++) acc[h][c] += p[h][c];
       }
-#pragma unroll
-      for (int h = 0; h < 2; h++)
-#pragma unroll
-        for (int c = 0; c < 4; c++) acc[h][c] += p[h][c];
-#pragma unroll
-      for (int s = 0; s < kSB; s++) { a[s] = an[s]; d[s] = dn[s]; }
+      __syncwarp();
     }
 #pragma unroll
-    for (int h = 0; h < 2; h++)
+    for (int h = 0; h < 4; h++)
 #pragma unroll
-      for (int c = 0; c < 4; c++) red[r][((lane >> 2) * 2 + h) * kTile + (lane & 3) * 4 + c] = acc[h][c];
+      for (int c = 0; c < 4; c++) red[r][(ti + h) * kTile + tj + c] = acc[h][c];
     __syncthreads();
-    const int t = threadIdx.x;   // one weight per thread
-    float gi = 0.f;
+    for (int e = threadIdx.x; e < kTile * kTile; e += kUpdateThreads) {
+      float gi = 0.f;
 #pragma unroll
-    for (int k = 0; k < kParts; k++) gi += red[k][t];
-    const int w = L.w[l] + (q / (kH / kTile) * kTile + t / kTile) * kH + q % (kH / kTile) * kTile + t % kTile;
-    grad[w] = gi;
-    if (update) adam_update(L, w, gi, P, WT, m, v, lr, bc1, bc2);
+      for (int k = 0; k < kParts; k++) gi += red[k][e];
+      const int w = L.w[l] + (q / (kH / kTile) * kTile + e / kTile) * kH + q % (kH / kTile) * kTile + e % kTile;
+      grad[w] = gi;
+      if (update) adam_update(L, w, gi, P, WT, m, v, lr, bc1, bc2);
+    }
     return;
   }
-  // the rest: lane = parameter, warp = partial sum
-  const int k = (tile - 2 * kTilesPerLayer) * kSmallPer + lane;
+  if (blockIdx.x == gridDim.x - 1) {
+    // the loss: the eights' losses in order
+    float e = 0.f;
+    float* const part = &ring[0][0][0][0][0];
+    for (int b0 = 0; b0 < nblk; b0 += kUpdateThreads) {
+      if (b0 + (int)threadIdx.x < nblk) part[threadIdx.x] = part_loss[b0 + threadIdx.x];
+      __syncthreads();
+      if (threadIdx.x == 0) {
+        const int m = min(kUpdateThreads, nblk - b0);
+#pragma unroll 8
+        for (int k = 0; k < m; k++) e += part[k];
+      }
+      __syncthreads();
+    }
+    if (threadIdx.x == 0) *loss = e;
+    return;
+  }
+  // the rest: 16 parameters, a thread per parameter and partial sum; four eights'
+  // factors are read before the first is used
+  const int t = threadIdx.x & 15, r = threadIdx.x >> 4;
+  const int k = (tile - 2 * kTilesPerLayer) * kSmallPer + t;
   int par = -1;
-  float acc = 0.f;
+  const float *u = nullptr, *v2 = nullptr;   // the factors' first values; v2 null: the sum of u alone
+  int su = kH, sv = 0;                        // and their strides from sample to sample
   if (k < kSmall) {
     int e = k;
     if (e < kMlpIn * kH) {
-      par = L.w[0] + e;
-      const int i = e / kH, j = e % kH;
-      for (int b = r; b < nblk; b += kParts) {
-        float p = 0.f;
-#pragma unroll
-        for (int s = 0; s < kSB; s++)
-          p = __fmaf_rn(x[(size_t)(b * kSB + s) * kMlpIn + i], O.d[0][(size_t)(b * kSB + s) * kH + j], p);
-        acc += p;
-      }
+      par = L.w[0] + e; u = x + e / kH; su = kMlpIn; v2 = O.d[0] + e % kH; sv = kH;
     } else if ((e -= kMlpIn * kH) < 3 * kH) {
-      const int l = e / kH, j = e % kH;
-      par = L.b[l] + j;
-      for (int b = r; b < nblk; b += kParts) {
-        float p = 0.f;
-#pragma unroll
-        for (int s = 0; s < kSB; s++) p += O.d[l][(size_t)(b * kSB + s) * kH + j];
-        acc += p;
-      }
+      par = L.b[e / kH] + e % kH; u = O.d[e / kH] + e % kH;
     } else if ((e -= 3 * kH) < kH) {
-      par = L.w[3] + e;
-      for (int b = r; b < nblk; b += kParts) {
-        float p = 0.f;
-#pragma unroll
-        for (int s = 0; s < kSB; s++) p = __fmaf_rn(O.a[2][(size_t)(b * kSB + s) * kH + e], O.d4[b * kSB + s], p);
-        acc += p;
-      }
+      par = L.w[3] + e; u = O.a[2] + e; v2 = O.d4; sv = 1;
     } else {
-      par = L.b[3];
-      for (int b = r; b < nblk; b += kParts) {
+      par = L.b[3]; u = O.d4; su = 1;
+    }
+  }
+  float acc = 0.f;
+  constexpr int kAhead = 4;
+  if (par >= 0)
+    for (int b0 = r; b0 < nblk; b0 += kAhead * kParts) {
+      float fu[kAhead][kSB], fv[kAhead][kSB];
+#pragma unroll
+      for (int a = 0; a < kAhead; a++)
+#pragma unroll
+        for (int s = 0; s < kSB; s++) {
+          const int row = (b0 + a * kParts) * kSB + s;
+          const bool in = b0 + a * kParts < nblk;
+          fu[a][s] = in ? u[(size_t)row * su] : 0.f;
+          fv[a][s] = in && v2 ? v2[(size_t)row * sv] : 0.f;
+        }
+#pragma unroll
+      for (int a = 0; a < kAhead; a++) {
+        if (b0 + a * kParts >= nblk) break;
         float p = 0.f;
 #pragma unroll
-        for (int s = 0; s < kSB; s++) p += O.d4[b * kSB + s];
+        for (int s = 0; s < kSB; s++) p = v2 ? __fmaf_rn(fu[a][s], fv[a][s], p) : p + fu[a][s];
         acc += p;
       }
     }
-  }
-  red[r][lane] = acc;
+  red[r][t] = acc;
   __syncthreads();
   if (r == 0 && par >= 0) {
     float gi = 0.f;
 #pragma unroll
-    for (int q = 0; q < kParts; q++) gi += red[q][lane];
+    for (int q = 0; q < kParts; q++) gi += red[q][t];
     grad[par] = gi;
     if (update) adam_update(L, par, gi, P, WT, m, v, lr, bc1, bc2);
-  }
-  // the loss: the eights' losses in order
-  if (tile == 2 * kTilesPerLayer && r == 1 && lane == 0) {
-    float e = 0.f;
-#pragma unroll 8
-    for (int b = 0; b < nblk; b++) e += part_loss[b];
-    *loss = e;
   }
 }
 
@@ -681,8 +725,8 @@ cudaError_t Mlp::step(float lr, bool update, cudaStream_t s)
     bc1 = 1.f - std::pow(0.9f, (float)t);
     bc2 = 1.f - std::pow(0.999f, (float)t);
   }
-  const int grid = 2 * kTilesPerLayer + (kSmall + kSmallPer - 1) / kSmallPer;
-  k_mlp_update<<<grid, 32 * kParts, 0, s>>>(L, x_, O, part_loss_, nblk, grads_, loss_, update ? 1 : 0, params_, wt_,
+  const int grid = 2 * kTilesPerLayer + (kSmall + kSmallPer - 1) / kSmallPer + 1;
+  k_mlp_update<<<grid, kUpdateThreads, 0, s>>>(L, x_, O, part_loss_, nblk, grads_, loss_, update ? 1 : 0, params_, wt_,
                                             m_, v_, lr, bc1, bc2);
   MLP_TRY(cudaGetLastError());
   if (update) steps_done_++;
