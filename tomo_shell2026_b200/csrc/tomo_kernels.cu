@@ -2170,35 +2170,103 @@ __device__ bool bed_candidate(const EngineParams& p, const uint8_t* bedf, int X,
   return false;
 }
 
-__global__ void __launch_bounds__(256) k_bed(EngineParams p)
+constexpr int kBedWarps = 4;
+constexpr int kBedRun = 32;      // slot columns a warp walks
+constexpr int kBedRing = 64;     // rows kept: a window has at most 2 * 31
+constexpr int kBedFar = 255;     // no contact within reach
+
+// Bed pixels of every orientation, for windows of up to 31 pixels (bed_candidate
+// for wider ones).  A warp walks kBedRun slot columns of 32 pixels each.  Three
+// ballots per column give its floor contacts, in which every lane finds the
+// nearest within the window on either side by a shift and a bit scan, once; a
+// pixel's squared distance is then the least dx^2 + dy^2 over the columns of its
+// window.  Distances compare as squared whole numbers, whose float root the
+// reference's minimum is.  Looking at every slot of every pixel's window took 134
+// us per 256 orientations of a 140-pixel part with a 3-pixel skirt, scanning the
+// ballots anew for every pixel column 138.
+__global__ void __launch_bounds__(32 * kBedWarps) k_bed(EngineParams p)
 {
-  __shared__ int wsum[8];
+  // per column of the window and lane: nearest contact of all; of those still
+  // visible from later scan positions; and for the pixel's own column, where a
+  // contact at an earlier position that a raft pixel hides does not count
+  __shared__ uint8_t ring[kBedWarps][3][kBedRing][32];
+  __shared__ int wsum[kBedWarps];
+  const unsigned full = 0xFFFFFFFFu;
   const int o = blockIdx.y;
   const int fl = p.flags[o];
-  if (fl & kFlagRedo) return;
+  if ((fl & kFlagRedo) || p.bbox[o * 4 + 2] < 0) return;   // out_nbed starts at zero
   const int id = p.ori[o];
-  if (p.bed_type == kBedNone || p.bed_r <= 0 || p.bbox[o * 4 + 2] < 0) {
-    if (blockIdx.x == 0 && threadIdx.x == 0) p.out_nbed[id] = 0;
-    return;
-  }
-  const int m = (int)p.bed_outer + 1;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int m = (int)p.bed_outer + 1, r = p.bed_r;
   const int bx0 = max(p.bbox[o * 4 + 0] - m, 0), bx1 = min(p.bbox[o * 4 + 2] + m + 1, p.G);
   const int by0 = max(p.bbox[o * 4 + 1] - m, 0), by1 = min(p.bbox[o * 4 + 3] + m + 1, p.G);
-  const int w = by1 - by0;
-  const int n = (bx1 - bx0) * w;
-  const uint8_t* bedf = p.bedf + (size_t)o * p.G * p.G;
+  const int words = (by1 - by0 + 31) >> 5, runs = (bx1 - bx0 + kBedRun - 1) / kBedRun;
+  const uint8_t* const bedf = p.bedf + (size_t)o * p.G * p.G;
+  const unsigned up_mask = r < 32 ? (1u << r) - 1u : 0u, down_mask = r < 32 ? full << (32 - r) : 0u;
   int cnt = 0;
-  for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < n; q += gridDim.x * blockDim.x) {
-    const int X = bx0 + q / w, Y = by0 + q % w;
-    const uint8_t f = bedf[X * p.G + Y];
-    if ((f & kBfPoss) && (f & kBfLand) && bed_candidate(p, bedf, X, Y)) cnt++;
+  for (int u = blockIdx.x * kBedWarps + wid; u < words * runs; u += gridDim.x * kBedWarps) {
+    const int Y0 = by0 + u % words * 32, Y = Y0 + lane;
+    const int X0 = bx0 + u / words * kBedRun, X1 = min(X0 + kBedRun, bx1);
+    if (r > 31) {
+      for (int X = X0; X < X1; X++) {
+        const uint8_t f = Y < by1 ? bedf[(size_t)X * p.G + Y] : 0;
+        cnt += (f & kBfPoss) && (f & kBfLand) && bed_candidate(p, bedf, X, Y);
+      }
+      continue;
+    }
+    constexpr int kRows = 4;             // columns read before the first is used
+    for (int s0 = X0 - r; s0 < X1 + r - 1; s0 += kRows) {
+      unsigned f[kRows][3];
+#pragma unroll
+      for (int i = 0; i < kRows; i++)
+#pragma unroll
+        for (int k = 0; k < 3; k++) {
+          const int sx = s0 + i, y = Y0 + 32 * (k - 1) + lane;
+          f[i][k] = (unsigned)sx < (unsigned)p.G && (unsigned)y < (unsigned)p.G ? bedf[(size_t)sx * p.G + y] : 0u;
+        }
+#pragma unroll
+      for (int i = 0; i < kRows; i++) {
+        const int sx = s0 + i;
+        unsigned all[3], late[3];
+#pragma unroll
+        for (int k = 0; k < 3; k++) {
+          all[k] = __ballot_sync(full, f[i][k] & kBfTouch);
+          late[k] = __ballot_sync(full, (f[i][k] & (kBfTouch | kBfSelfR)) == kBfTouch);
+        }
+        auto up = [&](const unsigned* w) {     // at or above the pixel: 0 .. r - 1
+          const unsigned x = __funnelshift_r(w[1], w[2], lane) & up_mask;
+          return x ? __ffs(x) - 1 : kBedFar;
+        };
+        auto down = [&](const unsigned* w) {   // below: 1 .. r
+          const unsigned x = __funnelshift_r(w[0], w[1], lane) & down_mask;
+          return x ? __clz(x) + 1 : kBedFar;
+        };
+        const int ua = up(all), dl = down(late);
+        ring[wid][0][sx & (kBedRing - 1)][lane] = (uint8_t)min(ua, down(all));
+        ring[wid][1][sx & (kBedRing - 1)][lane] = (uint8_t)min(up(late), dl);
+        ring[wid][2][sx & (kBedRing - 1)][lane] = (uint8_t)min(ua, dl);
+        const int X = sx - (r - 1);            // the pixel column whose window ends here
+        if (X < X0 || X >= X1) continue;
+        const uint8_t own = Y < by1 ? bedf[(size_t)X * p.G + Y] : 0;
+        const bool open = (own & kBfPoss) && (own & kBfLand);
+        if (!__any_sync(full, open)) continue;
+        int best = INT_MAX;
+        for (int dx = -r; dx < r; dx++) {
+          const int d = ring[wid][dx < 0 ? 1 : (dx > 0 ? 0 : 2)][(X + dx) & (kBedRing - 1)][lane];
+          if (d != kBedFar) best = min(best, dx * dx + d * d);
+        }
+        const float md = best < INT_MAX ? __fsqrt_rn((float)best) : 1e5f;
+        const bool near = md <= p.bed_outer && (p.bed_type != kBedSkirt || md > p.bed_inner);
+        cnt += open && near;
+      }
+    }
   }
-  cnt = warp_sum(cnt);
-  if ((threadIdx.x & 31) == 0) wsum[threadIdx.x >> 5] = cnt;
+  cnt = __reduce_add_sync(full, cnt);
+  if (lane == 0) wsum[wid] = cnt;
   __syncthreads();
   if (threadIdx.x == 0) {
     int t = 0;
-    for (int k = 0; k < 8; k++) t += wsum[k];
+    for (int k = 0; k < kBedWarps; k++) t += wsum[k];
     if (t) atomicAdd(&p.out_nbed[id], t);
   }
 }
@@ -2622,7 +2690,9 @@ cudaError_t launch_strip_bed(const EngineParams& p, cudaStream_t main, size_t st
   if (p.mode == 0) TOMO_LAUNCH(kind, main, (k_columns<<<dim3(p.S, p.Bo), kColThreads, strip_smem, main>>>(p)));
   else if (p.mode == 2) TOMO_LAUNCH(kind, main, (k_strip<2><<<dim3(p.S, p.Bo), 256, strip_smem, main>>>(p)));
   else TOMO_LAUNCH(kind, main, (k_strip<1><<<dim3(p.S, p.Bo), 256, strip_smem, main>>>(p)));
-  TOMO_LAUNCH(kKBed, main, (k_bed<<<dim3(8, p.Bo), 256, 0, main>>>(p)));
+  // without a bed the pixel counts stay the zeros they are initialised with
+  if (p.bed_type != kBedNone && p.bed_r > 0)
+    TOMO_LAUNCH(kKBed, main, (k_bed<<<dim3(16, p.Bo), 32 * kBedWarps, 0, main>>>(p)));
   return cudaGetLastError();
 }
 
