@@ -519,8 +519,8 @@ __global__ void __launch_bounds__(256) k_bin_fill(EngineParams p)
 // orientations in turn the strip counters' atomics were waited for (1.33 ms
 // per 256 orientations of the 82k solid; orientations mixed 1.15, with the
 // cheaper masks, the stash and several groups per warp 0.95).  Blocks of four
-// warps, seven to an SM: the 72 registers the loop needs (64 spill: 0.96 ms at
-// 32 warps; 80 without spills at 24 warps: 1.01).
+// warps, eight to an SM at 64 registers: 0.91 ms with the fallback pixel in shared
+// memory (seven at 72 registers 0.92, six at 80 1.01, nine at 56 0.95).
 //
 // Bound by instruction issue (80 % of cycles; 8 bytes written per accepted
 // pixel, 0.4 GB per 256 orientations of the 82k solid: 0.4 TB/s).  Rasterizing in the strip
@@ -541,6 +541,7 @@ struct RastWarp {
   float4 q0[32], q1[32], q2[32];   // margined vertices, vertex-normal z
   float4 q3[32];                   // d00, d01, d11, denom
   unsigned org[32];                // first pixel of each lane's cell, x | y << 16
+  float fb[3][32];                 // centroid fallback of each lane's triangle
   uint2 st[kStash];                // accepted pixels: key, slot x | y << 16 (0xFFFFFFFF: outside the grid)
   unsigned st2[kStash];            // their shell twins' keys
   unsigned short q[32 * 32];       // candidates: lane of the cell << 5 | pixel in the cell
@@ -633,7 +634,7 @@ __device__ __forceinline__ void flush(const EngineParams& p, int o, const RastWa
 }
 
 template <bool kTwin>
-__global__ void __launch_bounds__(32 * kRastWarps, 7) k_raster(EngineParams p)
+__global__ void __launch_bounds__(32 * kRastWarps, 8) k_raster(EngineParams p)
 {
   __shared__ RastWarp warps[kRastWarps];
   // consecutive blocks take the same triangles of kRastMix orientations: the
@@ -668,7 +669,6 @@ __global__ void __launch_bounds__(32 * kRastWarps, 7) k_raster(EngineParams p)
     const int t = (group << gshift) + (lane >> lsh);
     MaskTri T;
     int own = lane & ~(L - 1);            // lane that holds this lane's triangle
-    float fbx = 0.f, fby = 0.f, fbz = 0.f, n0 = 0.f;   // centroid fallback (STomoSh_INT3.cpp:1190-1206)
     unsigned hits = 0u;                   // lanes whose triangle has an accepted pixel (warp-uniform)
     unsigned big = 0u;                    // triangles left to the whole warp
     int from = 0;                         // their first cell left
@@ -696,8 +696,10 @@ __global__ void __launch_bounds__(32 * kRastWarps, 7) k_raster(EngineParams p)
         R.q2[own] = make_float4(cc.x, cc.y, cz.x, cz.y);
         R.q3[own] = make_float4(d00, d01, d11, denom);
         if (first) {
-          fbx = centroid(ua.x, ub.x, uc.x); fby = centroid(ua.y, ub.y, uc.y); fbz = centroid(va.x, vb.x, vc.x);
-          n0 = az.y;
+          // centroid fallback (STomoSh_INT3.cpp:1190-1206)
+          R.fb[0][lane] = centroid(ua.x, ub.x, uc.x);
+          R.fb[1][lane] = centroid(ua.y, ub.y, uc.y);
+          R.fb[2][lane] = centroid(va.x, vb.x, vc.x);
         }
         const float minx = fminf(fminf(a.x, b.x), cc.x), maxx = fmaxf(fmaxf(a.x, b.x), cc.x);
         const float miny = fminf(fminf(a.y, b.y), cc.y), maxy = fmaxf(fmaxf(a.y, b.y), cc.y);
@@ -797,7 +799,8 @@ __global__ void __launch_bounds__(32 * kRastWarps, 7) k_raster(EngineParams p)
       room();
       if (miss) {
         const int e = ns + __popc(who & below);
-        R.st[e] = make_uint2(pixel_key(fbz, n0), slot_xy(p, fbx, fby));
+        const float fbz = R.fb[2][lane], n0 = R.q0[lane].w;
+        R.st[e] = make_uint2(pixel_key(fbz, n0), slot_xy(p, R.fb[0][lane], R.fb[1][lane]));
         if (kTwin) R.st2[e] = pixel_key(__fadd_rn(fbz, (n0 >= 0.0f) ? -p.shell_off : p.shell_off), -n0);
       }
       ns += __popc(who);
@@ -2647,11 +2650,12 @@ int raster_lanes_log2(int nT, int Bo)
 }
 
 // Blocks per orientation: each warp takes several groups of triangles in turn
-// (its stash then fills whole rounds), while kRastFill warps are left.
+// (its stash then fills whole rounds), while four waves of warps are left (5k
+// solid, 256 orientations: 85 us at one wave, 81 at four).
 static int raster_blocks(int ngroup, int Bo)
 {
   int per = kRastGroups;
-  while (per > 1 && (long long)Bo * (ngroup / per) < kRastFill) per--;
+  while (per > 1 && (long long)Bo * (ngroup / per) < 4 * kRastFill) per--;
   return std::min((ngroup + kRastWarps * per - 1) / (kRastWarps * per), 65535);
 }
 
