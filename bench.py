@@ -13,8 +13,8 @@ shadows, theta_c = 60 degrees, no bed.
 Prints one JSON line (rank 0).  ``value`` is orientations/s of the device
 sweep with mesh and orientations resident in device memory (CUDA events on
 the engine's stream); ``e2e`` is the same metric through the reference
-C-ABI call TomoSh_CUDA with host buffers; ``roofline`` rates the dominant
-kernel (k_strip) against the measured HBM copy bandwidth; ``cpu_baseline``
+C-ABI call TomoSh_CUDA with host buffers; ``roofline`` rates the two dominant
+kernels (k_raster and k_columns) against the measured HBM copy bandwidth; ``cpu_baseline``
 is the reference INT3 engine (built from the reference sources) on the
 host cores over a bounded sample of the same orientations.  With N > 1
 (torchrun) the ranks split the one headline sweep into contiguous
@@ -304,15 +304,18 @@ def run_ours(args, rank, world, local_rank):
     except Exception as exc:   # a measurement aid: never costs the bench line
         print(f"read probe skipped: {exc}", file=sys.stderr)
 
-    # ---- roofline of the dominant kernel (k_strip), live event timing
+    # ---- roofline of the two dominant kernels, live event timing: k_raster
+    # writes each accepted pixel to its strip's list, k_columns (logged as
+    # k_strip) reads the lists
     peaks = _peaks()
-    strip = klog["k_strip"]
+    strip = dict(klog["k_strip"])
+    strip["ms"] += klog["k_raster"]["ms"]
     algo_bytes_per_orient = 24 * mesh.n_vtx + 12 * mesh.n_tri + 16 * res["entries"].astype(np.float64) + 16
     algo_bytes = float(algo_bytes_per_orient.sum()) * args.steps
     strip_ms = strip["ms"] if strip["timed"] else float("nan")
     achieved = algo_bytes / (strip_ms / 1000.0) / 1e9 if strip["timed"] else None
     launches_per_step = {k: v["launches"] / args.steps for k, v in klog.items()}
-    roof = {"bound": "hbm", "kernel": "k_strip", "achieved": achieved, "peak": peaks[0], "unit": "GB/s",
+    roof = {"bound": "hbm", "kernel": "k_raster + k_columns", "achieved": achieved, "peak": peaks[0], "unit": "GB/s",
             "frac": (achieved / peaks[0]) if achieved else None, "peak_source": peaks[1],
             "traffic": _traffic(mesh, res, strip["launches"] / args.steps),
             "avg_launch_ms": strip_ms / max(strip["timed"], 1),
@@ -419,8 +422,8 @@ def _peaks():
 
 
 def _traffic(mesh, res, launches_per_step):
-    """DRAM bytes per k_strip launch from the committed ncu summary, when
-    present, scaled from its launch size to this run's orientations per launch."""
+    """DRAM bytes per k_raster + k_columns launch pair from the committed ncu summary,
+    when present, scaled from its launch size to this run's orientations per launch."""
     p = ROOT / "profiles" / "k_strip_traffic.json"
     if not p.exists() or not launches_per_step:
         return None

@@ -190,8 +190,8 @@ struct DevBuf {
 constexpr int kMaxGrid = 4096;
 
 // Most bytes of one batch's strip pixel lists (256 orientations of the
-// 501-column grid take 1.2 GB, two such sets at once; wide grids sweep fewer
-// orientations per batch).
+// 491-column grid take 2.3 GB, two such sets at once; wide grids sweep fewer
+// orientations per batch, and so does a device that cannot hold them).
 constexpr size_t kListBytes = size_t(6) << 30;
 
 // Orientations the last tomoSweepStatic call re-ran, per strip configuration.
@@ -608,6 +608,18 @@ struct Engine {
     return 0;
   }
 
+  // reserve_batch for as many orientations as the device can hold: a batch is
+  // halved while its buffers do not fit.
+  int reserve_fitting(int mode, int* Bo, int bin_cap, int want, int* nprep)
+  {
+    for (;;) {
+      *nprep = want > *Bo ? 2 : 1;
+      const int rc = reserve_batch(mode, *Bo, bin_cap, *nprep);
+      if (rc == 0 || *Bo <= 1 || cudaGetLastError() != cudaErrorMemoryAllocation) return rc;
+      *Bo = (*Bo + 1) / 2;
+    }
+  }
+
   int reserve_outputs()
   {
     const size_t n = (size_t)std::max(nYPR, 1);
@@ -706,8 +718,9 @@ struct Engine {
     // PrepSet while batch k's strips run on main; each batch's fold follows
     // on the side stream.  A set is rebinned only after the fold of the
     // batch that last used it.
-    const bool pipe = n > Bo;
-    TOMO_TRY(reserve_batch(cfg[c].mode, Bo, bin_cap, pipe ? 2 : 1));
+    int nprep = 1;
+    TOMO_TRY(reserve_fitting(cfg[c].mode, &Bo, bin_cap, n, &nprep));
+    const bool pipe = nprep > 1;
     if (ids) TOMO_CUDA(launch_zero_ids(o_nbed.ptr, ids, n, main));
     else TOMO_CUDA(cudaMemsetAsync(o_nbed.ptr, 0, sizeof(int) * nYPR, main));
     if (pipe) {
@@ -743,7 +756,8 @@ struct Engine {
           // every launch so far has finished (adapt_after waited), so the
           // lists may move; the rest of the sweep may need smaller batches
           Bo = batch_size(Bo, cfg[c].mode);
-          TOMO_TRY(reserve_batch(cfg[c].mode, Bo, bin_cap, pipe ? 2 : 1));
+          int sets = nprep;
+          TOMO_TRY(reserve_fitting(cfg[c].mode, &Bo, bin_cap, pipe ? INT_MAX : 0, &sets));
           p = base_params(cfg[c].mode);
         }
       }
@@ -766,9 +780,9 @@ struct Engine {
     DevBuf<int> sub;
     TOMO_CUDA(sub.reserve(ids.size()));
     TOMO_CUDA(cudaMemcpyAsync(sub.ptr, ids.data(), sizeof(int) * ids.size(), cudaMemcpyHostToDevice, main));
-    const int Bo = batch_size(std::min<int>(batch, (int)ids.size()), mode);
+    int Bo = batch_size(std::min<int>(batch, (int)ids.size()), mode), one = 1;
     const int normal_cap = 4 * P.n_tri + 4096;
-    TOMO_TRY(reserve_batch(mode, Bo, mode != 1 ? normal_cap : 1));
+    TOMO_TRY(reserve_fitting(mode, &Bo, mode != 1 ? normal_cap : 1, 0, &one));
     EngineParams p = base_params(mode);
     p.variant = c;
     for (int first = 0; first < (int)ids.size(); first += Bo) {
@@ -2008,8 +2022,10 @@ struct MultiEngine {
       e->choose_strips(c);
       TOMO_TRY(e->configure());
       TOMO_TRY(e->reserve_outputs());
-      const int Bo = e->batch_size(std::min(e->batch, e->nYPR), mode);
-      TOMO_TRY(e->reserve_batch(mode, Bo, 4 * e->P.n_tri + 4096, e->nYPR > Bo ? 2 : 1));
+      const int ask = std::min(e->batch, e->nYPR);
+      int Bo = e->batch_size(ask, mode), sets = 1;
+      TOMO_TRY(e->reserve_fitting(mode, &Bo, 4 * e->P.n_tri + 4096, e->nYPR, &sets));
+      if (Bo < ask) e->batch = Bo;   // the capture must find every buffer in place
     }
     return 0;
   }
