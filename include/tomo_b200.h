@@ -90,7 +90,7 @@ void tomoVolToMass(const float* f32info, const int* i32info, float* vm22);
 #define TOMO_OPT_STRIP_H 2      /* force strip height 1, 2, 4 or 8 (0 = automatic) */
 #define TOMO_OPT_FORCE_SAFE 3   /* 1 = evaluate every orientation in safe mode */
 #define TOMO_OPT_NORMAL_SMEM 4  /* shared-memory budget of a normal strip, in bytes: its pixel capacity is what is left beside four
-                                   bytes and a bit per slot and a 20 KB work area, at 6 bytes a pixel (0 = what four CTAs per SM hold) */
+                                   bytes and a bit per slot and a 20 KB work area, at 6 bytes a pixel (0 = what six CTAs per SM hold) */
 #define TOMO_OPT_EXPORT 5       /* 0 = skip the best orientation's pixel export (default 1) */
 #define TOMO_OPT_ADAPTIVE 6     /* 0 = keep the planned strip budget even when early batches overflow (default 1) */
 #define TOMO_OPT_PROPOSAL 7     /* tomoSurrogateSearch proposals: 0 = the trained network (default), 1 = bilinear
@@ -174,7 +174,7 @@ int TomoSh_CUDA_Batch(int n_mesh, const float* const* f32info, const int* const*
  * orientations re-run, time of the last run in microseconds (sweep and
  * re-runs, as device_ms), time of its sweep alone (the graph replay) */
 int tomoBatchStats(long long* out, int n);
-/* out4 = orientations per batch, normal-CTA shared-memory budget (0 = four CTAs per SM),
+/* out4 = orientations per batch, normal-CTA shared-memory budget (0 = six CTAs per SM),
  * strip height, slot-grid edge chosen for mesh `mesh` */
 int tomoBatchConfig(int mesh, int* out4);
 /* The TomoSh_CUDA tail for mesh `mesh` of the last tomoBatchRun: the getters

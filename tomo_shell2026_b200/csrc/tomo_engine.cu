@@ -190,7 +190,7 @@ struct DevBuf {
 constexpr int kMaxGrid = 4096;
 
 // Most bytes of one batch's strip pixel lists (256 orientations of the
-// 491-column grid take 2.3 GB, two such sets at once; wide grids sweep fewer
+// 491-column grid take 1.2 GB, two such sets at once; wide grids sweep fewer
 // orientations per batch, and so does a device that cannot hold them).
 constexpr size_t kListBytes = size_t(6) << 30;
 
@@ -347,7 +347,7 @@ struct Engine {
   int batch = 256;
   int force_h = 0;        // test hook: strip height override
   int force_safe = 0;     // test hook: run every orientation in safe mode
-  int normal_smem = 0;    // shared-memory budget of a normal strip CTA (0 = four CTAs per SM)
+  int normal_smem = 0;    // shared-memory budget of a normal strip CTA (0 = six CTAs per SM)
   int export_pixels = 1;  // rebuild the best orientation's pixels and vm_info (TomoSh_CUDA tail)
   int adaptive = 1;       // raise the entry budget after overflowing early batches (full sweeps)
   int fold_lim = 32767;   // largest |column value| of a packed fold record (TOMO_OPT_FOLD_LIMIT)
@@ -398,7 +398,7 @@ struct Engine {
 
   // Strip configurations.
   //   0 normal     : H0-column strips whose columns k_columns resolves from
-  //                  k_raster's pixel lists, four CTAs per SM; H0 is the
+  //                  k_raster's pixel lists, six CTAs per SM; H0 is the
   //                  tallest strip with room for two pixels per slot;
   //   1 safe       : strips that rasterize their own triangles, whole-box
   //                  evaluation, priorities, all opt-in shared memory;
@@ -418,13 +418,13 @@ struct Engine {
     const size_t budget1 = std::min<size_t>(optin, 227 * 1024) - 2048;
     const size_t shared = strip_default_budget();
     // Pixels of an h-column normal strip.  By default what the shared memory of
-    // four CTAs per SM holds (k_columns needs its 64 registers); a budget given by
+    // six CTAs per SM holds; a budget given by
     // TOMO_OPT_NORMAL_SMEM (or a later one of adapt_after) buys 6 bytes per
     // pixel beside four bytes and a bit per slot and a 20 KB work area.
     auto pixels = [&](int h, size_t budget) -> int {
       const size_t HG = (size_t)h * G;
       const size_t fixed = budget ? 4 * HG + HG / 8 + 32 + std::max<size_t>(20816, 6 * HG + 2048) : strip_smem_bytes(0, h, G, 0);
-      const size_t all = budget ? std::min(optin - 2048, budget) : (shared ? shared : 55296), per = budget ? 6 : 4;
+      const size_t all = budget ? std::min(optin - 2048, budget) : (shared ? shared : 37888), per = budget ? 6 : 4;
       if (all < fixed + 32 * per) return 16;
       const size_t most = (budget1 - strip_smem_bytes(0, h, G, 0)) / 4 - 16;
       return (int)std::min<size_t>(std::min<size_t>((all - fixed) / per - 16, most), 32767);
@@ -1048,7 +1048,7 @@ struct Engine {
   // sweep of the sample, re-runs included: the configuration-0 strips, then
   // the ladder that re-runs what they flagged (Engine::resolve), so a budget
   // too small for the mesh pays for its overflows.  Candidates: 128 or 256
-  // orientations per batch x the normal strip budget (four CTAs per SM, 72 KB,
+  // orientations per batch x the normal strip budget (six CTAs per SM, 72 KB,
   // 99 KB) x the strip height (the planned one and half of it).  When most of
   // the sample passes the 63-pixel cap in some column, every candidate starts
   // in the priority-carrying strips (configuration 4), as an adaptive sweep
@@ -1056,7 +1056,7 @@ struct Engine {
   int autotune(int sample, TuneResult* best)
   {
     static const int kBatches[] = {128, 256};
-    static const int kSmem[] = {0, 73728, 101376};   // 0: four CTAs per SM
+    static const int kSmem[] = {0, 73728, 101376};   // 0: six CTAs per SM
     best->batch = batch; best->normal_smem = normal_smem; best->strip_h = force_h; best->start_cfg = start_cfg;
     best->us_per_orientation = 0.0;
     if (nYPR == 0 || P.n_tri == 0) return 0;

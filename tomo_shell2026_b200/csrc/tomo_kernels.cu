@@ -1665,15 +1665,17 @@ __global__ void __launch_bounds__(256, 1) k_strip(EngineParams p)
 // latency between its barriers.  Per 256 orientations of the 82k solid: 1,060 us
 // with linked lists per column, a thread per column of up to 11 pixels and a
 // serial scan of longer ones; 545 with the counting sort and whole columns side
-// by side in a warp's lanes, ranked by shuffles and paired by ballots; 521 now.
-// The thin shell (seven pixels to a column) gains more: its 2-degree sweep took
-// 557, 220 and now 169 ms.  Sorting networks in registers for 4, 8 and 16 keys
+// by side in a warp's lanes, ranked by shuffles and paired by ballots; 502 with a
+// thread per column, at four CTAs of 256 threads per SM; 439 now, at six of 160
+// (five of 192: 467, seven of 128 on half the strip height: 538): fewer warps wait
+// at a barrier together.  The thin shell (seven pixels to a column) gains more:
+// its 2-degree sweep took 557, 220, 169 and now 157 ms.  Sorting networks in registers for 4, 8 and 16 keys
 // were slower than the insertion sort (555 with the first two, 669 with all): the
-// unrolled walks do not fit the instruction cache.  Five CTAs per SM with 48
-// registers spill: 548.  Other class limits (8 / 16, 6 / 12 / 20, 5 / 9, 3 / 6 /
+// unrolled walks do not fit the instruction cache.  Five CTAs of 256 threads need
+// 48 registers and spill: 548.  Other class limits (8 / 16, 6 / 12 / 20, 5 / 9, 3 / 6 /
 // 12) are within 1 %.
-constexpr int kColThreads = 256;
-constexpr int kColBlocks = 4;    // CTAs per SM
+constexpr int kColThreads = 160;
+constexpr int kColBlocks = 6;    // CTAs per SM
 constexpr int kLongKeys = 128;   // raw pixels of a column that a warp sorts in its scratch
 
 // Shared-memory bytes of one k_columns CTA.
@@ -1824,7 +1826,7 @@ __global__ void __launch_bounds__(kColThreads, kColBlocks) k_columns(EngineParam
   if (tid < 4) nq[tid] = 0;
   if (tid == 0) sflag = 0;
   const uint2* const ents = p.ents + ((size_t)o * p.S + s) * C;
-  constexpr int kHold = 8;               // pixels a thread keeps between the two passes
+  constexpr int kHold = 10;               // pixels a thread keeps between the two passes
   uint2 held[kHold];
 #pragma unroll
   for (int j = 0; j < kHold; j++)
@@ -2076,7 +2078,7 @@ __global__ void __launch_bounds__(kColThreads, kColBlocks) k_columns(EngineParam
   for (int cls = 0; cls < 4; cls++) {
     const int nc = nq[cls], chunks = (nc + 31) >> 5;
     const unsigned short* const qu = cls < 2 ? queue : queue2;
-    for (int ch = (wid - c0) & (kColThreads / 32 - 1); ch < chunks; ch += kColThreads / 32) {
+    for (int ch = (wid + kColThreads / 32 - c0) % (kColThreads / 32); ch < chunks; ch += kColThreads / 32) {
       const int at = ch * 32 + lane;
       int l = 0, ls = 0, beg = 0, cnt = 0;
       if (at < nc) {
@@ -2112,7 +2114,7 @@ __global__ void __launch_bounds__(kColThreads, kColBlocks) k_columns(EngineParam
                     __shfl_sync(full, cnt, from));
       }
     }
-    c0 = (c0 + chunks) & (kColThreads / 32 - 1);
+    c0 = (c0 + chunks) % (kColThreads / 32);
   }
 
   // ---- reductions
