@@ -290,8 +290,17 @@ __global__ void k_reset(EngineParams p)
 // One thread per vertex and kRotGroup orientations: the vertex is loaded
 // once and rotated by each orientation of the group (independent chains for
 // the scheduler), the group's matrices sit in shared memory, and the AABB
-// minima are reduced per warp, then per block, before one atomic each.
-constexpr int kRotGroup = 8;
+// minima are reduced per warp as ordered keys (one instruction a coordinate),
+// then per block, before one atomic each.  Every input is finite (upload
+// checks), so the order of keys is the order of values; of two zeros either
+// serves, since the minimum is only subtracted.
+//
+// 168 MB written per 256 orientations of the 82k solid: 51 us with five
+// shuffles a coordinate and eight orientations a thread, 35 with keys, 37 at four
+// and 34 at sixteen orientations.  Four it is: the 82k sweep is the same
+// (123.8, 123.7, 123.5 ms), the 5k solid's 10.74 ms against 11.01 and 11.01 (its few
+// blocks spread better beside the column kernel).
+constexpr int kRotGroup = 4;
 
 __global__ void __launch_bounds__(256) k_rotate(EngineParams p)
 {
@@ -310,6 +319,7 @@ __global__ void __launch_bounds__(256) k_rotate(EngineParams p)
   if (v < p.nV) { a = p.vpos[v]; n = p.vnrm[v]; }
   const float t0 = __fsub_rn(a.x, p.cx), t1 = __fsub_rn(a.y, p.cy), t2 = __fsub_rn(a.z, p.cz);
   const int lane = threadIdx.x & 31;
+  unsigned kx = 0, ky = 0, kz = 0;   // lane k: the warp's minima of orientation k
 #pragma unroll
   for (int k = 0; k < kRotGroup; k++) {
     if (k >= ng) break;   // block-uniform
@@ -323,16 +333,14 @@ __global__ void __launch_bounds__(256) k_rotate(EngineParams p)
     } else {
       x = y = z = 1e5f;   // STomoAABB3Df::Init
     }
-    for (int off = 16; off > 0; off >>= 1) {
-      x = fmin_ref(x, __shfl_xor_sync(0xFFFFFFFFu, x, off));
-      y = fmin_ref(y, __shfl_xor_sync(0xFFFFFFFFu, y, off));
-      z = fmin_ref(z, __shfl_xor_sync(0xFFFFFFFFu, z, off));
-    }
-    if (lane == 0) {
-      atomicMin(&kmin[k][0], f2key(x));
-      atomicMin(&kmin[k][1], f2key(y));
-      atomicMin(&kmin[k][2], f2key(z));
-    }
+    const unsigned mx = __reduce_min_sync(0xFFFFFFFFu, f2key(x)), my = __reduce_min_sync(0xFFFFFFFFu, f2key(y)),
+                   mz = __reduce_min_sync(0xFFFFFFFFu, f2key(z));
+    if (lane == k) { kx = mx; ky = my; kz = mz; }
+  }
+  if (lane < ng) {
+    atomicMin(&kmin[lane][0], kx);
+    atomicMin(&kmin[lane][1], ky);
+    atomicMin(&kmin[lane][2], kz);
   }
   __syncthreads();
   if (threadIdx.x < ng * 3) atomicMin(&p.minkey[(o0 + threadIdx.x / 3) * 4 + threadIdx.x % 3], kmin[threadIdx.x / 3][threadIdx.x % 3]);
