@@ -2215,6 +2215,7 @@ __global__ void __launch_bounds__(32 * kBedWarps) k_bed(EngineParams p)
   const int by0 = max(p.bbox[o * 4 + 1] - m, 0), by1 = min(p.bbox[o * 4 + 3] + m + 1, p.G);
   const int words = (by1 - by0 + 31) >> 5, runs = (bx1 - bx0 + kBedRun - 1) / kBedRun;
   const uint8_t* const bedf = p.bedf + (size_t)o * p.G * p.G;
+  const bool plain = p.bed_type == kBedBrim || p.bed_type == kBedRaft;   // an unknown type lays no bed
   const unsigned up_mask = r < 32 ? (1u << r) - 1u : 0u, down_mask = r < 32 ? full << (32 - r) : 0u;
   int cnt = 0;
   for (int u = blockIdx.x * kBedWarps + wid; u < words * runs; u += gridDim.x * kBedWarps) {
@@ -2269,7 +2270,7 @@ __global__ void __launch_bounds__(32 * kBedWarps) k_bed(EngineParams p)
           if (d != kBedFar) best = min(best, dx * dx + d * d);
         }
         const float md = best < INT_MAX ? __fsqrt_rn((float)best) : 1e5f;
-        const bool near = md <= p.bed_outer && (p.bed_type != kBedSkirt || md > p.bed_inner);
+        const bool near = md <= p.bed_outer && (plain || (p.bed_type == kBedSkirt && md > p.bed_inner));
         cnt += open && near;
       }
     }
