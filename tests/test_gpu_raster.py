@@ -47,3 +47,16 @@ def test_raster_splits(oracle, kind, n_ypr):
     for k in ("Mo", "Mss", "Vtc"):
         assert np.array_equal(getattr(got, k).view(np.int32), np.asarray(want[k], np.float32).view(np.int32)), k
     assert got.optID == want["optID"]
+
+
+@pytest.mark.parametrize("dvoxel", [14.0, 300.0, 1.0e7, 1.0e10, -1.0e10])
+def test_raster_at_any_pixel_size(oracle, dvoxel):
+    """Pixel centres far outside the triangles: the cells stay those of the pixel
+    box and the triangles fall back to their centroids."""
+    m = _mesh("cube_and_sphere")
+    ypr = np.random.default_rng(3).uniform(0.0, 2.0 * np.pi, (5, 3)).astype(np.float32)
+    opts = PrintOptions(dVoxel=dvoxel)
+    got, want = native.sweep(m, ypr, opts), oracle.sweep(m, ypr, opts)
+    for k in ("Vo64", "Vss64", "Vtc64"):
+        assert np.array_equal(getattr(got, k), want[k]), k
+    assert np.array_equal(got.entries, want["entries"]) and got.optID == want["optID"]

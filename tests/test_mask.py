@@ -27,3 +27,16 @@ def test_masks_hold_every_accepted_pixel(tmp_path, seed):
     accepted, cand, box = int(m["accepted"]), int(m["candidates"]), int(m["pixels"])
     # the masks hold every accepted pixel and little else
     assert 0 < accepted <= cand < 0.5 * box
+
+
+@pytest.mark.skipif(shutil.which("g++") is None, reason="needs g++")
+def test_masks_at_any_pixel_size(tmp_path):
+    """tests/mask_range_check.cpp: the masks' cell grid stays within the pixel box
+    and holds every accepted pixel, for pixel sizes up to the largest float."""
+    exe = tmp_path / "mask_range_check"
+    subprocess.run(["g++", "-O2", "-std=c++17", "-ffp-contract=off", "-fno-fast-math", "-fwrapv",
+                    str(HERE / "mask_range_check.cpp"), "-o", str(exe)], check=True)
+    out = subprocess.run([str(exe), "2000", "31"], capture_output=True, text=True)
+    m = dict(zip(*[iter(out.stdout.strip().splitlines()[-1].split())] * 2))
+    assert out.returncode == 0 and int(m["violations"]) == 0, out.stdout[-2000:]
+    assert int(m["cases"]) > 10000 and int(m["accepted"]) > 10000

@@ -191,12 +191,14 @@ struct MaskTri {
 
 constexpr int kCellX = 8, kCellY = 4;
 
+// Whole numbers at or above / below f, held at the ends of int (what the
+// device's conversion does).
 TOMO_HD int ceil_int(float f)
 {
 #ifdef __CUDA_ARCH__
   return __float2int_ru(f);
 #else
-  return (int)ceilf(f);
+  return f >= 2147483648.0f ? 2147483647 : (f <= -2147483648.0f ? -2147483647 - 1 : (int)ceilf(f));
 #endif
 }
 TOMO_HD int floor_int(float f)
@@ -204,7 +206,7 @@ TOMO_HD int floor_int(float f)
 #ifdef __CUDA_ARCH__
   return __float2int_rd(f);
 #else
-  return (int)floorf(f);
+  return f >= 2147483648.0f ? 2147483647 : (f <= -2147483648.0f ? -2147483647 - 1 : (int)floorf(f));
 #endif
 }
 
@@ -229,8 +231,11 @@ TOMO_HD MaskTri mask_setup(float ax, float ay, float e0x, float e0y, float e1x, 
   const float DL = (d00 + d11) * L, es = DL * ((L + (2.0f + ah)) * (3.0f / 262144.0f));
   const float e = fmaf(DL, m * (1.5f / 1048576.0f), es);
   const float c = 0.001f + half;
-  // a sliver's numerators are too uncertain: no tighter box than the pixel box
-  const float d = es <= 0.002f * ad ? fmaf(0.025f, L, fmaf(m, 1.0f / 524288.0f, 0.001f)) : 1.0e6f;
+  // A sliver's numerators are too uncertain: no tighter box than the pixel box,
+  // whatever the pixel size (|c| < 1.8e38).  Elsewhere |half| is below 175 L
+  // (|denom| is at most (D / 2)^2 and D at most 4 L^2), so that the counts below
+  // stay far within int.
+  const float d = es <= 0.002f * ad ? fmaf(0.025f, L, fmaf(m, 1.0f / 524288.0f, 0.001f)) : 3.0e38f;
   const float lo = d + c, hi = d - c;
   const int cx0 = ceil_int(minx - lo), cx1 = floor_int(maxx + hi);
   const int cy0 = ceil_int(miny - lo), cy1 = floor_int(maxy + hi);
