@@ -98,6 +98,8 @@ void tomoVolToMass(const float* f32info, const int* i32info, float* vm22);
                                    2 = the mean of the two */
 #define TOMO_OPT_FOLD_LIMIT 8   /* largest |column value| a packed 16-bit fold record holds (1..32767, default 32767);
                                    larger values go through the batch's escape table.  Lower only to test that table */
+#define TOMO_OPT_MEM_LIMIT 9    /* KiB of device memory the sweeps' buffers may hold (0 = what the device has): batches
+                                   shrink to fit, and a call whose single orientation does not fit is an error */
 int tomoSetOption(int key, int value);
 
 /* out[0..8] = grid edge, strip height, strips, entry capacity, orientations re-run

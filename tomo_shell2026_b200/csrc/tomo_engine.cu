@@ -170,6 +170,12 @@ float largest_float_not_above(double c)
   return f;
 }
 
+// Bytes of all DevBufs together, how many they may hold (TOMO_OPT_MEM_LIMIT;
+// 0: what the device has), and whether a request was refused since the flag was
+// last cleared.
+size_t g_dev_bytes = 0, g_dev_limit = 0;
+bool g_dev_refused = false;
+
 template <typename T>
 struct DevBuf {
   T* ptr = nullptr;
@@ -177,13 +183,25 @@ struct DevBuf {
   cudaError_t reserve(size_t count)
   {
     if (count <= n && ptr) return cudaSuccess;
-    if (ptr) cudaFree(ptr);
-    ptr = nullptr; n = 0;
-    cudaError_t e = cudaMalloc((void**)&ptr, sizeof(T) * (count ? count : 1));
-    if (e == cudaSuccess) n = count;
+    release();
+    const size_t bytes = sizeof(T) * (count ? count : 1);
+    // past the limit the device is asked for more than any has, so that the
+    // refusal is its own
+    const bool over = g_dev_limit && g_dev_bytes + bytes > g_dev_limit;
+    const cudaError_t e = cudaMalloc((void**)&ptr, over ? ~size_t(0) >> 1 : bytes);
+    if (e == cudaSuccess) { n = count; g_dev_bytes += bytes; return e; }
+    ptr = nullptr;
+    if (e == cudaErrorMemoryAllocation) {
+      g_dev_refused = true;
+      cudaGetLastError();   // the caller has the error: the next launch check must not find it again
+    }
     return e;
   }
-  void release() { if (ptr) cudaFree(ptr); ptr = nullptr; n = 0; }
+  void release()
+  {
+    if (ptr) { cudaFree(ptr); g_dev_bytes -= sizeof(T) * (n ? n : 1); }
+    ptr = nullptr; n = 0;
+  }
 };
 
 // Largest slot grid edge (columns of the rotated footprint at the voxel pitch).
@@ -609,13 +627,18 @@ struct Engine {
   }
 
   // reserve_batch for as many orientations as the device can hold: a batch is
-  // halved while its buffers do not fit.
+  // halved while its buffers do not fit.  A refusal that a smaller batch makes
+  // good is no error of the call.
   int reserve_fitting(int mode, int* Bo, int bin_cap, int want, int* nprep)
   {
     for (;;) {
+      const int code = g_last_error;
+      const std::string why = g_last_error_str;
+      g_dev_refused = false;
       *nprep = want > *Bo ? 2 : 1;
       const int rc = reserve_batch(mode, *Bo, bin_cap, *nprep);
-      if (rc == 0 || *Bo <= 1 || cudaGetLastError() != cudaErrorMemoryAllocation) return rc;
+      if (rc == 0 || *Bo <= 1 || !g_dev_refused) return rc;
+      g_last_error = code; g_last_error_str = why;
       *Bo = (*Bo + 1) / 2;
     }
   }
@@ -1206,7 +1229,7 @@ struct PinnedBuf {
     release();
     const size_t want = std::max<size_t>(bytes + bytes / 4, size_t(1) << 20);
     const cudaError_t e = cudaHostAlloc((void**)&ptr, want, cudaHostAllocDefault);
-    if (e == cudaSuccess) n = want; else ptr = nullptr;
+    if (e == cudaSuccess) n = want; else { ptr = nullptr; cudaGetLastError(); }
     return e;
   }
   void release() { if (ptr) cudaFreeHost(ptr); ptr = nullptr; n = 0; }
@@ -1375,6 +1398,7 @@ int tomoSetOption(int key, int value)
     case TOMO_OPT_ADAPTIVE: E.adaptive = value ? 1 : 0; E.adapt_smem = E.adapt_h = E.adapt_cfg = 0; return 0;
     case TOMO_OPT_PROPOSAL: if (value < 0 || value > 2) return TOMO_ERR_ARG; g_proposal = value; return 0;
     case TOMO_OPT_FOLD_LIMIT: if (value < 1 || value > 32767) return TOMO_ERR_ARG; E.fold_lim = value; return 0;
+    case TOMO_OPT_MEM_LIMIT: if (value < 0) return TOMO_ERR_ARG; g_dev_limit = (size_t)value << 10; return 0;
     default: return TOMO_ERR_ARG;
   }
 }

@@ -26,6 +26,7 @@ TOMO_OPT_BATCH, TOMO_OPT_STRIP_H, TOMO_OPT_FORCE_SAFE, TOMO_OPT_NORMAL_SMEM, TOM
 TOMO_OPT_ADAPTIVE = 6
 TOMO_OPT_PROPOSAL = 7
 TOMO_OPT_FOLD_LIMIT = 8
+TOMO_OPT_MEM_LIMIT = 9
 
 # (name, restype, argtypes) for every export of include/tomo_b200.h
 EXPORTS = [
