@@ -35,7 +35,7 @@ def test_shrunk_sweeps_match_and_leave_no_error():
     m = meshgen.perturbed_sphere(3000, 60.0, 8, with_hull=False)
     opts = PrintOptions(explicit_ss=False)
     ref = native.sweep(m, YPR, opts)
-    refused = 0
+    shrunk = refused = 0
     for kib in _limits():
         native.lib().OnDestroy()
         native.set_option(native.TOMO_OPT_MEM_LIMIT, kib)
@@ -45,8 +45,10 @@ def test_shrunk_sweeps_match_and_leave_no_error():
             refused += 1
             native.set_option(native.TOMO_OPT_MEM_LIMIT, 0)
             got = native.sweep(m, YPR, opts)   # nothing of the refusal is left
+        else:
+            shrunk += native.kernel_log()["k_raster"]["launches"] > 2 + 1   # two batches and the export
         assert native.lib().tomoGetLastError() == 0 and native.lib().tomoGetLastErrorString() == b"", kib
         for k in ("Mo", "Mss", "Vtc", "VoF", "VssF"):
             assert np.array_equal(bits(getattr(got, k)), bits(getattr(ref, k))), (kib, k)
         assert np.array_equal(got.Vss64, ref.Vss64) and got.optID == ref.optID
-    assert refused > 0
+    assert shrunk > 0 and refused > 0

@@ -288,10 +288,15 @@ struct Workspace {
     return 0;
   }
 
-  void release()
+  void release_batch()   // the buffers of reserve_batch
   {
     for (auto& q : prep) q.release();
     for (auto& s : set) { s.acc.release(); s.flags.release(); s.foldcnt.release(); s.foldp.release(); s.foldtc.release(); s.foldx.release(); s.foldxn.release(); s.foldmeta.release(); }
+  }
+
+  void release()
+  {
+    release_batch();
     dump_cols.release(); dump_keys.release(); dump_types.release();
     exp_bed.release(); exp_blocks.release(); exp_head.release(); exp_pix.release(); exp_sums.release();
     log.destroy();
@@ -627,8 +632,9 @@ struct Engine {
   }
 
   // reserve_batch for as many orientations as the device can hold: a batch is
-  // halved while its buffers do not fit.  A refusal that a smaller batch makes
-  // good is no error of the call.
+  // halved while its buffers do not fit, what the larger one had taken given back
+  // first (no launch that uses it is left: cudaFree waits for the device).  A
+  // refusal that a smaller batch makes good is no error of the call.
   int reserve_fitting(int mode, int* Bo, int bin_cap, int want, int* nprep)
   {
     for (;;) {
@@ -639,6 +645,7 @@ struct Engine {
       const int rc = reserve_batch(mode, *Bo, bin_cap, *nprep);
       if (rc == 0 || *Bo <= 1 || !g_dev_refused) return rc;
       g_last_error = code; g_last_error_str = why;
+      W.release_batch();
       *Bo = (*Bo + 1) / 2;
     }
   }
