@@ -2044,19 +2044,29 @@ struct MultiEngine {
     return v;
   }
 
-  // Every buffer the sweep touches, at its final size, before capture.
+  // Every buffer the sweep touches, at its final size, before capture.  The
+  // meshes share one workspace, and a batch that has to shrink gives back what
+  // the meshes before it had reserved: the pass is repeated until none shrinks
+  // (buffers only grow in such a pass, so that every mesh's are in place then).
   int reserve_all()
   {
-    for (auto* e : meshes) {
-      if (e->nYPR == 0 || e->P.n_tri == 0) continue;
-      const int c = e->start_cfg == 4 ? 4 : 0, mode = e->cfg[c].mode;   // as sweep_batches starts
-      e->choose_strips(c);
-      TOMO_TRY(e->configure());
-      TOMO_TRY(e->reserve_outputs());
-      const int ask = std::min(e->batch, e->nYPR);
-      int Bo = e->batch_size(ask, mode), sets = 1;
-      TOMO_TRY(e->reserve_fitting(mode, &Bo, 4 * e->P.n_tri + 4096, e->nYPR, &sets));
-      if (Bo < ask) e->batch = Bo;   // the capture must find every buffer in place
+    for (bool again = true; again;) {
+      again = false;
+      for (auto* e : meshes) {
+        if (e->nYPR == 0 || e->P.n_tri == 0) continue;
+        const int c = e->start_cfg == 4 ? 4 : 0, mode = e->cfg[c].mode;   // as sweep_batches starts
+        e->choose_strips(c);
+        TOMO_TRY(e->configure());
+        TOMO_TRY(e->reserve_outputs());
+        const int ask = std::min(e->batch, e->nYPR), most = e->batch_size(ask, mode);
+        int Bo = most, sets = 1;
+        TOMO_TRY(e->reserve_fitting(mode, &Bo, 4 * e->P.n_tri + 4096, e->nYPR, &sets));
+        if (Bo < ask && e->batch != Bo) {   // the capture must find every buffer in place
+          e->batch = Bo;
+          clear_graph();
+        }
+        again = again || Bo < most;
+      }
     }
     return 0;
   }
