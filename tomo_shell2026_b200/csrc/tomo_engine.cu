@@ -30,7 +30,8 @@
 namespace tomo {
 
 size_t strip_smem_bytes(int mode, int H, int G, int ent_cap);
-size_t strip_default_budget();
+int strip_ctas();
+size_t strip_budget(int ctas);
 int raster_lanes_log2(int nT, int Bo);
 cudaError_t configure_kernels(size_t normal_smem, size_t safe_smem, size_t prio_smem);
 cudaError_t launch_batch(const EngineParams& p, cudaStream_t main, size_t strip_smem, LaunchLog* L);
@@ -434,29 +435,53 @@ struct Engine {
   struct StripCfg { int H, S, C; size_t smem; int mode; };
   StripCfg cfg[5];
 
+  // Dynamic shared memory of a strip CTA that has its SM to itself (the strip
+  // kernels also hold ~0.7 KB of static shared memory).
+  size_t whole_sm() const { return std::min<size_t>(smem_optin ? smem_optin : 232448, 227 * 1024) - 2048; }
+
+  // Pixels of an h-column normal strip at `ctas` CTAs per SM.
+  int strip_pixels(int h, int ctas) const
+  {
+    const size_t fixed = strip_smem_bytes(0, h, G, 0), share = strip_budget(ctas);
+    const size_t all = std::min(whole_sm(), share ? share : 233472 / (size_t)ctas - 1536);
+    return all < fixed + 32 * 4 ? 16 : (int)std::min<size_t>((all - fixed) / 4 - 16, 32767);
+  }
+
+  // The most CTAs per SM that leave it room for two pixels per slot (one if none does).
+  int strip_ctas_for(int h) const
+  {
+    int k = strip_ctas();
+    while (k > 1 && strip_pixels(h, k) < 2 * h * G) k--;
+    return k;
+  }
+
+  // Pixels of an h-column normal strip under an explicit budget
+  // (TOMO_OPT_NORMAL_SMEM, or a later one of adapt_after): 6 bytes a pixel beside
+  // four bytes and a bit per slot and a 20 KB work area, as the option is documented.
+  int budget_pixels(int h, size_t budget) const
+  {
+    const size_t HG = (size_t)h * G, fixed = 4 * HG + HG / 8 + 32 + std::max<size_t>(20816, 6 * HG + 2048);
+    const size_t all = std::min((smem_optin ? smem_optin : 232448) - 2048, budget);
+    if (all < fixed + 32 * 6) return 16;
+    const size_t most = (whole_sm() - strip_smem_bytes(0, h, G, 0)) / 4 - 16;
+    return (int)std::min<size_t>(std::min<size_t>((all - fixed) / 6 - 16, most), 32767);
+  }
+
   void plan_strips()
   {
-    const size_t optin = smem_optin ? smem_optin : 232448;
-    // the strip kernels also hold ~0.7 KB of static shared memory
-    const size_t budget1 = std::min<size_t>(optin, 227 * 1024) - 2048;
-    const size_t shared = strip_default_budget();
-    // Pixels of an h-column normal strip.  By default what the shared memory of
-    // six CTAs per SM holds; a budget given by
-    // TOMO_OPT_NORMAL_SMEM (or a later one of adapt_after) buys 6 bytes per
-    // pixel beside four bytes and a bit per slot and a 20 KB work area.
-    auto pixels = [&](int h, size_t budget) -> int {
-      const size_t HG = (size_t)h * G;
-      const size_t fixed = budget ? 4 * HG + HG / 8 + 32 + std::max<size_t>(20816, 6 * HG + 2048) : strip_smem_bytes(0, h, G, 0);
-      const size_t all = budget ? std::min(optin - 2048, budget) : (shared ? shared : 37888), per = budget ? 6 : 4;
-      if (all < fixed + 32 * per) return 16;
-      const size_t most = (budget1 - strip_smem_bytes(0, h, G, 0)) / 4 - 16;
-      return (int)std::min<size_t>(std::min<size_t>((all - fixed) / per - 16, most), 32767);
+    const size_t budget1 = whole_sm();
+    const size_t budget = (size_t)normal_smem;
+    // by default six CTAs per SM; a height the caller forces takes as many as hold
+    // it, where the priority strips hold two pixels per slot too (H * G up to 5,900)
+    auto pixels = [&](int h) {
+      return budget ? budget_pixels(h, budget) : strip_pixels(h, force_h == h ? strip_ctas_for(h) : strip_ctas());
     };
     int h0 = 1;
     for (int h : {8, 4, 2, 1}) {
       if (force_h && h != force_h) continue;
       if (strip_smem_bytes(0, h, G, 256) > budget1) continue;
-      const int cap = pixels(h, (size_t)normal_smem);
+      if (force_h && !budget && strip_smem_bytes(2, h, G, 2 * h * G) > budget1) continue;
+      const int cap = pixels(h);
       if (cap < 256) continue;
       if (force_h || cap >= 2 * h * G) { h0 = h; break; }
     }
@@ -471,7 +496,7 @@ struct Engine {
       c.smem = strip_smem_bytes(mode, h, G, c.C);
       return c;
     };
-    cfg[0] = make(0, h0, pixels(h0, (size_t)normal_smem));
+    cfg[0] = make(0, h0, pixels(h0));
     cfg[1] = make(1, h0, 0);
     cfg[2] = make(0, h0, (int)std::min<size_t>((budget1 - strip_smem_bytes(0, h0, G, 0)) / 4 - 16, 32767));
     cfg[3] = make(1, 1, 0);

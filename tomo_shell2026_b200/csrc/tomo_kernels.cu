@@ -2565,22 +2565,25 @@ __global__ void __launch_bounds__(kExportThreads) k_export_write(EngineParams p,
 
 namespace tomo {
 
-// Largest dynamic shared-memory budget that keeps kColBlocks k_columns CTAs
-// resident per SM (its registers are bounded for as many), or 0.
-size_t strip_default_budget()
+// Most k_columns CTAs an SM takes (its registers are bounded for as many).
+int strip_ctas() { return kColBlocks; }
+
+// Largest dynamic shared-memory budget that keeps `ctas` k_columns CTAs resident
+// per SM, or 0.
+size_t strip_budget(int ctas)
 {
-  static size_t cache[64];
+  static size_t cache[64][kColBlocks + 1];
   int dev = 0, per_sm = 0, reserved = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
-  if (cache[dev]) return cache[dev];
+  if (ctas < 1 || ctas > kColBlocks || cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
+  if (cache[dev][ctas]) return cache[dev][ctas];
   cudaFuncAttributes fa;
   if (cudaDeviceGetAttribute(&per_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev) != cudaSuccess ||
       cudaDeviceGetAttribute(&reserved, cudaDevAttrReservedSharedMemoryPerBlock, dev) != cudaSuccess ||
       cudaFuncGetAttributes(&fa, k_columns) != cudaSuccess)
     return 0;
-  const long long per_cta = per_sm / kColBlocks / 128 * 128 - reserved - (long long)fa.sharedSizeBytes;
-  cache[dev] = per_cta > 0 ? (size_t)per_cta / 128 * 128 : 0;
-  return cache[dev];
+  const long long per_cta = per_sm / ctas / 128 * 128 - reserved - (long long)fa.sharedSizeBytes;
+  cache[dev][ctas] = per_cta > 0 ? (size_t)per_cta / 128 * 128 : 0;
+  return cache[dev][ctas];
 }
 
 size_t strip_smem_bytes(int mode, int H, int G, int ent_cap)
