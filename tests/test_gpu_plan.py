@@ -1,4 +1,4 @@
-"""Strip plans (Engine::plan_strips): the height a caller forces is the
+"""Strip plans (Engine::plan_strips, adapt_after): the height a caller forces is the
 height that runs, and results never depend on the plan."""
 from __future__ import annotations
 
@@ -19,6 +19,15 @@ def default_options():
         native.set_option(key, value)
 
 
+def plates(n, a=200.0, b=140.0, gap=3.0):
+    """n thin plates above one another: 2 n pixels in every column."""
+    box = np.array([(0, 2, 1), (0, 3, 2), (4, 5, 6), (4, 6, 7), (0, 1, 5), (0, 5, 4), (1, 2, 6), (1, 6, 5), (2, 3, 7),
+                    (2, 7, 6), (3, 0, 4), (3, 4, 7)])
+    v = [(x, y, gap * k + z) for k in range(n) for z in (0.0, 1.0) for x, y in ((0, 0), (a, 0), (a, b), (0, b))]
+    return meshgen.mesh_from_arrays(np.array(v, float), np.vstack([box + 8 * k for k in range(n)]), "plates",
+                                    with_hull=False)
+
+
 def _same(got, ref):
     for k in ("Mo", "Mss", "Vtc", "VoF", "VssF"):
         assert np.array_equal(bits(getattr(got, k)), bits(getattr(ref, k))), k
@@ -37,3 +46,17 @@ def test_forced_height_runs(h, scale):
     assert h * st["grid"] <= 5900
     assert st["strip_h"] == h and st["overflow_reruns"] == 0
     _same(got, ref)
+
+
+@pytest.mark.parametrize("h", [2, 8])
+def test_adaptation_keeps_a_forced_height(h):
+    m = plates(7)
+    ypr = np.ascontiguousarray(meshgen.ypr_grid(np.arange(0, 20, 0.25), [0.0, 3.0]))   # 160
+    ref = native.sweep(m, ypr, PrintOptions())
+    native.set_option(native.TOMO_OPT_STRIP_H, h)
+    native.set_option(native.TOMO_OPT_BATCH, 32)
+    s = native.Session(m, ypr, PrintOptions())
+    for _ in range(2):   # the second sweep starts where the first adapted to
+        s.run_device()
+        assert native.stats()["strip_h"] == h
+        assert np.array_equal(bits(s.finish()[2]), bits(ref.Mss))

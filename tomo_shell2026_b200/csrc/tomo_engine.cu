@@ -711,7 +711,7 @@ struct Engine {
     const int user_smem = normal_smem, user_h = force_h;
     const bool adapt = adaptive && !ids;
     if (adapt && adapt_h) { normal_smem = adapt_smem; force_h = adapt_h; plan_strips(); }
-    const int rc = sweep_batches(ids, n, adapt);
+    const int rc = sweep_batches(ids, n, adapt, user_h != 0);
     if (adapt && (normal_smem != user_smem || force_h != user_h)) {
       normal_smem = user_smem; force_h = user_h; plan_strips();
     }
@@ -721,18 +721,19 @@ struct Engine {
   // After an early batch: if more than a fifth of its orientations overflowed
   // their strip lists, the rest of the sweep gets strips of half the height at
   // the same occupancy (twice the pixels per column of the strip) or, past
-  // one-column strips, the next larger budget (one host wait per check; the
-  // overflowed orientations are re-run by the ladder as usual).  Returns true
-  // when the configuration changed.
+  // one-column strips or at a height the caller forced, the next larger budget
+  // (one host wait per check; the overflowed orientations are re-run by the
+  // ladder as usual).  Sets *changed when the configuration did.
   // A batch where most orientations passed the 63-pixel cap in some column
   // switches the rest of the sweep to the priority-carrying strips
   // (configuration 4), which resolve those columns in one pass.
-  int adapt_after(int first, int nb, int* c, bool* changed)
+  int adapt_after(int first, int nb, bool keep_h, int* c, bool* changed)
   {
     *changed = false;
     static const int kBudgets[] = {73728, 101376, 150528, 232448};
     int next = -1;
-    if (*c == 0 && H == 1) {
+    const bool halve = H > 1 && !keep_h;
+    if (*c == 0 && !halve) {
       for (int b : kBudgets)
         if (b > normal_smem && next < 0) next = b;
     }
@@ -745,9 +746,9 @@ struct Engine {
     if (cap * 2 > nb) {
       *c = 4;
       adapt_cfg = 4;
-    } else if ((H > 1 || next >= 0) && over * 5 > nb) {
-      force_h = std::max(H / 2, 1);
-      if (H == 1) normal_smem = next;
+    } else if ((halve || next >= 0) && over * 5 > nb) {
+      force_h = halve ? H / 2 : H;
+      if (!halve) normal_smem = next;
       plan_strips();
       adapt_smem = normal_smem; adapt_h = force_h;
     } else {
@@ -759,7 +760,7 @@ struct Engine {
     return 0;
   }
 
-  int sweep_batches(const int* ids, int n, bool adapt)
+  int sweep_batches(const int* ids, int n, bool adapt, bool keep_h)
   {
     int c = (start_cfg == 4 || (adapt && adapt_cfg == 4)) ? 4 : 0;
     choose_strips(c);
@@ -806,7 +807,7 @@ struct Engine {
       TOMO_CUDA(cudaEventRecord(set[which].folded, side));
       if (adapt && k < 3 && first + nb < n) {
         bool changed = false;
-        TOMO_TRY(adapt_after(first, nb, &c, &changed));
+        TOMO_TRY(adapt_after(first, nb, keep_h, &c, &changed));
         if (changed) {
           // every launch so far has finished (adapt_after waited), so the
           // lists may move; the rest of the sweep may need smaller batches
