@@ -60,3 +60,16 @@ def test_adaptation_keeps_a_forced_height(h):
         s.run_device()
         assert native.stats()["strip_h"] == h
         assert np.array_equal(bits(s.finish()[2]), bits(ref.Mss))
+
+
+@pytest.mark.parametrize("radius", [1160.0, 1500.0])
+def test_wide_grids_hold_a_solid(radius):
+    """One-column strips of a grid far wider than the reference's: a part that fills
+    it is not run twice."""
+    m = meshgen.perturbed_icosphere(4, radius, 5, with_hull=False)
+    ypr = meshgen.ypr_grid([0.0, 50.0], [0.0, 40.0])
+    got = native.sweep(m, ypr, PrintOptions())
+    st = native.stats()
+    assert st["grid"] > 2500 and st["strip_h"] == 1 and st["overflow_reruns"] == 0
+    native.set_option(native.TOMO_OPT_NORMAL_SMEM, 150528)
+    _same(got, native.sweep(m, ypr, PrintOptions()))

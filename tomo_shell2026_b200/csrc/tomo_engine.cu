@@ -434,6 +434,7 @@ struct Engine {
   //                  for orientations where a column passed the 63-pixel cap.
   struct StripCfg { int H, S, C; size_t smem; int mode; };
   StripCfg cfg[5];
+  bool wide = false;   // configuration 0: one-column strips of a wide grid (plan_strips)
 
   // Dynamic shared memory of a strip CTA that has its SM to itself (the strip
   // kernels also hold ~0.7 KB of static shared memory).
@@ -447,11 +448,11 @@ struct Engine {
     return all < fixed + 32 * 4 ? 16 : (int)std::min<size_t>((all - fixed) / 4 - 16, 32767);
   }
 
-  // The most CTAs per SM that leave it room for two pixels per slot (one if none does).
-  int strip_ctas_for(int h) const
+  // The most CTAs per SM that leave it room for `px` pixels (one if none does).
+  int strip_ctas_for(int h, int px) const
   {
     int k = strip_ctas();
-    while (k > 1 && strip_pixels(h, k) < 2 * h * G) k--;
+    while (k > 1 && strip_pixels(h, k) < px) k--;
     return k;
   }
 
@@ -471,10 +472,20 @@ struct Engine {
   {
     const size_t budget1 = whole_sm();
     const size_t budget = (size_t)normal_smem;
-    // by default six CTAs per SM; a height the caller forces takes as many as hold
-    // it, where the priority strips hold two pixels per slot too (H * G up to 5,900)
+    // By default six CTAs per SM.  A height the caller forces takes fewer where it
+    // must, to have room for two pixels per slot (and so that the priority strips
+    // have it too: H * G up to 5,900).  One-column strips, below which there is no
+    // shorter strip to turn to, get room for three (from about 1,700 columns on):
+    // solids that fill a grid of 2,600 to 3,300 columns have 2.0 to 2.8, and with
+    // six CTAs, 1.4 down to 0.5, all their orientations ran twice (96 of a sphere on
+    // 2,577 columns: 587 ms, now 283; on 3,463: 1,314 and 641).
+    bool wide_now = false;
     auto pixels = [&](int h) {
-      return budget ? budget_pixels(h, budget) : strip_pixels(h, force_h == h ? strip_ctas_for(h) : strip_ctas());
+      if (budget) return budget_pixels(h, budget);
+      if (h > 1) return strip_pixels(h, force_h ? strip_ctas_for(h, 2 * h * G) : strip_ctas());
+      const int k = strip_ctas_for(1, 3 * G), px = strip_pixels(1, k);
+      wide_now = k < strip_ctas();
+      return wide_now ? std::min(px, 3 * G) : px;
     };
     int h0 = 1;
     for (int h : {8, 4, 2, 1}) {
@@ -497,6 +508,7 @@ struct Engine {
       return c;
     };
     cfg[0] = make(0, h0, pixels(h0));
+    wide = h0 == 1 && wide_now;
     cfg[1] = make(1, h0, 0);
     cfg[2] = make(0, h0, (int)std::min<size_t>((budget1 - strip_smem_bytes(0, h0, G, 0)) / 4 - 16, 32767));
     cfg[3] = make(1, 1, 0);
@@ -615,12 +627,16 @@ struct Engine {
   }
 
   // Orientations per batch: `want`, or fewer where the strips' pixel lists
-  // (normal strips, the current configuration) would pass kListBytes.
+  // (normal strips, the current configuration) would pass kListBytes (twice that
+  // on wide grids, where a batch's fold takes 20 ms and more for however few
+  // orientations: a search over 120 of a sphere on 2,133 columns takes 113 ms at
+  // 110 a batch and 180 at 38).
   int batch_size(int want, int mode) const
   {
     if (mode != 0) return want;
     const size_t per = (size_t)S * ent_cap * sizeof(uint2);
-    return (int)std::min<size_t>(want, std::max<size_t>(1, kListBytes / std::max<size_t>(per, 1)));
+    const size_t most = wide && ent_cap == cfg[0].C ? 2 * kListBytes : kListBytes;
+    return (int)std::min<size_t>(want, std::max<size_t>(1, most / std::max<size_t>(per, 1)));
   }
 
   // Buffers of a batch of Bo orientations in the current strip configuration.
