@@ -73,3 +73,16 @@ def test_wide_grids_hold_a_solid(radius):
     assert st["grid"] > 2500 and st["strip_h"] == 1 and st["overflow_reruns"] == 0
     native.set_option(native.TOMO_OPT_NORMAL_SMEM, 150528)
     _same(got, native.sweep(m, ypr, PrintOptions()))
+
+
+def test_adaptation_steps_are_worth_a_check():
+    """One-column strips that hold a few pixels too few: the first check of the sweep
+    already gets the rest of it through (up to the next budget's own room)."""
+    m = plates(22, 140.0, 200.0)   # 8,800 pixels and more in a column of the grid
+    ypr = np.ascontiguousarray(meshgen.ypr_grid(np.arange(0, 10, 0.25), [0.0, 1.0, 2.0]))   # 120
+    ref = native.sweep(m, ypr, PrintOptions())
+    native.set_option(native.TOMO_OPT_STRIP_H, 1)
+    native.set_option(native.TOMO_OPT_BATCH, 30)
+    got = native.sweep(m, ypr, PrintOptions())
+    assert 0 < native.stats()["overflow_reruns"] <= 30
+    _same(got, ref)

@@ -750,8 +750,11 @@ struct Engine {
     int next = -1;
     const bool halve = H > 1 && !keep_h;
     if (*c == 0 && !halve) {
+      // the first budget that buys half as much room again (at the smallest,
+      // one-column strips of the 256 grid gain 4 % over the default), else the largest
       for (int b : kBudgets)
-        if (b > normal_smem && next < 0) next = b;
+        if (2 * budget_pixels(H, b) >= 3 * ent_cap && next < 0) next = b;
+      if (next < 0 && budget_pixels(H, kBudgets[3]) > ent_cap) next = kBudgets[3];
     }
     if (*c != 0) return 0;
     std::vector<int> fl(nb);
