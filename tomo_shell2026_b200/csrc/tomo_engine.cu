@@ -1631,9 +1631,9 @@ constexpr size_t kStaticArenaBytes = size_t(32) << 20;  // 32 MiB of device scra
 constexpr size_t kStaticListBytes = size_t(16) << 20;   // of which the strips' pixel lists
 constexpr int kStaticMaxTri = 16384;
 constexpr int kStaticMaxVtx = 16384;
-// Orientations per batch at most (fewer for the largest meshes).  A batch is a
-// chain of launches and one wait, so it costs the same for 4 orientations as for
-// 16: the 5k solid's 684 orientations took 17.6 ms four at a time.
+// Orientations per batch.  A batch is a chain of launches and one wait, so it
+// costs the same for 4 orientations as for 16: the 5k solid's 684 orientations
+// took 17.6 ms four at a time.
 constexpr int kStaticBatch = 16;
 constexpr int kStaticGrid = 256;                        // the reference's slot grid
 constexpr int kStaticMaxDevices = 64;
@@ -1644,12 +1644,12 @@ namespace {
 
 constexpr size_t static_round(size_t b) { return (b + 255) & ~size_t(255); }
 
-// Bytes of the arena layout below for nV vertices, nT triangles and batches of
-// B orientations.  The triangle bins serve the re-runs of single orientations
-// only; safe mode may use more of them than a batch slot's worth.
-constexpr size_t static_bytes(size_t nV, size_t nT, size_t B)
+// Bytes of the arena layout below for nV vertices and nT triangles.  The
+// triangle bins serve the re-runs of single orientations only; safe mode may use
+// more of them than a batch slot's worth.
+constexpr size_t static_bytes(size_t nV, size_t nT)
 {
-  const size_t GG = (size_t)kStaticGrid * kStaticGrid, S = kStaticGrid;  // S bound: 1-column strips
+  const size_t B = kStaticBatch, GG = (size_t)kStaticGrid * kStaticGrid, S = kStaticGrid;  // S bound: 1-column strips
   return static_round(16 * nV) * 2 + static_round(16 * nT) + static_round(4 * 9 * B) + static_round(4 * B) +
          static_round(16 * B * nV) + static_round(4 * 4 * B) + static_round(4 * nT) +
          static_round(4 * (S + 1)) + static_round(4 * S) + static_round(4 * 4 * (4 * nT + 4096)) +
@@ -1658,16 +1658,8 @@ constexpr size_t static_bytes(size_t nV, size_t nT, size_t B)
          static_round(4 * B * S) + static_round(4 * B * GG) + static_round(2 * B * GG) + static_round(sizeof(FoldEscape) * kFoldEscapes) +
          static_round(4) + static_round(4 * B * S * 8) + 5 * static_round(8 * B) + static_round(5 * 4 * B);
 }
-static_assert(static_bytes(kStaticMaxVtx, kStaticMaxTri, 8) <= kStaticArenaBytes,
+static_assert(static_bytes(kStaticMaxVtx, kStaticMaxTri) <= kStaticArenaBytes,
               "the static scratch must hold the largest accepted mesh");
-
-// Orientations per batch for a mesh.
-int static_batch(int nV, int nT)
-{
-  int B = kStaticBatch;
-  while (B > 1 && static_bytes((size_t)nV, (size_t)nT, (size_t)B) > kStaticArenaBytes) B--;
-  return B;
-}
 
 struct StaticLayout {
   float4 *vpos, *vnrm, *xf;
@@ -1687,9 +1679,9 @@ struct StaticLayout {
 };
 
 // Same order and sizes as static_bytes().
-StaticLayout static_layout(unsigned char* base, int nV, int nT, int nB)
+StaticLayout static_layout(unsigned char* base, int nV, int nT)
 {
-  const size_t B = nB, GG = (size_t)kStaticGrid * kStaticGrid, S = kStaticGrid;
+  const size_t B = kStaticBatch, GG = (size_t)kStaticGrid * kStaticGrid, S = kStaticGrid;
   size_t off = 0;
   auto take = [&](size_t bytes) { unsigned char* q = base + off; off += static_round(bytes); return (void*)q; };
   StaticLayout L;
@@ -1884,8 +1876,8 @@ extern "C" int tomoSweepStatic(const float* f32info, const int* i32info, const f
   StreamDrain drain{st};   // declared after the lock: runs before it is released
   void* base = nullptr;
   TOMO_TRY(static_arena(&base));
-  const int B = static_batch(P.n_vtx, P.n_tri);
-  const StaticLayout L = static_layout((unsigned char*)base, P.n_vtx, P.n_tri, B);
+  constexpr int B = kStaticBatch;
+  const StaticLayout L = static_layout((unsigned char*)base, P.n_vtx, P.n_tri);
   int dev = 0, optin = 0;
   TOMO_CUDA(cudaGetDevice(&dev));
   TOMO_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
