@@ -1628,7 +1628,9 @@ int tomoFinish(float* Mo, float* Mss, float* Vtc)
 namespace tomo {
 
 constexpr size_t kStaticArenaBytes = size_t(32) << 20;  // 32 MiB of device scratch per device
-constexpr size_t kStaticListBytes = size_t(16) << 20;   // of which the strips' pixel lists
+// Of which the strips' pixel lists: 4,608 pixels for each of the 32 eight-column
+// strips of sixteen orientations, as many as six CTAs per SM hold (4,588).
+constexpr size_t kStaticListBytes = size_t(18) << 20;
 constexpr int kStaticMaxTri = 16384;
 constexpr int kStaticMaxVtx = 16384;
 // Orientations per batch.  A batch is a chain of launches and one wait, so it
