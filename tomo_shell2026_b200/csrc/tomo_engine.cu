@@ -1652,7 +1652,7 @@ constexpr size_t static_round(size_t b) { return (b + 255) & ~size_t(255); }
 constexpr size_t static_bytes(size_t nV, size_t nT)
 {
   const size_t B = kStaticBatch, GG = (size_t)kStaticGrid * kStaticGrid, S = kStaticGrid;  // S bound: 1-column strips
-  return static_round(16 * nV) * 2 + static_round(16 * nT) + static_round(4 * 9 * B) + static_round(4 * B) +
+  return static_round(16 * nV) * 2 + static_round(16 * nT) + static_round(4 * 9 * B) + static_round(2 * 4 * B) +
          static_round(16 * B * nV) + static_round(4 * 4 * B) + static_round(4 * nT) +
          static_round(4 * (S + 1)) + static_round(4 * S) + static_round(4 * 4 * (4 * nT + 4096)) +
          static_round(4 * B * S) + static_round(kStaticListBytes) +
@@ -1691,7 +1691,7 @@ StaticLayout static_layout(unsigned char* base, int nV, int nT)
   L.vnrm = (float4*)take(16 * (size_t)nV);
   L.tri = (int4*)take(16 * (size_t)nT);
   L.rot = (float*)take(4 * 9 * B);
-  L.ori = (int*)take(4 * B);
+  L.ori = (int*)take(2 * 4 * B);   // the batch slots, then the slots of a re-run
   L.xf = (float4*)take(16 * B * nV);
   L.minkey = (unsigned*)take(4 * 4 * B);
   L.trange = (unsigned*)take(4 * (size_t)nT);
@@ -1725,6 +1725,7 @@ int4 g_static_htri[kStaticMaxTri];
 float g_static_hrot[kStaticBatch * 9];
 int g_static_hori[kStaticBatch] = {0, 1, 2, 3, 4, 5, 6, 7, 8, 9, 10, 11, 12, 13, 14, 15};
 int g_static_hout[5 * kStaticBatch];   // flags, bed pixels, Vo, Vss, Vtc (float bits)
+int g_static_hcnt[kStaticBatch * kStaticGrid];   // pixels of each slot's strips
 float g_static_bedfold[kStaticGrid * kStaticGrid + 1];
 void* g_static_addr[kStaticMaxDevices];
 static_assert(kStaticBatch == 16, "g_static_hori lists the batch slots");
@@ -1745,10 +1746,10 @@ int static_arena(void** out)
   return 0;
 }
 
-void static_bind(EngineParams& p, const StaticLayout& L, int nb, int slot, int bin_cap)
+void static_bind(EngineParams& p, const StaticLayout& L, int nb, const int* ori, int bin_cap)
 {
   p.vpos = L.vpos; p.vnrm = L.vnrm; p.tri = L.tri; p.rot = L.rot;
-  p.ori = L.ori + slot; p.Bo = nb;
+  p.ori = ori; p.Bo = nb;
   p.xf = L.xf; p.minkey = L.minkey; p.trange = L.trange;
   p.bin_off = L.bin_off; p.bin_cur = L.bin_cur; p.bins = L.bins; p.bin_cap = bin_cap;
   p.ents = L.ents; p.ent_cnt = L.ent_cnt; p.rast_shift = raster_lanes_log2(p.nT, nb);
@@ -1764,6 +1765,46 @@ void static_bind(EngineParams& p, const StaticLayout& L, int nb, int slot, int b
   p.dump_slot = -1; p.dump_cols = nullptr; p.dump_keys = nullptr; p.dump_types = nullptr;
 }
 
+// Batch slots whose strip lists overflowed re-run in configuration 2, as many at
+// a time as the lists hold (their strips' pixels were counted), with the shared
+// memory that takes; fl: the slots' flags, brought up to date.  One orientation
+// after the other -- a rasterizer launch of a few large triangles each time, which
+// is latency -- 22 of the 36 orientations of three 150 mm plates made the call 7.9
+// ms; it takes 2.3.
+int static_rerun_big(Engine& X, const StaticLayout& L, const int* slots, int n, int* fl, cudaStream_t st)
+{
+  X.choose_strips(2);
+  EngineParams p = X.base_params(X.cfg[2].mode);
+  p.variant = 2;
+  const int S = X.S;
+  int need[kStaticBatch] = {X.ent_cap};   // one alone takes all there is
+  if (n > 1) {
+    TOMO_CUDA(cudaMemcpyAsync(g_static_hcnt, L.ent_cnt, sizeof(int) * kStaticBatch * S, cudaMemcpyDeviceToHost, st));
+    TOMO_CUDA(cudaStreamSynchronize(st));
+    for (int k = 0; k < n; k++) need[k] = *std::max_element(g_static_hcnt + slots[k] * S, g_static_hcnt + (slots[k] + 1) * S);
+  }
+  for (int k = 0, g; k < n; k += g) {
+    int most = 0;
+    for (g = 0; k + g < n; g++) {
+      const int px = std::max(most, need[k + g]);
+      if (g > 0 && (size_t)px * (g + 1) * S * sizeof(uint2) > kStaticListBytes) break;
+      most = px;
+    }
+    TOMO_CUDA(cudaMemcpyAsync(L.ori + kStaticBatch, slots + k, sizeof(int) * g, cudaMemcpyHostToDevice, st));
+    TOMO_CUDA(launch_zero_ids(L.o_nbed, L.ori + kStaticBatch, g, st));
+    p.ent_cap = X.ent_cap;
+    static_bind(p, L, g, L.ori + kStaticBatch, 4 * X.P.n_tri + 4096);
+    p.ent_cap = std::min(p.ent_cap, most);
+    TOMO_CUDA(launch_batch(p, st, strip_smem_bytes(X.cfg[2].mode, X.H, X.G, p.ent_cap), nullptr));
+    TOMO_CUDA(launch_fold(p, st, nullptr));
+  }
+  TOMO_CUDA(cudaMemcpyAsync(g_static_hout, L.o_flags, sizeof(int) * kStaticBatch, cudaMemcpyDeviceToHost, st));
+  TOMO_CUDA(cudaStreamSynchronize(st));
+  for (int k = 0; k < n; k++) fl[slots[k]] = g_static_hout[slots[k]];
+  g_static_reruns[2] += n;
+  return 0;
+}
+
 // One batch slot re-run in strip configuration c (Engine::run_subset for a
 // single orientation); returns the slot's new status flags or an error.
 int static_rerun(Engine& X, const StaticLayout& L, int slot, int c, cudaStream_t st)
@@ -1773,7 +1814,7 @@ int static_rerun(Engine& X, const StaticLayout& L, int slot, int c, cudaStream_t
   EngineParams p = X.base_params(mode);
   p.variant = c;
   const int normal_cap = 4 * X.P.n_tri + 4096;
-  static_bind(p, L, 1, slot, mode != 1 ? normal_cap : INT_MAX);
+  static_bind(p, L, 1, L.ori + slot, mode != 1 ? normal_cap : INT_MAX);
   TOMO_CUDA(cudaMemsetAsync(L.o_nbed + slot, 0, sizeof(int), st));
   if (mode != 1) {
     TOMO_CUDA(launch_batch(p, st, X.cfg[c].smem, nullptr));
@@ -1909,24 +1950,25 @@ extern "C" int tomoSweepStatic(const float* f32info, const int* i32info, const f
     TOMO_CUDA(cudaMemsetAsync(L.o_nbed, 0, sizeof(int) * nb, st));
     X.choose_strips(0);
     EngineParams p = X.base_params(0);
-    static_bind(p, L, nb, 0, normal_cap);
+    static_bind(p, L, nb, L.ori, normal_cap);
     TOMO_CUDA(launch_batch(p, st, X.cfg[0].smem, nullptr));
     TOMO_CUDA(launch_fold(p, st, nullptr));
     TOMO_CUDA(cudaMemcpyAsync(g_static_hout, L.o_flags, sizeof(int) * 5 * B, cudaMemcpyDeviceToHost, st));
     TOMO_CUDA(cudaStreamSynchronize(st));
     bool rerun = false;
-    // the re-run ladder of Engine::resolve_ids, per flagged slot
+    // the re-run ladder of Engine::resolve_ids: overflowed strips together, the
+    // rest per flagged slot
+    int flags[B], big[B], n_big = 0;
     for (int o = 0; o < nb; o++) {
-      int fl = g_static_hout[o];
-      rerun = rerun || (fl & kFlagRedo);
-      if (fl & kFlagGrid) return set_error(TOMO_ERR_CAPACITY, "slot index outside the grid");
-      bool safe = (fl & (kFlagStray | kFlagBinCap)) != 0;
-      if (!safe && (fl & kFlagOverflow)) {
-        fl = static_rerun(X, L, o, 2, st);
-        if (fl < 0) return fl;
-        g_static_reruns[2]++;
-        safe = (fl & (kFlagStray | kFlagBinCap | kFlagOverflow)) != 0;
-      }
+      flags[o] = g_static_hout[o];
+      rerun = rerun || (flags[o] & kFlagRedo);
+      if (flags[o] & kFlagGrid) return set_error(TOMO_ERR_CAPACITY, "slot index outside the grid");
+      if (!(flags[o] & (kFlagStray | kFlagBinCap)) && (flags[o] & kFlagOverflow)) big[n_big++] = o;
+    }
+    if (n_big) TOMO_TRY(static_rerun_big(X, L, big, n_big, flags, st));
+    for (int o = 0; o < nb; o++) {
+      int fl = flags[o];
+      bool safe = (fl & (kFlagStray | kFlagBinCap | kFlagOverflow)) != 0;
       if (!safe && (fl & kFlagCap)) {
         fl = static_rerun(X, L, o, 4, st);
         if (fl < 0) return fl;
