@@ -33,3 +33,13 @@ def test_sample_counts(n):
     out = surrogate.mlp_predict(x)
     want = mo.forward(p.astype(np.float64), x.astype(np.float64))[-1][:, 0]
     assert np.max(np.abs(out - want)) <= 2e-5
+
+
+def test_predictions_do_not_depend_on_the_count():
+    """Eights of samples go to the CTAs in turn: the same bits for a sample whatever
+    the number of samples, around one eight per CTA and eight per CTA."""
+    surrogate.mlp_init(6)
+    x, _ = _data(9480, 3)
+    full = surrogate.mlp_predict(x)
+    for n in (1, 8, 9, 100, 1183, 1184, 1185, 1193, 9471, 9472, 9473):
+        assert np.array_equal(surrogate.mlp_predict(x[:n]).view(np.int32), full[:n].view(np.int32)), n
