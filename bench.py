@@ -14,7 +14,7 @@ Prints one JSON line (rank 0).  ``value`` is orientations/s of the device
 sweep with mesh and orientations resident in device memory (CUDA events on
 the engine's stream); ``e2e`` is the same metric through the reference
 C-ABI call TomoSh_CUDA with host buffers; ``roofline`` rates the two dominant
-kernels (k_raster and k_columns) against the measured HBM copy bandwidth; ``cpu_baseline``
+kernels (k_raster and k_columns, over the sweep's time) against the measured HBM copy bandwidth; ``cpu_baseline``
 is the reference INT3 engine (built from the reference sources) on the
 host cores over a bounded sample of the same orientations.  With N > 1
 (torchrun) the ranks split the one headline sweep into contiguous
@@ -304,28 +304,23 @@ def run_ours(args, rank, world, local_rank):
     except Exception as exc:   # a measurement aid: never costs the bench line
         print(f"read probe skipped: {exc}", file=sys.stderr)
 
-    # ---- roofline of the two dominant kernels, live event timing: k_raster
-    # writes each accepted pixel to its strip's list, k_columns (logged as
-    # k_strip) reads the lists
+    # ---- roofline of the two dominant kernels: k_raster writes each accepted
+    # pixel to its strip's list, k_columns (logged as k_strip) reads the lists
     peaks = _peaks()
-    strip = dict(klog["k_strip"])
-    strip["ms"] += klog["k_raster"]["ms"]
     algo_bytes_per_orient = 24 * mesh.n_vtx + 12 * mesh.n_tri + 16 * res["entries"].astype(np.float64) + 16
     algo_bytes = float(algo_bytes_per_orient.sum()) * args.steps
-    strip_ms = strip["ms"] if strip["timed"] else float("nan")
-    achieved = algo_bytes / (strip_ms / 1000.0) / 1e9 if strip["timed"] else None
+    rates = _rates(klog, algo_bytes, float(sum(step_ms)))
+    achieved = rates["achieved"]
     launches_per_step = {k: v["launches"] / args.steps for k, v in klog.items()}
-    roof = {"bound": "hbm", "kernel": "k_raster + k_columns", "achieved": achieved, "peak": peaks[0], "unit": "GB/s",
-            "frac": (achieved / peaks[0]) if achieved else None, "peak_source": peaks[1],
-            "traffic": _traffic(mesh, res, strip["launches"] / args.steps),
-            "avg_launch_ms": strip_ms / max(strip["timed"], 1),
-            "bytes_per_launch": algo_bytes / max(strip["launches"], 1),
-            "l2_read_gbs": l2_gbs, "frac_of_l2": (achieved / l2_gbs) if (achieved and l2_gbs) else None,
+    roof = {"bound": "hbm", "kernel": "k_raster + k_columns", **rates, "peak": peaks[0], "unit": "GB/s",
+            "frac": achieved / peaks[0], "peak_source": peaks[1],
+            "traffic": _traffic(mesh, res, klog["k_strip"]["launches"] / args.steps),
+            "l2_read_gbs": l2_gbs, "frac_of_l2": (achieved / l2_gbs) if l2_gbs else None,
             "l2_source": "the library's read probe over a 48 MB buffer, 40 passes after one untimed pass",
             # Event spans per kernel kind and step, each on its launching stream.  These are stream spans,
-            # not kernel times: the binning kernels of batch k+1 run on their own stream beside batch k's
-            # strips, so their spans include time spent waiting for SMs and for the other stream.  The
-            # per-kernel breakdown is the serialised ncu launch list summarised under profiles/.
+            # not kernel times: k_rotate and k_raster of batch k+1 run on their own stream beside batch k's
+            # k_columns, so the spans overlap and include time spent waiting for SMs.  The per-kernel
+            # breakdown is the serialised ncu launch list summarised under profiles/.
             "stream_spans_ms_per_step": {k: v["ms"] / args.steps for k, v in klog.items() if v["timed"]}}
 
     line = {"metric": METRIC, "value": value, "unit": UNIT, "n_gpus": world, "steps": args.steps,
@@ -419,6 +414,16 @@ def _peaks():
         except (ValueError, KeyError):
             pass
     return 6650.0, "fallback"
+
+
+def _rates(klog, algo_bytes, sweep_ms):
+    """What k_raster and k_columns reach together: their algorithmic bytes over the
+    device time of the sweeps they ran in.  The two run beside each other on two
+    streams (batch k+1 is rasterized while batch k's columns run), so that adding
+    their event spans would count the shared time twice."""
+    launches = max(klog["k_strip"]["launches"], 1)
+    return {"achieved": algo_bytes / (sweep_ms / 1000.0) / 1e9, "avg_launch_ms": sweep_ms / launches,
+            "bytes_per_launch": algo_bytes / launches}
 
 
 def _traffic(mesh, res, launches_per_step):

@@ -28,3 +28,16 @@ def test_reference_arm_line():
     assert line["e2e"]["h2d_bytes_per_step"] == 0 and line["e2e"]["d2h_bytes_per_step"] == 0
     assert line["cpu_baseline"]["kind"] in ("reference", "port") and line["cpu_baseline"]["cores"] >= 1
     assert line["config"]["workload"] == "solid82k_1deg"
+
+
+def test_roofline_rate_is_one_the_device_ran_at():
+    """k_raster and k_columns overlap: spans of 100 and 60 ms in a sweep of 110 ms
+    moved their bytes in 110 ms."""
+    import importlib.util
+    spec = importlib.util.spec_from_file_location("bench", ROOT / "bench.py")
+    bench = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(bench)
+    klog = {"k_raster": dict(launches=10, ms=100.0, timed=10), "k_strip": dict(launches=10, ms=60.0, timed=10)}
+    r = bench._rates(klog, 110e6, 110.0)
+    assert r["achieved"] == pytest.approx(1.0) and r["avg_launch_ms"] == pytest.approx(11.0)
+    assert r["bytes_per_launch"] == pytest.approx(11e6)
