@@ -86,3 +86,17 @@ def test_adaptation_steps_are_worth_a_check():
     got = native.sweep(m, ypr, PrintOptions())
     assert 0 < native.stats()["overflow_reruns"] <= 30
     _same(got, ref)
+
+
+@pytest.mark.parametrize("far", [5.0e3, 3.0e9, 1.0e20, 3.0e38])
+def test_meshes_beyond_any_grid_are_refused(far):
+    """Extents past the largest grid, also those whose span is no int."""
+    m = plates(1, 30.0, 20.0)
+    v = m.vertices.copy()
+    v[0, 0] = far
+    bad = meshgen.MeshArrays(v, m.faces, m.vertex_normals, m.face_normals, m.area)
+    ypr = meshgen.ypr_grid([0.0, 30.0], [0.0])
+    with pytest.raises(native.TomoError, match="mesh extent exceeds the supported slot grid"):
+        native.sweep(bad, ypr, PrintOptions())
+    with pytest.raises(native.TomoError, match="above the static limit"):
+        native.sweep_static(bad, ypr, PrintOptions())

@@ -417,6 +417,7 @@ struct Engine {
     }
     const double span = 2.0 * std::sqrt(r2) * 1.004 + std::max(0.0, (double)P.bed_outer) + 6.0;
     if (span <= 256.0) return 256;
+    if (!(span <= (double)kMaxGrid)) return kMaxGrid + 1;   // refused; (int)span may not exist
     return (int)span + (int)std::max(0.0f, P.bed_outer) + 2;
   }
 
