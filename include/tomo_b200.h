@@ -87,12 +87,15 @@ void tomoVolToMass(const float* f32info, const int* i32info, float* vm22);
 
 /* Tuning / test hooks. */
 #define TOMO_OPT_BATCH 1        /* orientations per device batch (default 256) */
-#define TOMO_OPT_STRIP_H 2      /* force strip height 1, 2, 4 or 8 (0 = automatic) */
+#define TOMO_OPT_STRIP_H 2      /* force strip height 1, 2, 4 or 8 (0 = automatic); a height times the grid edge past about
+                                   5,900 slots falls back to one column */
 #define TOMO_OPT_FORCE_SAFE 3   /* 1 = evaluate every orientation in safe mode */
 #define TOMO_OPT_NORMAL_SMEM 4  /* shared-memory budget of a normal strip, in bytes: its pixel capacity is what is left beside four
-                                   bytes and a bit per slot and a 20 KB work area, at 6 bytes a pixel (0 = what six CTAs per SM hold) */
+                                   bytes and a bit per slot and a 20 KB work area, at 6 bytes a pixel.  That is more than a strip takes (4
+                                   bytes a pixel and about 8 a slot), so a budget names a capacity, not a CTA's size.  0 = what six
+                                   CTAs per SM hold (fewer CTAs on grids past about 1,700 columns) */
 #define TOMO_OPT_EXPORT 5       /* 0 = skip the best orientation's pixel export (default 1) */
-#define TOMO_OPT_ADAPTIVE 6     /* 0 = keep the planned strip budget even when early batches overflow (default 1) */
+#define TOMO_OPT_ADAPTIVE 6     /* 0 = keep the planned strips even when early batches overflow (default 1) */
 #define TOMO_OPT_PROPOSAL 7     /* tomoSurrogateSearch proposals: 0 = the trained network (default), 1 = bilinear
                                    interpolation of the exact coarse values (the search without the network),
                                    2 = the mean of the two */
@@ -124,7 +127,8 @@ int tomoSweepDevice(void* ev_start, void* ev_stop, float* kernel_ms);
 int tomoFinish(float* Mo, float* Mss, float* Vtc);
 
 /* Launch accounting.  Kernel kinds, in order: reset, rotate, bin_count,
- * bin_scan, bin_fill, strip, bed, fold, strip re-runs, raster.  tomoProfile(enable, reset) turns
+ * bin_scan, bin_fill, strip (k_columns, or k_strip in sweeps that start in
+ * priority strips), bed, fold, strip re-runs, raster.  tomoProfile(enable, reset) turns
  * per-launch CUDA-event timing on or off (events are recorded on the stream
  * each kernel is launched on) and optionally clears the log;
  * tomoGetKernelLog fills launches / total ms / timed launches per kind and
@@ -176,7 +180,7 @@ int TomoSh_CUDA_Batch(int n_mesh, const float* const* f32info, const int* const*
  * orientations re-run, time of the last run in microseconds (sweep and
  * re-runs, as device_ms), time of its sweep alone (the graph replay) */
 int tomoBatchStats(long long* out, int n);
-/* out4 = orientations per batch, normal-CTA shared-memory budget (0 = six CTAs per SM),
+/* out4 = orientations per batch, normal strip budget (as TOMO_OPT_NORMAL_SMEM),
  * strip height, slot-grid edge chosen for mesh `mesh` */
 int tomoBatchConfig(int mesh, int* out4);
 /* The TomoSh_CUDA tail for mesh `mesh` of the last tomoBatchRun: the getters

@@ -371,9 +371,9 @@ struct Engine {
   int batch = 256;
   int force_h = 0;        // test hook: strip height override
   int force_safe = 0;     // test hook: run every orientation in safe mode
-  int normal_smem = 0;    // shared-memory budget of a normal strip CTA (0 = six CTAs per SM)
+  int normal_smem = 0;    // budget of a normal strip (budget_pixels; 0 = the plan's own: plan_strips)
   int export_pixels = 1;  // rebuild the best orientation's pixels and vm_info (TomoSh_CUDA tail)
-  int adaptive = 1;       // raise the entry budget after overflowing early batches (full sweeps)
+  int adaptive = 1;       // shorter strips or a larger budget after overflowing early batches (full sweeps)
   int fold_lim = 32767;   // largest |column value| of a packed fold record (TOMO_OPT_FOLD_LIMIT)
   int adapt_smem = 0, adapt_h = 0;   // configuration adapted to by an earlier sweep of this upload
   int adapt_cfg = 0;                  // 4 once a sweep of this upload switched to priority strips
@@ -424,7 +424,8 @@ struct Engine {
   // Strip configurations.
   //   0 normal     : H0-column strips whose columns k_columns resolves from
   //                  k_raster's pixel lists, six CTAs per SM; H0 is the
-  //                  tallest strip with room for two pixels per slot;
+  //                  tallest strip with room for two pixels per slot (one
+  //                  column, and fewer CTAs, on the widest grids);
   //   1 safe       : strips that rasterize their own triangles, whole-box
   //                  evaluation, priorities, all opt-in shared memory;
   //   2 big normal : configuration 0 semantics with all opt-in shared memory
@@ -789,11 +790,10 @@ struct Engine {
     int Bo = batch_size(std::min(batch, n), cfg[c].mode);
     const int bin_cap = 4 * P.n_tri + 4096;
     TOMO_TRY(reserve_outputs());
-    // Two batches in flight: batch k+1's binning (reset, rotate, bin
-    // count / scan / fill) runs on the binning stream into the other
-    // PrepSet while batch k's strips run on main; each batch's fold follows
-    // on the side stream.  A set is rebinned only after the fold of the
-    // batch that last used it.
+    // Two batches in flight: batch k+1 is rotated and rasterized (priority
+    // strips: binned) on the binning stream into the other PrepSet while batch
+    // k's columns run on main; each batch's fold follows on the side stream.  A
+    // set is filled again only after the fold of the batch that last used it.
     int nprep = 1;
     TOMO_TRY(reserve_fitting(cfg[c].mode, &Bo, bin_cap, n, &nprep));
     const bool pipe = nprep > 1;
@@ -1124,8 +1124,10 @@ struct Engine {
   // sweep of the sample, re-runs included: the configuration-0 strips, then
   // the ladder that re-runs what they flagged (Engine::resolve), so a budget
   // too small for the mesh pays for its overflows.  Candidates: 128 or 256
-  // orientations per batch x the normal strip budget (six CTAs per SM, 72 KB,
-  // 99 KB) x the strip height (the planned one and half of it).  When most of
+  // orientations per batch x the normal strip budget (six CTAs per SM, or the
+  // pixels that budgets of 73,728 and 101,376 bytes buy: budget_pixels, CTAs of 48
+  // and 67 KB on the 256 grid) x the strip height (the planned one and half of
+  // it).  When most of
   // the sample passes the 63-pixel cap in some column, every candidate starts
   // in the priority-carrying strips (configuration 4), as an adaptive sweep
   // would switch to them.

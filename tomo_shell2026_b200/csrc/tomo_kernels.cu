@@ -6,7 +6,8 @@
 // see the launch sequence in tomo_engine.cu.  The work per orientation is the
 // reference INT3 pipeline (Tomo_Shell2026.cpp thread_func:138-156):
 // Rotate -> Pixelize -> Pairing -> GenerateBed -> Calculate, re-organised so
-// that the per-column pixel lists never leave shared memory:
+// that an accepted pixel crosses device memory once and columns exist in shared
+// memory only:
 //
 //  * the slot grid is cut into strips of H x-columns; k_raster rasterizes
 //    every triangle once and appends its accepted pixels to their strips'
@@ -347,7 +348,7 @@ __global__ void __launch_bounds__(256) k_rotate(EngineParams p)
 }
 
 // ---------------------------------------------------------------- K2 binning
-// Strip range of one triangle.  Normal mode: the strips its pixel box
+// Strip range of one triangle.  Priority strips: the strips its pixel box
 // covers; a triangle spanning several strips whose box holds no accepted
 // pixel centre goes only to the strip of its centroid pixel, flagged as
 // "fallback only" (code 2).  Safe mode: the box widened by e columns on both
@@ -356,8 +357,7 @@ __global__ void __launch_bounds__(256) k_rotate(EngineParams p)
 
 struct BinRange { int s0, s1, code; };
 
-__device__ __forceinline__ BinRange bin_range(const EngineParams& p, int o, int t, const Shift& sh, int* flag,
-                                              const uint8_t* known_code)
+__device__ __forceinline__ BinRange bin_range(const EngineParams& p, int o, int t, const Shift& sh, int* flag)
 {
   TriGeo g;
   float4 raw[3];
@@ -370,15 +370,10 @@ __device__ __forceinline__ BinRange bin_range(const EngineParams& p, int o, int 
     r.s0 = min(x0 / p.H, p.S - 1);
     r.s1 = min(max(x1, 0) / p.H, p.S - 1);
     if (r.s0 != r.s1) {
-      int code;
-      if (known_code) code = *known_code;
-      else {
-        Bary b;
-        bary_setup(g, b);
-        code = any_hit(p, g, b) ? 1 : 2;
-      }
-      r.code = code;
-      if (code == 2) {
+      Bary b;
+      bary_setup(g, b);
+      r.code = any_hit(p, g, b) ? 1 : 2;
+      if (r.code == 2) {
         const int cxs = centroid_slot_x(raw, sh);
         const int sc = min(max(cxs, 0), p.G - 1) / p.H;
         r.s0 = r.s1 = min(sc, p.S - 1);
@@ -424,7 +419,7 @@ __global__ void __launch_bounds__(256) k_bin_count(EngineParams p)
     const int t = tb + threadIdx.x;
     BinRange r; r.s0 = 0; r.s1 = -1; r.code = 0;
     if (t < p.nT) {
-      r = bin_range(p, o, t, sh, &sflag, nullptr);
+      r = bin_range(p, o, t, sh, &sflag);
       p.trange[(size_t)o * p.nT + t] = pack_range(r);
     }
     for (int s = r.s0; s <= r.s1; s++) atomicAdd(&sh_cnt[s], 1);
@@ -835,9 +830,9 @@ struct StripSmem {
   unsigned* occ;       // [ceil(H*G/32)] occupied-slot bitmap
   unsigned* ekey;      // [C] (z+32768) << 16 | (nz+32768)
   short* enext;        // [C] next entry of the same column, -1 at the end
-  unsigned* et;        // [C] safe mode: triangle index (priority, major)
-  unsigned* elo;       // [C] safe mode: pixel index * 2 + twin (priority, minor)
-  uint8_t* emark;      // [C] safe mode: first-come marks
+  unsigned* et;        // [C] triangle index (priority, major)
+  unsigned* elo;       // [C] pixel index * 2 + twin (priority, minor)
+  uint8_t* emark;      // [C] first-come marks
   float4* q0; float4* q1; float4* q2;   // [kChunk] margined vertices, vertex-normal z
   int4* tm;            // [kChunk] t, x0, y0, ylen
   int* pref;           // [kChunk + 4]
@@ -1101,9 +1096,8 @@ __device__ ColOut column(const EngineParams& p, const StripSmem& sm, int head, b
       d++;
     }
   }
-  // Past 63 distinct keys the first-come cap decides which survive, which
-  // needs priorities: normal strips hand the orientation on; priority strips
-  // start the column over with them.
+  // Past 63 distinct keys the first-come cap decides which survive: the column
+  // starts over with its pixels' priorities.
   if (need_prio) {
     col_init(s);
     d = 0;
@@ -1203,7 +1197,7 @@ struct TriReg {
   int t, x0, y0, ylen, xc0;
 };
 
-// xlo: first slot row of the strip (normal modes) or INT_MIN (safe mode walks
+// xlo: first slot row of the strip (priority strips) or INT_MIN (safe mode walks
 // the whole box).
 __device__ __forceinline__ void tri_from_smem(const StripSmem& sm, int ti, int xlo, TriReg& r)
 {
@@ -1386,8 +1380,7 @@ __global__ void __launch_bounds__(256, 1) k_strip(EngineParams p)
     int npix = 0;
     // centroid fallback pixel of this thread's triangle (STomoSh_INT3.cpp:1190-1206), from the
     // translated unmargined vertices while they are in registers; used after the walk if the
-    // triangle had no accepted pixel: slot x, y packed as two int16 (normal strips keep them in
-    // the staged triangle record, whose triangle index only priority strips read), and z (fbz)
+    // triangle had no accepted pixel: slot x, y packed as two int16, and z (fbz)
     fb_xy = 0;
     if (i < nchunk) {
       const int entry = list[cb + i];
@@ -2651,7 +2644,7 @@ static dim3 tri_grid(const EngineParams& p)
 }
 
 // Lanes per triangle in k_raster: one, unless that gives fewer warps than
-// kRastFill; then the lanes of a triangle share its cells (256 orientations of a
+// kRastFill (64 for each of a B200's 148 SMs); then the lanes of a triangle share its cells (256 orientations of a
 // 320-triangle solid 330 pixels across: 1,112 us with a quarter of this, 943
 // with half, 732).
 constexpr int kRastFill = 148 * 64;
