@@ -135,6 +135,8 @@ def vol_to_mass(f32info, i32info, vm22) -> np.ndarray:
     return vm
 
 
+# "k_strip" counts the column stage of every batch that is no re-run: k_columns, or
+# k_strip itself in sweeps that start in priority strips
 KERNEL_KINDS = ("k_reset", "k_rotate", "k_bin_count", "k_bin_scan", "k_bin_fill", "k_strip", "k_bed", "k_fold",
                 "k_strip_redo", "k_raster")
 
